@@ -9,6 +9,7 @@
 #include <mutex>
 
 #include "common.cuh"
+#include "fft_inplace.cuh"
 #include "internal.h"
 
 #define ZR_VERSION 100
@@ -38,8 +39,9 @@ int launched(const char* what) {
 }
 
 // W_TWN^k = exp(-2 pi i k / TWN), then its contiguous copies per
-// sub-transform length (tw_compact_off), one table per device.
-static __device__ float2 d_twiddle[TWN + TW_COMPACT];
+// sub-transform length (tw_compact_off) and the in-place transforms' tables
+// (ip_tw_off), one table per device.
+static __device__ float2 d_twiddle[TWN + TW_COMPACT + IP_TW];
 
 static std::mutex g_init_mu;
 static bool g_init_done[64];
@@ -52,7 +54,7 @@ static int init_device(int dev) {
   int prev = 0;
   ZR_TRY(cuda_check(cudaGetDevice(&prev), "cudaGetDevice"));
   if (prev != dev) ZR_TRY(cuda_check(cudaSetDevice(dev), "cudaSetDevice"));
-  static float2 host[TWN + TW_COMPACT];
+  static float2 host[TWN + TW_COMPACT + IP_TW];
   for (int k = 0; k < TWN; k++) {
     const double a = -2.0 * M_PI * (double)k / (double)TWN;
     host[k] = make_float2((float)cos(a), (float)sin(a));
@@ -62,6 +64,16 @@ static int init_device(int dev) {
     for (int j = 0; j < M; j++) host[TWN + tw_compact_off(M) + j] = host[(size_t)j * (TWN / M)];
     if (3 * M <= 12288)
       for (int j = 0; j < 3 * M; j++) host[TWN + tw_compact_off(3 * M) + j] = host[(size_t)j * (TWN / (3 * M))];
+  }
+  for (int i = 0; i <= IP_LENGTHS; i++) {
+    const int L = ip_length(i);
+    float2* t = host + TWN + TW_COMPACT + ip_tw_off(L);
+    const int M2 = 16 * ip_r2(L), RL = ip_rl(L), NS = L / RL;
+    if (ip_r3(L) > 1)
+      for (int r = 1; r < ip_r2(L); r++)
+        for (int k = 0; k < 16; k++) *t++ = host[(size_t)(r * k % M2) * (TWN / M2)];
+    for (int q = 0; q < ip_slots(RL); q++)
+      for (int k = 0; k < NS; k++) *t++ = host[(size_t)(ip_slot_r(q) * k % L) * (TWN / L)];
   }
   int rc = cuda_check(cudaMemcpyToSymbol(d_twiddle, host, sizeof(host)), "twiddle upload");
   void* p = nullptr;

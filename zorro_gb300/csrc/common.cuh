@@ -128,13 +128,20 @@ __device__ __forceinline__ uint4 raw_quad(const void* raw, long long i) {
   return r;
 }
 
+// Integers below 2^23 become floats by placing them in the mantissa of 2^23
+// and subtracting it: exact, and on the FP32 pipe (conversions run at an
+// eighth of its rate).
+__device__ __forceinline__ float mantissa_value(unsigned int bits) { return __uint_as_float(bits) - 8388608.0f; }
+
 template <int TYPE>
 __device__ __forceinline__ float4 quad_value(const uint4 r) {
+  constexpr unsigned int E = 0x4b000000u;  // 2^23
   if (TYPE == ZR_U8)
-    return make_float4((float)(r.x & 0xffu), (float)((r.x >> 8) & 0xffu), (float)((r.x >> 16) & 0xffu),
-                       (float)(r.x >> 24));
+    return make_float4(mantissa_value(__byte_perm(r.x, E, 0x7440)), mantissa_value(__byte_perm(r.x, E, 0x7441)),
+                       mantissa_value(__byte_perm(r.x, E, 0x7442)), mantissa_value(__byte_perm(r.x, E, 0x7443)));
   if (TYPE == ZR_U16)
-    return make_float4((float)(r.x & 0xffffu), (float)(r.x >> 16), (float)(r.y & 0xffffu), (float)(r.y >> 16));
+    return make_float4(mantissa_value(__byte_perm(r.x, E, 0x7410)), mantissa_value(__byte_perm(r.x, E, 0x7432)),
+                       mantissa_value(__byte_perm(r.y, E, 0x7410)), mantissa_value(__byte_perm(r.y, E, 0x7432)));
   if (TYPE == ZR_F16)
     return make_float4(__half2float(__ushort_as_half((unsigned short)(r.x & 0xffffu))),
                        __half2float(__ushort_as_half((unsigned short)(r.x >> 16))),
@@ -202,6 +209,65 @@ __device__ __forceinline__ float4 finish4(const FrameSrc& f, const Px4& q) {
     v = make_float4(__fmaf_rn(q.a.x, v.x, q.b.x), __fmaf_rn(q.a.y, v.y, q.b.y), __fmaf_rn(q.a.z, v.z, q.b.z),
                     __fmaf_rn(q.a.w, v.w, q.b.w));
   return v;
+}
+
+// Corrected pixels (load_corrected) x = j + r STEP (r < 16) of row y of frame
+// n: every load of the row's counts and maps is issued before any value is
+// used.  The caller knows that the first FULL of them lie inside the row for
+// every j; the others are loaded where x < cols and are 0 elsewhere.
+template <int STEP, int FULL>
+__device__ __forceinline__ void corrected16(const FrameSrc& f, int n, int y, int j, int cols, float* u) {
+  const int lim = cols - j;
+  const long long q = (long long)y * f.W + j;
+  const long long p = q + map_off(f, n);
+  const long long i = (long long)n * f.fstride + q;
+  unsigned int bits[16];
+  float g[16], a[16], b[16];
+#define ZR_INSIDE(r) (r < FULL || r * STEP < lim)
+  if (f.type == ZR_U8) {
+#pragma unroll
+    for (int r = 0; r < 16; r++) bits[r] = ZR_INSIDE(r) ? __ldg((const uint8_t*)f.raw + i + r * STEP) : 0u;
+  } else if (f.type == ZR_F32) {
+#pragma unroll
+    for (int r = 0; r < 16; r++) bits[r] = ZR_INSIDE(r) ? __ldg((const unsigned int*)f.raw + i + r * STEP) : 0u;
+  } else {
+#pragma unroll
+    for (int r = 0; r < 16; r++) bits[r] = ZR_INSIDE(r) ? __ldg((const uint16_t*)f.raw + i + r * STEP) : 0u;
+  }
+  if (f.gain) {
+#pragma unroll
+    for (int r = 0; r < 16; r++) g[r] = ZR_INSIDE(r) ? __ldg(f.gain + p + r * STEP) : 0.0f;
+  }
+  if (f.ha) {
+#pragma unroll
+    for (int r = 0; r < 16; r++) {
+      a[r] = ZR_INSIDE(r) ? __ldg(f.ha + p + r * STEP) : 0.0f;
+      b[r] = ZR_INSIDE(r) ? __ldg(f.hb + p + r * STEP) : 0.0f;
+    }
+  }
+#undef ZR_INSIDE
+  if (f.type == ZR_F32) {
+#pragma unroll
+    for (int r = 0; r < 16; r++) u[r] = __uint_as_float(bits[r]);
+  } else if (f.type == ZR_F16) {
+#pragma unroll
+    for (int r = 0; r < 16; r++) u[r] = __half2float(__ushort_as_half((unsigned short)bits[r]));
+  } else {
+#pragma unroll
+    for (int r = 0; r < 16; r++) u[r] = (float)bits[r];
+  }
+  if (f.gain) {
+#pragma unroll
+    for (int r = 0; r < 16; r++) u[r] = __fmul_rn(g[r], u[r]);
+  }
+  if (f.gdiv != 0.0f) {
+#pragma unroll
+    for (int r = 0; r < 16; r++) u[r] = __fdiv_rn(u[r], f.gdiv);
+  }
+  if (f.ha) {
+#pragma unroll
+    for (int r = 0; r < 16; r++) u[r] = __fmaf_rn(a[r], u[r], b[r]);
+  }
 }
 
 __device__ __forceinline__ int ilog2c(int v) { return 31 - __clz(v); }

@@ -6,171 +6,180 @@
 // Hermitian symmetry), only the C1/2+1 non-negative kx columns the crop keeps
 // are written, and the column pass keeps only the C0+1 cropped ky rows.
 //
-// Row-pass output layout (scratch): [frame][y/4][K4][y%4] complex, so that
-// the row pass (4 rows per CTA) and the column pass (4 columns per CTA) both
-// move whole 128-byte lines.
+// Row-pass output layout (scratch): [frame][y/16][K4][y%16] complex (the last
+// group of a frame as many rows as it has, a multiple of 4), so that the row
+// pass (4 rows per CTA) writes whole 32-byte sectors and a warp of the column
+// pass reads 128-byte runs.
 #include <stdio.h>
 
+#include <type_traits>
+
 #include "common.cuh"
+#include "fft_inplace.cuh"
 #include "internal.h"
 
 namespace zr {
 
-constexpr int NBR = 4;  // rows per group of the row-pass output layout
+constexpr int NBR = 16;  // rows per group of the row-pass output layout
+// Element (k, y) of one frame's row-pass output of 4 H4 rows.
+__device__ __forceinline__ int ru_rows(int y, int H4) { return min(NBR, 4 * H4 - (y & ~(NBR - 1))); }
+__device__ __forceinline__ size_t ru_at(int k, int y, int K4, int H4) {
+  return (size_t)(y & ~(NBR - 1)) * K4 + (size_t)k * ru_rows(y, H4) + (y & (NBR - 1));
+}
 // rows per CTA of the row pass and columns per CTA of the column pass: the
-// defaults (two CTAs share an SM at 4096 points), or the planner's choice of
-// 1, 2 or 4 per transform length (tune_get)
-constexpr int FR_DEFAULT = 2, FC_DEFAULT = 2;
+// defaults (the row pass's four rows fill whole sectors of its output, up to
+// 4096 points), or the planner's choice of 1, 2 or 4 per transform length
+// (tune_get)
+constexpr int FC_DEFAULT = 2;
+__host__ __device__ constexpr int fr_default(int P1) { return P1 > 4096 ? 2 : 4; }
 // CTAs per SM to ask the register allocator for: 128 registers a thread
 constexpr int minb_of(int T) { return sm_minb(T); }
 
+// Row pass: FR rows of one frame per CTA.  The first FFT pass reads the
+// pixels (consecutive lanes, consecutive pixels) and the last one untangles
+// the half-plane rows of u and u^2 in registers, so the rows pass through
+// shared memory twice and the CTA meets at two barriers.
 template <int P1, int FR>
-__global__ void __launch_bounds__(fft_threads(P1, FR), minb_of(fft_threads(P1, FR)))
+__global__ void __launch_bounds__(ip_threads(P1, FR), minb_of(ip_threads(P1, FR)))
     k_fwd_rows(FrameSrc f, const float* __restrict__ mask, const double* __restrict__ mean_sub,
                double inv_area, int frame0, int mode, int rows, int cols, int C1, int K4, int H4,
                float2* __restrict__ RU, float2* __restrict__ RV, const float2* __restrict__ tw) {
-  constexpr int T = fft_threads(P1, FR);
-  constexpr int LD = ld_of(P1);
+  constexpr int T = ip_threads(P1, FR);
+  using P = Ip<P1>;
   extern __shared__ float2 sm[];
   // frames vary fastest so that concurrent CTAs read the same rows of the
   // gain and hot-pixel maps through L2
-  const int g = blockIdx.y;
+  const int y0 = blockIdx.y * FR;
   const int nl = blockIdx.x;
   const int n = frame0 + nl;
   float mu = 0.0f;
   if (mode == 0 && mean_sub) mu = (float)(mean_sub[n] * inv_area);
-  if (mode == 0 && !mask && (f.fstride & 3) == 0 && (f.mstride & 3) == 0) {
-    // 4 pixels per thread and step: aligned vector loads of the raw frame and
-    // every map; the unaligned head (< 4 pixels) and tail go pixel by pixel
-    // FR_UNR quads per thread are fetched before any is used, so that several
-    // loads per thread are in flight
-    constexpr int NQ = FR * (P1 / 4);
-    constexpr int FR_UNR = 4;
-    for (int e0 = threadIdx.x; e0 < NQ; e0 += T * FR_UNR) {
-      Px4 px[FR_UNR];
-#pragma unroll
-      for (int u = 0; u < FR_UNR; u++) {
-        const int e = e0 + u * T;
-        if (e < NQ) {
-          const int r = e / (P1 / 4), q = e - r * (P1 / 4);
-          const int y = g * FR + r;
-          if (y < rows) {
-            const long long p0 = (long long)y * f.W;
-            const int x = (int)((4 - (p0 & 3)) & 3) + 4 * q;
-            if (x + 3 < cols) fetch4(f, n, p0 + x, px[u]);
-          }
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < FR_UNR; u++) {
-        const int e = e0 + u * T;
-        if (e >= NQ) continue;
-        const int r = e / (P1 / 4), q = e - r * (P1 / 4);
-        const int y = g * FR + r;
-        float2* srow = sm + r * LD;
+  if (mode == 0 && !mask) {
+    auto pixels = [&](auto full) {
+      constexpr int FULL = decltype(full)::value;
+      ip_pass1<P1, FR, T, -1, false>(sm, [&](int b, int j, float2* v) {
+        const int y = y0 + b;
         if (y >= rows) {
 #pragma unroll
-          for (int j = 0; j < 4; j++) srow[pidx(4 * q + j)] = make_float2(0.0f, 0.0f);
-          continue;
+          for (int r = 0; r < 16; r++) v[r] = make_float2(0.0f, 0.0f);
+          return;
         }
-        const long long p0 = (long long)y * f.W;
-        const int off = (int)((4 - (p0 & 3)) & 3);  // first x with (p0 + x) % 4 == 0
-        const int x = off + 4 * q;
-        if (x + 3 < cols) {
-          const float4 v = finish4(f, px[u]);
-          const float u0 = v.x - mu, u1 = v.y - mu, u2 = v.z - mu, u3 = v.w - mu;
-          srow[pidx(x)] = make_float2(u0, u0 * u0);
-          srow[pidx(x + 1)] = make_float2(u1, u1 * u1);
-          srow[pidx(x + 2)] = make_float2(u2, u2 * u2);
-          srow[pidx(x + 3)] = make_float2(u3, u3 * u3);
-        } else {
+        float u[16];
+        corrected16<P::A1, FULL>(f, n, y, j, cols, u);
+        const int lim = cols - j;
 #pragma unroll
-          for (int j = 0; j < 4; j++) {
-            const int xx = x + j;
-            if (xx < P1) {
-              float2 z = make_float2(0.0f, 0.0f);
-              if (xx < cols) {
-                const float u = load_corrected(f, n, y, xx) - mu;
-                z = make_float2(u, u * u);
-              }
-              srow[pidx(xx)] = z;
-            }
-          }
+        for (int r = 0; r < 16; r++) {
+          const float w = r < FULL || r * P::A1 < lim ? u[r] - mu : 0.0f;
+          v[r] = make_float2(w, w * w);
         }
-        if (q == 0) {
-          for (int xx = 0; xx < off; xx++) {
-            float2 z = make_float2(0.0f, 0.0f);
-            if (xx < cols) {
-              const float u = load_corrected(f, n, y, xx) - mu;
-              z = make_float2(u, u * u);
-            }
-            srow[pidx(xx)] = z;
-          }
-        }
-      }
-    }
+      });
+    };
+    // pixels that need no test against the row's end (frames fill most of
+    // their padded rows)
+    if (cols >= 14 * P::A1) pixels(std::integral_constant<int, 14>());
+    else pixels(std::integral_constant<int, 0>());
   } else {
-    for (int e = threadIdx.x; e < FR * P1; e += T) {
-      const int r = e / P1, x = e - (e / P1) * P1;
-      const int y = g * FR + r;
-      float2 z = make_float2(0.0f, 0.0f);
-      if (y < rows && x < cols) {
-        const float m = mask ? __ldg(mask + (size_t)y * P1 + x) : 1.0f;
-        if (mode == 0) {
-          const float u = m * (load_corrected(f, n, y, x) - mu);
-          z = make_float2(u, u * u);
-        } else {
-          z.x = m;
+    ip_pass1<P1, FR, T, -1, false>(sm, [&](int b, int j, float2* v) {
+      const int y = y0 + b;
+#pragma unroll
+      for (int r = 0; r < 16; r++) {
+        const int x = j + r * P::A1;
+        v[r] = make_float2(0.0f, 0.0f);
+        if (y < rows && x < cols) {
+          const float m = mask ? __ldg(mask + (size_t)y * P1 + x) : 1.0f;
+          if (mode == 0) {
+            const float w = m * (load_corrected(f, n, y, x) - mu);
+            v[r] = make_float2(w, w * w);
+          } else {
+            v[r].x = m;
+          }
         }
       }
-      sm[r * LD + pidx(x)] = z;
-    }
+    });
   }
   __syncthreads();
-  block_fft<P1, FR, T, -1>(sm, tw);
+  ip_pass2<P1, FR, T, -1, false>(sm, tw);
   const int half = C1 / 2;
-  for (int e = threadIdx.x; e < K4 * FR; e += T) {
-    const int k = e / FR, r = e - (e / FR) * FR;
-    const int y = g * FR + r;
-    const size_t o = (((size_t)nl * H4 + (y >> 2)) * K4 + k) * NBR + (y & 3);
-    float2 U = make_float2(0.0f, 0.0f), V = U;
-    if (k <= half) {
-      const float2 zk = sm[r * LD + pidx(k)];
-      const float2 zm = sm[r * LD + pidx(k == 0 ? 0 : P1 - k)];
-      U = make_float2(0.5f * (zk.x + zm.x), 0.5f * (zk.y - zm.y));
-      V = make_float2(0.5f * (zk.y + zm.y), -0.5f * (zk.x - zm.x));
+  const size_t frame_out = (size_t)nl * 4 * H4 * K4;
+  const int step = ru_rows(y0, H4);  // between consecutive k (the CTA's rows share a group)
+  ip_last_paired<P1, FR, T, -1>(sm, tw, [&](int b, int k0, const float2* X0, int k1, const float2* X1) {
+    if ((y0 + b) >> 2 >= H4) return;
+    const size_t o = frame_out + ru_at(0, y0 + b, K4, H4);
+    float2 *ou = RU + o, *ov = RV + o;
+    auto put = [&](int k, float2 zk, float2 zm) {
+      ou[k * step] = make_float2(0.5f * (zk.x + zm.x), 0.5f * (zk.y - zm.y));
+      if (mode == 0) ov[k * step] = make_float2(0.5f * (zk.y + zm.y), -0.5f * (zk.x - zm.x));
+    };
+#pragma unroll
+    for (int q = 0; q < P::RL; q++) {
+      const int m0 = k0 + q * P::NS, m1 = k1 + q * P::NS;
+      if (m0 <= half) put(m0, X0[q], k0 > 0 ? X1[P::RL - 1 - q] : X0[(P::RL - q) % P::RL]);
+      if (m1 <= half) put(m1, X1[q], k0 > 0 ? X0[P::RL - 1 - q] : X1[P::RL - 1 - q]);
     }
-    RU[o] = U;
-    if (mode == 0) RV[o] = V;
+  });
+  // the pitch's columns past C1/2 are zero
+  for (int e = threadIdx.x; e < FR * (K4 - half - 1); e += T) {
+    const int b = e % FR, k = half + 1 + e / FR;
+    if ((y0 + b) >> 2 >= H4) continue;
+    const size_t o = frame_out + ru_at(k, y0 + b, K4, H4);
+    RU[o] = make_float2(0.0f, 0.0f);
+    if (mode == 0) RV[o] = make_float2(0.0f, 0.0f);
   }
 }
 
+// Column pass: FC columns of one spectrum per CTA, read from the row pass's
+// output by the first FFT pass (zero past the frame: the zero padding to P0)
+// and written by the last one: consecutive lanes hold consecutive ky.
 template <int P0, int FC>
-__global__ void __launch_bounds__(fft_threads(P0, FC), minb_of(fft_threads(P0, FC)))
+__global__ void __launch_bounds__(ip_threads(P0, FC), minb_of(ip_threads(P0, FC)))
     k_fwd_cols(const float2* __restrict__ RU, const float2* __restrict__ RV, int rows, int C0, int K4, int H4,
                long long spec_elems, float2* __restrict__ G, float2* __restrict__ S,
                const float2* __restrict__ tw) {
-  constexpr int T = fft_threads(P0, FC);
-  constexpr int LD = ld_of(P0);
+  constexpr int T = ip_threads(P0, FC);
+  using P = Ip<P0>;
   extern __shared__ float2 sm[];
   const int k0 = blockIdx.x * FC;
   const int nl = blockIdx.y;
-  const float2* R = (blockIdx.z == 0 ? RU : RV) + (size_t)nl * H4 * K4 * NBR;
-  float2* out = (blockIdx.z == 0 ? G : S) + (size_t)nl * spec_elems;
-  // element y of column k0 + c: row y of the row-pass output, zero past the
-  // frame (the zero padding to P0)
-  block_fft_from<P0, FC, T, -1>(sm, tw, [&](int c, int y) {
-    return y < rows ? __ldg(R + ((size_t)(y >> 2) * K4 + k0 + c) * NBR + (y & 3)) : make_float2(0.0f, 0.0f);
-  });
+  const float2* R = (blockIdx.z == 0 ? RU : RV) + (size_t)nl * 4 * H4 * K4;
   const int hc = C0 / 2;
   const int RP = C0 + 4;
+  float2* out = (blockIdx.z == 0 ? G : S) + (size_t)nl * spec_elems + (size_t)k0 * RP;
+  // (whole groups of rows and a butterfly step of whole groups: one stride)
+  const bool even = (H4 & 3) == 0 && P::A1 % NBR == 0;
+  ip_pass1<P0, FC, T, -1, false>(sm, [&](int c, int j, float2* v) {
+    if (even) {
+      const float2* src = R + (size_t)(j & ~(NBR - 1)) * K4 + (k0 + c) * NBR + (j & (NBR - 1));
+      const size_t step = (size_t)P::A1 * K4;
+      const int lim = rows - j;
+#pragma unroll
+      for (int r = 0; r < 16; r++) {
+        v[r] = make_float2(0.0f, 0.0f);
+        if (r * P::A1 < lim) v[r] = __ldg(src);
+        src += step;
+      }
+    } else {
+#pragma unroll
+      for (int r = 0; r < 16; r++) {
+        const int y = j + r * P::A1;
+        v[r] = y < rows ? __ldg(R + ru_at(k0 + c, y, K4, H4)) : make_float2(0.0f, 0.0f);
+      }
+    }
+  });
   // rows C0 + 1 .. C0 + 3 pad the column to its pitch: written as zeros, so
   // that every element of a spectrum is defined (zr_pack_half scans them all)
-  for (int e = threadIdx.x; e < RP * FC; e += T) {
-    const int c = e / RP, r = e - c * RP;
-    const int ky = r < hc ? r : (r < C0 ? P0 - C0 + r : hc);
-    out[(size_t)(k0 + c) * RP + r] = r <= C0 ? sm[c * LD + pidx(ky)] : make_float2(0.0f, 0.0f);
-  }
+  for (int e = threadIdx.x; e < 3 * FC; e += T) out[(size_t)(e / 3) * RP + C0 + 1 + e % 3] = make_float2(0.0f, 0.0f);
+  __syncthreads();
+  ip_pass2<P0, FC, T, -1, false>(sm, tw);
+  ip_last<P0, FC, T, -1, false>(sm, tw, [&](int c, int k, const float2* v) {
+    float2* col = out + (size_t)c * RP;
+#pragma unroll
+    for (int r = 0; r < P::RL; r++) {
+      const int ky = k + r * P::NS;
+      if (ky < hc) col[ky] = v[r];
+      if (ky == hc) col[C0] = v[r];
+      if (ky >= P0 - hc) col[ky - (P0 - C0)] = v[r];
+    }
+  });
 }
 
 __global__ void k_frame_sums(FrameSrc f, double* __restrict__ sums) {
@@ -201,8 +210,8 @@ template <int P, int FR>
 static int launch_rows_v(const FrameSrc& f, const float* mask, const double* mean_sub, double inv_area,
                          int frame0, int nfr, int mode, int rows, int cols, int C1, int K4, int H4,
                          float2* RU, float2* RV, const float2* tw, cudaStream_t st) {
-  constexpr int T = fft_threads(P, FR);
-  const size_t smem = (size_t)FR * ld_of(P) * sizeof(float2);
+  constexpr int T = ip_threads(P, FR);
+  const size_t smem = (size_t)FR * ip_ld(P, FR) * sizeof(float2);
   ZR_TRY(cuda_check(cudaFuncSetAttribute(k_fwd_rows<P, FR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                     "k_fwd_rows attr"));
   k_fwd_rows<P, FR><<<dim3(nfr, (rows + FR - 1) / FR), T, smem, st>>>(f, mask, mean_sub, inv_area, frame0, mode,
@@ -214,20 +223,22 @@ template <int P>
 static int launch_rows(const FrameSrc& f, const float* mask, const double* mean_sub, double inv_area,
                        int frame0, int nfr, int mode, int rows, int cols, int C1, int K4, int H4,
                        float2* RU, float2* RV, const float2* tw, cudaStream_t st) {
+  // 6144-point rows: at most two fit a CTA's shared memory and registers
+  constexpr int MOST = fr_default(P);
   switch (tune_get(TUNE_FWD_ROWS, P)) {
     case 1: return launch_rows_v<P, 1>(f, mask, mean_sub, inv_area, frame0, nfr, mode, rows, cols, C1, K4, H4, RU, RV, tw, st);
-    case 4: return launch_rows_v<P, 4>(f, mask, mean_sub, inv_area, frame0, nfr, mode, rows, cols, C1, K4, H4, RU, RV, tw, st);
+    case 2: return launch_rows_v<P, 2>(f, mask, mean_sub, inv_area, frame0, nfr, mode, rows, cols, C1, K4, H4, RU, RV, tw, st);
     default:
-      return launch_rows_v<P, FR_DEFAULT>(f, mask, mean_sub, inv_area, frame0, nfr, mode, rows, cols, C1, K4, H4, RU,
-                                          RV, tw, st);
+      return launch_rows_v<P, MOST>(f, mask, mean_sub, inv_area, frame0, nfr, mode, rows, cols, C1, K4, H4, RU, RV, tw,
+                                    st);
   }
 }
 
 template <int P, int FC>
 static int launch_cols_v(const float2* RU, const float2* RV, int rows, int C0, int K4, int H4, long long se,
                          int nfr, int nz, float2* G, float2* S, const float2* tw, cudaStream_t st) {
-  constexpr int T = fft_threads(P, FC);
-  const size_t smem = (size_t)FC * ld_of(P) * sizeof(float2);
+  constexpr int T = ip_threads(P, FC);
+  const size_t smem = (size_t)FC * ip_ld(P, FC) * sizeof(float2);
   ZR_TRY(cuda_check(cudaFuncSetAttribute(k_fwd_cols<P, FC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                     "k_fwd_cols attr"));
   k_fwd_cols<P, FC><<<dim3(K4 / FC, nfr, nz), T, smem, st>>>(RU, RV, rows, C0, K4, H4, se, G, S, tw);
@@ -239,7 +250,7 @@ static int launch_cols(const float2* RU, const float2* RV, int rows, int C0, int
                        int nfr, int nz, float2* G, float2* S, const float2* tw, cudaStream_t st) {
   switch (tune_get(TUNE_FWD_COLS, P)) {
     case 1: return launch_cols_v<P, 1>(RU, RV, rows, C0, K4, H4, se, nfr, nz, G, S, tw, st);
-    case 4: return launch_cols_v<P, 4>(RU, RV, rows, C0, K4, H4, se, nfr, nz, G, S, tw, st);
+    case 4: return launch_cols_v<P, fr_default(P)>(RU, RV, rows, C0, K4, H4, se, nfr, nz, G, S, tw, st);
     default: return launch_cols_v<P, FC_DEFAULT>(RU, RV, rows, C0, K4, H4, se, nfr, nz, G, S, tw, st);
   }
 }

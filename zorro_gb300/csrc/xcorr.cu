@@ -23,29 +23,17 @@
 // is DenomB point-reflected: one transform per frame gives both, over the
 // (w+1) x (w+1) window [-maxShift, maxShift]^2 that the reflection needs.
 #include "common.cuh"
+#include "fft_inplace.cuh"
 #include "internal.h"
 
 namespace zr {
 
-// Column pass: columns per CTA (by default fewer for the long 3072 and 4096
-// columns; the planner may choose 1, 2 or 4 per length) and threads
-// (ZR_XC_EPT elements per thread and pass).
-#ifndef ZR_XC_EPT
-#define ZR_XC_EPT 32
-#endif
-#ifndef ZR_XC_MINB
-#define ZR_XC_MINB 2
-#endif
-__host__ __device__ constexpr int xc_nbc_default(int C0) { return C0 >= 3072 ? 1 : 4; }
-__host__ __device__ constexpr int xc_threads(int C0, int NBC) { return fft_threads(C0, NBC, ZR_XC_EPT); }
-// Row pass: packed row pairs per CTA (default 2; the planner may choose 1,
-// 2 or 4), elements per thread and pass
-#ifndef ZR_XR_EPT
-#define ZR_XR_EPT 32
-#endif
+// Column pass: columns per CTA (by default four, which write whole sectors of
+// the window rows, and two of the long 3072 and 4096 columns; the planner may
+// choose 1, 2 or 4 per length).  Row pass: packed row pairs per CTA (default
+// 2; the planner may choose 1, 2 or 4).
+__host__ __device__ constexpr int xc_nbc_default(int C0) { return C0 >= 3072 ? 2 : 4; }
 constexpr int XC_NBR_DEFAULT = 2;
-__host__ __device__ constexpr int xr_threads(int C1, int NBR) { return fft_threads(C1, NBR, ZR_XR_EPT); }
-__host__ __device__ constexpr int xr_minb(int T) { return sm_minb(T); }
 
 struct XcJobs {
   const void* G;     // spectra: float2, or __half2 when ``sc`` is set
@@ -122,21 +110,17 @@ __device__ __forceinline__ float2 xc_product(const E* a, const E* b, int row, in
 // Column pass: CTA (job, column group) transforms NBC columns of the
 // job's product.  Jobs vary fastest across the grid, so the CTAs resident at
 // one time read the same columns of every spectrum and share them through L2.
-// The first radix-16 pass forms the products while it loads its butterflies
-// from the (column-major) spectra, so no product buffer passes through shared
-// memory; the other passes run in shared memory, and the window rows
-// [-maxShift, ...) of the result are kept.
-template <int C0, typename E, int NBC>
-__global__ void __launch_bounds__(xc_threads(C0, NBC), ZR_XC_MINB)
+// The first FFT pass forms the products while it loads its butterflies from
+// the (column-major) spectra.  The last pass computes the window rows
+// [-maxShift, ...) alone: a window of at most NS rows takes at most one
+// output of each RL-point butterfly, so it sums the twiddled inputs of those
+// (PRUNED); a wider one (whole planes) runs the full butterflies.
+template <int C0, typename E, int NBC, bool PRUNED>
+__global__ void __launch_bounds__(ip_threads(C0, NBC), sm_minb(ip_threads(C0, NBC)))
     k_xc_cols(XcJobs J, int C1, int K4, int mS, float2* __restrict__ Tw, const float2* __restrict__ tw) {
-  constexpr int T = xc_threads(C0, NBC);
-  constexpr int LD = ld_of(C0);
+  constexpr int T = ip_threads(C0, NBC);
+  using P = Ip<C0>;
   constexpr int RP = C0 + 4;  // column pitch of the spectra
-  constexpr int R = fft_radix(C0);
-  constexpr int LR = C0 / R;
-  constexpr int NBF = NBC * LR;
-  constexpr int K = (NBF + T - 1) / T;
-  static_assert(R < C0, "at least two passes");
   extern __shared__ float2 sm[];
   const int k0 = blockIdx.y * NBC;
   const int jl = blockIdx.x;
@@ -144,66 +128,62 @@ __global__ void __launch_bounds__(xc_threads(C0, NBC), ZR_XC_MINB)
   float us;
   job_operands(J, J.job0 + jl, A, B, us);
   const int half = C1 / 2;
-  float2 v[K][R];
+  ip_pass1<C0, NBC, T, 1, false>(sm, [&](int b, int j, float2* v) {
+    const int k = k0 + b;
+    const E* a = A + (size_t)k * RP;
+    const E* bb = B + (size_t)k * RP;
+    if (k < half) {
+      // every load of the butterfly first (all in bounds), then the products
+      E av[16], bv[16];
 #pragma unroll
-  for (int i = 0; i < K; i++) {
-    const int bf = threadIdx.x + i * T;
-    if ((NBF % T) == 0 || bf < NBF) {
-      const int b = bf / LR, j = bf - b * LR;
-      const int k = k0 + b;
-      const E* a = A + (size_t)k * RP;
-      const E* bb = B + (size_t)k * RP;
-      if (k < half) {
-        // every load of the butterfly first (all in bounds), then the products
-        E av[R], bv[R];
-#pragma unroll
-        for (int r = 0; r < R; r++) {
-          av[r] = __ldg(a + j + r * LR);
-          bv[r] = __ldg(bb + j + r * LR);
-        }
-#pragma unroll
-        for (int r = 0; r < R; r++) {
-          float2 h = cmulc(to_f2(av[r]), to_f2(bv[r]));
-          if (k > 0 && j + r * LR == C0 / 2) {  // row -C0/2: average with the +C0/2 product
-            const float2 h2 = cmulc(load_one(a + C0), load_one(bb + C0));
-            h = make_float2(0.5f * (h.x + h2.x), 0.5f * (h.y + h2.y));
-          }
-          if (sizeof(E) != sizeof(float2)) h = cscale(h, us);  // undo the power-of-two scales (exact)
-          v[i][r] = h;
-        }
-      } else {
-#pragma unroll
-        for (int r = 0; r < R; r++) v[i][r] = xc_product<C0>(a, bb, j + r * LR, k, half, us);
+      for (int r = 0; r < 16; r++) {
+        av[r] = __ldg(a + j + r * P::A1);
+        bv[r] = __ldg(bb + j + r * P::A1);
       }
-      dft<R, 1>(v[i]);
-    }
-  }
 #pragma unroll
-  for (int i = 0; i < K; i++) {
-    const int bf = threadIdx.x + i * T;
-    if ((NBF % T) == 0 || bf < NBF) {
-      const int b = bf / LR, j = bf - b * LR;
+      for (int r = 0; r < 16; r++) {
+        float2 h = cmulc(to_f2(av[r]), to_f2(bv[r]));
+        if (k > 0 && r == 8 && j == 0) {  // row -C0/2: average with the +C0/2 product
+          const float2 h2 = cmulc(load_one(a + C0), load_one(bb + C0));
+          h = make_float2(0.5f * (h.x + h2.x), 0.5f * (h.y + h2.y));
+        }
+        if (sizeof(E) != sizeof(float2)) h = cscale(h, us);  // undo the power-of-two scales (exact)
+        v[r] = h;
+      }
+    } else {
 #pragma unroll
-      for (int r = 0; r < R; r++) sm[b * LD + pidx(j * R + r)] = v[i][r];
+      for (int r = 0; r < 16; r++) v[r] = xc_product<C0>(a, bb, j + r * P::A1, k, half, us);
     }
-  }
+  });
   __syncthreads();
+  ip_pass2<C0, NBC, T, 1, false>(sm, tw);
   const int rows = J.rows;
-  float2* out = Tw + (size_t)jl * rows * K4;
-  fft_pass<C0, NBC, T, 1, R>(sm, tw);
-  for (int e = threadIdx.x; e < rows * NBC; e += T) {
-    const int a = e / NBC, c = e - a * NBC;
-    const int y = a < mS ? a - mS + C0 : a - mS;
-    out[(size_t)a * K4 + k0 + c] = sm[c * LD + pidx(y)];
+  float2* out = Tw + (size_t)jl * rows * K4 + k0;
+  if (PRUNED) {
+    for (int e = threadIdx.x; e < rows * NBC; e += T) {
+      const int a = e / NBC, c = e - a * NBC;
+      out[(size_t)a * K4 + c] = ip_last_one<C0, NBC, 1>(sm, c, a - mS, tw);
+    }
+  } else {
+    ip_last<C0, NBC, T, 1, true>(sm, tw, [&](int c, int k, const float2* v) {
+#pragma unroll
+      for (int r = 0; r < P::RL; r++) {  // y = k + r NS or that less C0 (both when 2 maxShift = C0)
+        const int a0 = k + r * P::NS + mS, a1 = a0 - C0;
+        if (a0 < rows) out[(size_t)a0 * K4 + c] = v[r];
+        if (a1 >= 0) out[(size_t)a1 * K4 + c] = v[r];
+      }
+    });
   }
 }
 
-template <int C1, int XC_NBR>
-__global__ void __launch_bounds__(xr_threads(C1, XC_NBR), xr_minb(xr_threads(C1, XC_NBR)))
+// Row pass: NBR pairs of window rows per CTA, each pair one complex inverse
+// FFT; the last pass is pruned to the window columns like the column pass's.
+template <int C1, int XC_NBR, bool PRUNED>
+__global__ void __launch_bounds__(ip_threads(C1, XC_NBR), sm_minb(ip_threads(C1, XC_NBR)))
     k_xc_rows(XcJobs J, int C0, int K4, int mS, float scale, const float2* __restrict__ Tw,
               const float* __restrict__ terms, float* __restrict__ out, const float2* __restrict__ tw) {
-  constexpr int T = xr_threads(C1, XC_NBR);
-  constexpr int LD = ld_of(C1);
+  constexpr int T = ip_threads(C1, XC_NBR);
+  using P = Ip<C1>;
   extern __shared__ float2 sm[];
   const int w = 2 * mS;
   const int rows = J.rows;  // w + 1 for the frame terms (rows and columns -mS..mS)
@@ -211,20 +191,20 @@ __global__ void __launch_bounds__(xr_threads(C1, XC_NBR), xr_minb(xr_threads(C1,
   const int job = J.job0 + jl;
   const int arow0 = blockIdx.x * (2 * XC_NBR);
   const float2* src = Tw + (size_t)jl * rows * K4;
-  block_fft_from<C1, XC_NBR, T, 1>(sm, tw, [&](int p, int i) {
+  ip_pass1<C1, XC_NBR, T, 1, false>(sm, [&](int p, int j, float2* v) {
     const int a0 = arow0 + 2 * p, a1 = a0 + 1;
-    return packed_rows<C1>(a0 < rows ? src + (size_t)a0 * K4 : nullptr, a1 < rows ? src + (size_t)a1 * K4 : nullptr, i);
+    const float2* r0 = a0 < rows ? src + (size_t)a0 * K4 : nullptr;
+    const float2* r1 = a1 < rows ? src + (size_t)a1 * K4 : nullptr;
+#pragma unroll
+    for (int r = 0; r < 16; r++) v[r] = packed_rows<C1>(r0, r1, j + r * P::A1);
   });
+  __syncthreads();
+  ip_pass2<C1, XC_NBR, T, 1, false>(sm, tw);
   const size_t w2 = (size_t)w * w;
   const int cols = rows;  // the terms window is square, w + 1 wide
-  for (int e = threadIdx.x; e < XC_NBR * 2 * cols; e += T) {
-    const int q = e / cols, b = e - q * cols;
-    const int p = q >> 1;
-    const int a = arow0 + q;
-    if (a >= rows) continue;
-    const int x = b < mS ? b - mS + C1 : b - mS;
-    const float2 yv = sm[p * LD + pidx(x)];
-    const float v = ((q & 1) ? yv.y : yv.x) * scale;
+  auto emit = [&](int a, int b, float v) {  // window element (a, b)
+    if (a >= rows) return;
+    v *= scale;
     const size_t pix = (size_t)a * w + b;
     if (J.kind == 0) {
       // output slots: CorrTM [0,N), CorrBM [N,2N), DenomT [2N,3N), DenomB [3N,4N), maskProduct 4N
@@ -248,57 +228,73 @@ __global__ void __launch_bounds__(xr_threads(C1, XC_NBR), xr_minb(xr_threads(C1,
       den = (den < 1.0f) ? 1.0f : den;  // np.clip(Denom, 1, inf); NaN stays NaN
       out[(size_t)job * w2 + pix] = (v - ctm * cbm / mp) / den;
     }
+  };
+  if (!PRUNED) {
+    ip_last_inplace<C1, XC_NBR, T, 1>(sm, tw);
+    __syncthreads();
+  }
+  for (int e = threadIdx.x; e < XC_NBR * cols; e += T) {
+    const int p = e / cols, b = e - p * cols;
+    const int x = b - mS;
+    const float2 v = PRUNED ? ip_last_one<C1, XC_NBR, 1>(sm, p, x, tw)
+                            : sm[p * ip_ld(C1, XC_NBR) + ip_at<C1>(x < 0 ? x + C1 : x)];
+    emit(arow0 + 2 * p, b, v.x);
+    emit(arow0 + 2 * p + 1, b, v.y);
   }
 }
 
-template <int C0, typename E, int NBC>
+template <int C0, typename E, int NBC, bool PRUNED>
 static int launch_xc_cols_t(const XcJobs& J, int nj, int C1, int K4, int mS, float2* Tw, const float2* tw,
                             cudaStream_t st) {
-  constexpr int T = xc_threads(C0, NBC);
-  const size_t smem = (size_t)NBC * ld_of(C0) * sizeof(float2);
-  ZR_TRY(cuda_check(cudaFuncSetAttribute(k_xc_cols<C0, E, NBC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem), "k_xc_cols attr"));
-  k_xc_cols<C0, E, NBC><<<dim3(nj, K4 / NBC), T, smem, st>>>(J, C1, K4, mS, Tw, tw);
+  constexpr int T = ip_threads(C0, NBC);
+  const size_t smem = (size_t)NBC * ip_ld(C0, NBC) * sizeof(float2);
+  const auto kern = k_xc_cols<C0, E, NBC, PRUNED>;
+  ZR_TRY(cuda_check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+                    "k_xc_cols attr"));
+  kern<<<dim3(nj, K4 / NBC), T, smem, st>>>(J, C1, K4, mS, Tw, tw);
   return launched("k_xc_cols");
 }
 
-template <int C0, typename E>
-static int launch_xc_cols_e(const XcJobs& J, int nj, int C1, int K4, int mS, float2* Tw, const float2* tw,
-                            cudaStream_t st) {
-  switch (tune_get(TUNE_XC_COLS, C0)) {
-    case 1: return launch_xc_cols_t<C0, E, 1>(J, nj, C1, K4, mS, Tw, tw, st);
-    case 2: return launch_xc_cols_t<C0, E, 2>(J, nj, C1, K4, mS, Tw, tw, st);
-    case 4: return launch_xc_cols_t<C0, E, 4>(J, nj, C1, K4, mS, Tw, tw, st);
-    default: return launch_xc_cols_t<C0, E, xc_nbc_default(C0)>(J, nj, C1, K4, mS, Tw, tw, st);
-  }
-}
-
+// The planner's choices of columns per CTA apply to the float32 spectra's
+// pruned windows, which are what it measures.
 template <int C0>
 static int launch_xc_cols(const XcJobs& J, int nj, int C1, int K4, int mS, float2* Tw, const float2* tw,
                           cudaStream_t st) {
-  if (J.sc) return launch_xc_cols_e<C0, __half2>(J, nj, C1, K4, mS, Tw, tw, st);
-  return launch_xc_cols_e<C0, float2>(J, nj, C1, K4, mS, Tw, tw, st);
+  constexpr int D = xc_nbc_default(C0);
+  const bool pruned = J.rows <= Ip<C0>::NS;
+  if (J.sc)
+    return pruned ? launch_xc_cols_t<C0, __half2, D, true>(J, nj, C1, K4, mS, Tw, tw, st)
+                  : launch_xc_cols_t<C0, __half2, D, false>(J, nj, C1, K4, mS, Tw, tw, st);
+  if (!pruned) return launch_xc_cols_t<C0, float2, D, false>(J, nj, C1, K4, mS, Tw, tw, st);
+  switch (tune_get(TUNE_XC_COLS, C0)) {
+    case 1: return launch_xc_cols_t<C0, float2, 1, true>(J, nj, C1, K4, mS, Tw, tw, st);
+    case 2: return launch_xc_cols_t<C0, float2, 2, true>(J, nj, C1, K4, mS, Tw, tw, st);
+    case 4: return launch_xc_cols_t<C0, float2, 4, true>(J, nj, C1, K4, mS, Tw, tw, st);
+    default: return launch_xc_cols_t<C0, float2, D, true>(J, nj, C1, K4, mS, Tw, tw, st);
+  }
 }
 
-template <int C1, int NBR>
+template <int C1, int NBR, bool PRUNED>
 static int launch_xc_rows_v(const XcJobs& J, int nj, int C0, int K4, int mS, float scale, const float2* Tw,
                             const float* terms, float* out, const float2* tw, cudaStream_t st) {
-  constexpr int T = xr_threads(C1, NBR);
-  const size_t smem = (size_t)NBR * ld_of(C1) * sizeof(float2);
-  ZR_TRY(cuda_check(cudaFuncSetAttribute(k_xc_rows<C1, NBR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+  constexpr int T = ip_threads(C1, NBR);
+  const size_t smem = (size_t)NBR * ip_ld(C1, NBR) * sizeof(float2);
+  const auto kern = k_xc_rows<C1, NBR, PRUNED>;
+  ZR_TRY(cuda_check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                     "k_xc_rows attr"));
-  k_xc_rows<C1, NBR><<<dim3((J.rows + 2 * NBR - 1) / (2 * NBR), nj), T, smem, st>>>(J, C0, K4, mS, scale, Tw,
-                                                                                   terms, out, tw);
+  kern<<<dim3((J.rows + 2 * NBR - 1) / (2 * NBR), nj), T, smem, st>>>(J, C0, K4, mS, scale, Tw, terms, out, tw);
   return launched("k_xc_rows");
 }
 
 template <int C1>
 static int launch_xc_rows(const XcJobs& J, int nj, int C0, int K4, int mS, float scale, const float2* Tw,
                           const float* terms, float* out, const float2* tw, cudaStream_t st) {
+  constexpr int D = XC_NBR_DEFAULT;
+  if (J.rows > Ip<C1>::NS) return launch_xc_rows_v<C1, D, false>(J, nj, C0, K4, mS, scale, Tw, terms, out, tw, st);
   switch (tune_get(TUNE_XC_ROWS, C1)) {
-    case 1: return launch_xc_rows_v<C1, 1>(J, nj, C0, K4, mS, scale, Tw, terms, out, tw, st);
-    case 4: return launch_xc_rows_v<C1, 4>(J, nj, C0, K4, mS, scale, Tw, terms, out, tw, st);
-    default: return launch_xc_rows_v<C1, XC_NBR_DEFAULT>(J, nj, C0, K4, mS, scale, Tw, terms, out, tw, st);
+    case 1: return launch_xc_rows_v<C1, 1, true>(J, nj, C0, K4, mS, scale, Tw, terms, out, tw, st);
+    case 4: return launch_xc_rows_v<C1, 4, true>(J, nj, C0, K4, mS, scale, Tw, terms, out, tw, st);
+    default: return launch_xc_rows_v<C1, D, true>(J, nj, C0, K4, mS, scale, Tw, terms, out, tw, st);
   }
 }
 
