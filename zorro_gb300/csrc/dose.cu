@@ -13,7 +13,10 @@
 // output rows and the final row pass packs two rows per complex inverse FFT.
 #include <math.h>
 
+#include <type_traits>
+
 #include "common.cuh"
+#include "fft_inplace.cuh"
 #include "internal.h"
 
 namespace zr {
@@ -37,43 +40,54 @@ __device__ __forceinline__ int sym_idx(int i, int n) {
 }
 
 template <int P1>
-__global__ void __launch_bounds__(fft_threads(P1, ds_nbr(P1)), ds_minb(fft_threads(P1, ds_nbr(P1))))
+__global__ void __launch_bounds__(ip_threads(P1, ds_nbr(P1)), ds_minb(ip_threads(P1, ds_nbr(P1))))
     k_dose_rows(const float* __restrict__ img, int N, int H, int W, int f0, int K4, int P0,
                 float2* __restrict__ RW, const float2* __restrict__ tw) {
-  constexpr int T = fft_threads(P1, ds_nbr(P1));
-  constexpr int LD = ld_of(P1);
+  constexpr int NB = ds_nbr(P1);
+  constexpr int T = ip_threads(P1, NB);
+  using P = Ip<P1>;
   extern __shared__ float2 sm[];
-  const int g = blockIdx.x;
+  const int y0 = blockIdx.x * NB;
   const int pl = blockIdx.y;              // frame pair within the chunk
   const int na = f0 + 2 * pl, nb = na + 1;
   const float* ia = img + (size_t)na * H * W;
   const float* ib = img + (size_t)(nb < N ? nb : na) * H * W;
-  // element x of row r: the symmetric padding of the two frames' row; every
-  // pass but the last, which pairs X[k] with X[P1 - k] in registers
-  constexpr int NB = ds_nbr(P1);
-  constexpr int RL = last_radix(P1), NSL = P1 / RL;
-  block_fft_from<P1, NB, T, -1, NSL>(sm, tw, [&](int r, int x) {
-    const int yy = g * NB + r;
-    const int ys = yy < H ? yy : (yy < 2 * H ? 2 * H - 1 - yy : sym_idx(yy, H));
-    const int xs = x < W ? x : (x < 2 * W ? 2 * W - 1 - x : sym_idx(x, W));
-    const size_t p = (size_t)ys * W + xs;
-    return make_float2(__ldg(ia + p), nb < N ? __ldg(ib + p) : 0.0f);
-  });
-  // output: column-major per frame, [frame][kx][ky]
+  // element x of row b: the symmetric padding of the two frames' row.  The
+  // first FULL of a butterfly's columns lie inside the image for every j.
+  auto rows = [&](auto full) {
+    constexpr int FULL = decltype(full)::value;
+    ip_pass1<P1, NB, T, -1, false>(sm, [&](int b, int j, float2* v) {
+      const int yy = y0 + b;
+      const int ys = yy < H ? yy : (yy < 2 * H ? 2 * H - 1 - yy : sym_idx(yy, H));
+      const size_t row = (size_t)ys * W;
+      const float *pa = ia + row, *pb = ib + row;
+#pragma unroll
+      for (int r = 0; r < 16; r++) {
+        const int x = j + r * P::A1;
+        const int xs = r < FULL || x < W ? x : (x < 2 * W ? 2 * W - 1 - x : sym_idx(x, W));
+        v[r] = make_float2(__ldg(pa + xs), nb < N ? __ldg(pb + xs) : 0.0f);
+      }
+    });
+  };
+  if (W >= 14 * P::A1) rows(std::integral_constant<int, 14>());
+  else rows(std::integral_constant<int, 0>());
+  __syncthreads();
+  ip_pass2<P1, NB, T, -1, false>(sm, tw);
+  // output: column-major per frame, [frame][kx][ky]; the last pass pairs X[k]
+  // with X[P1 - k] in registers
   const size_t fa = (size_t)(2 * pl) * K4 * P0;
   const size_t fb = fa + (size_t)K4 * P0;
-  const int y0 = g * NB;
-  fft_last_paired<P1, NB, T, -1>(sm, tw, [&](int r, int k0, const float2* x0, int k1, const float2* x1) {
+  ip_last_paired<P1, NB, T, -1>(sm, tw, [&](int r, int k0, const float2* x0, int k1, const float2* x1) {
     auto put = [&](int k, float2 zk, float2 zm) {
       const size_t o = (size_t)k * P0 + y0 + r;
       RW[fa + o] = make_float2(0.5f * (zk.x + zm.x), 0.5f * (zk.y - zm.y));
       if (nb < N) RW[fb + o] = make_float2(0.5f * (zk.y + zm.y), -0.5f * (zk.x - zm.x));
     };
 #pragma unroll
-    for (int q = 0; q < RL; q++) {
-      const int m0 = k0 + q * NSL, m1 = k1 + q * NSL;
-      if (m0 <= P1 / 2) put(m0, x0[q], k0 > 0 ? x1[RL - 1 - q] : x0[(RL - q) % RL]);
-      if (m1 <= P1 / 2) put(m1, x1[q], k0 > 0 ? x0[RL - 1 - q] : x1[RL - 1 - q]);
+    for (int q = 0; q < P::RL; q++) {
+      const int m0 = k0 + q * P::NS, m1 = k1 + q * P::NS;
+      if (m0 <= P1 / 2) put(m0, x0[q], k0 > 0 ? x1[P::RL - 1 - q] : x0[(P::RL - q) % P::RL]);
+      if (m1 <= P1 / 2) put(m1, x1[q], k0 > 0 ? x0[P::RL - 1 - q] : x1[P::RL - 1 - q]);
     }
   });
   // the pitch's columns past P1/2 are zero
@@ -107,24 +121,30 @@ __device__ __forceinline__ void dose_weight(const zr_dose_params_t& p, int P0, i
   w = thres * filt;
 }
 
+// The whole filter of 40 K2 frames went from 2708 to 2395 us with the in-place
+// transforms (fft_inplace.cuh); the row and column passes' intermediates (2.7
+// GB each way) and the 2.3 GB of frames take 1130 us of it at copy bandwidth.
+//
 // One column kx per CTA: for every frame, the column's forward FFT, times the
-// frame's filter, accumulated in registers (each thread owns P0/T rows).
-constexpr int DS_CT = 256;
+// frame's filter, accumulated in registers: thread k holds the rows k + r NS
+// that its last-pass butterfly puts out, so the spectrum is weighted and
+// summed straight from that pass.
+__host__ __device__ constexpr int ds_ct(int P0) { return P0 / ip_rl(P0) < 64 ? 64 : P0 / ip_rl(P0); }
 
 template <int P0>
-__global__ void __launch_bounds__(DS_CT, 2)
+__global__ void __launch_bounds__(ds_ct(P0), ds_minb(ds_ct(P0)))
     k_dose_cols(const float2* __restrict__ RW, int f0, int nfr, int K4, int P1, zr_dose_params_t prm,
                 const float* __restrict__ thres_q, const float* __restrict__ dose_end, int first,
                 float2* __restrict__ ACC, float* __restrict__ FM, const float2* __restrict__ tw) {
-  constexpr int LD = ld_of(P0);
-  constexpr int PER = P0 / DS_CT;
+  constexpr int T = ds_ct(P0);
+  using P = Ip<P0>;
   extern __shared__ float2 sm[];
   // per-element constants of this column: 1/critDose(q) and log2(q)
-  float* inv_crit = reinterpret_cast<float*>(sm + LD);
+  float* inv_crit = reinterpret_cast<float*>(sm + ip_ld(P0, 1));
   float* lq = inv_crit + P0;
   const int kx = blockIdx.x;
   const bool live = kx <= P1 / 2;
-  for (int y = threadIdx.x; y < P0 && live; y += DS_CT) {
+  for (int y = threadIdx.x; y < P0 && live; y += T) {
     const int fy = y < P0 / 2 ? y : y - P0;
     const float q = sqrtf((float)kx * (float)kx * (prm.inv_ps_x * prm.inv_ps_x) +
                           (float)fy * (float)fy * (prm.inv_ps_y * prm.inv_ps_y));
@@ -138,99 +158,114 @@ __global__ void __launch_bounds__(DS_CT, 2)
     inv_crit[y] = 1.0f / crit;
     lq[y] = log2f(q);
   }
-  float2 acc[PER];
-  float fm[PER];
+  const bool mine = (int)threadIdx.x < P::NS;
+  float2 acc[P::RL];
+  float fm[P::RL];
 #pragma unroll
-  for (int j = 0; j < PER; j++) {
-    const int y = threadIdx.x + j * DS_CT;
-    acc[j] = first ? make_float2(0.0f, 0.0f) : ACC[(size_t)kx * P0 + y];
-    fm[j] = (first || !prm.normalize) ? 0.0f : FM[(size_t)kx * P0 + y];
+  for (int r = 0; r < P::RL; r++) {
+    const size_t o = (size_t)kx * P0 + threadIdx.x + r * P::NS;
+    acc[r] = first || !mine ? make_float2(0.0f, 0.0f) : ACC[o];
+    fm[r] = (first || !mine || !prm.normalize) ? 0.0f : FM[o];
   }
   const float LOG2E = 1.4426950408889634f;
-  // the last pass's butterfly j = thread holds elements j + r P0/R: with
-  // P0/R = DS_CT those are exactly the thread's accumulator rows, so the
-  // spectrum is weighted and summed straight from its registers
-  constexpr bool ACC_DIRECT = P0 / last_radix(P0) == DS_CT && last_radix(P0) == PER;
   for (int nl = 0; nl < nfr; nl++) {
     const float2* col = RW + ((size_t)nl * K4 + kx) * P0;
     // filt = exp(-0.5 D / crit), thres = exp(-(q / thresQ)^order)
     const float cd = (-0.5f * dose_end[f0 + nl]) * LOG2E;
     const float ltq = log2f(thres_q[f0 + nl]);
-    auto accumulate = [&](int j, int y, float2 F) {
-      const float filt = exp2f(cd * inv_crit[y]);
-      const float thres = exp2f(-LOG2E * exp2f(prm.cutoff_order * (lq[y] - ltq)));
-      const float w = thres * filt;
-      acc[j] = make_float2(acc[j].x + F.x * w, acc[j].y + F.y * w);
-      if (prm.normalize) fm[j] += w;
-    };
     __syncthreads();  // the previous frame's spectrum has been read
-    if constexpr (ACC_DIRECT) {
-      block_fft_from<P0, 1, DS_CT, -1>(
-          sm, tw, [&](int, int y) { return __ldg(col + y); },
-          all_out([&](int, int y, int r, float2 F) {
-            if (live) accumulate(r, y, F);
-          }));
-    } else {
-      block_fft_from<P0, 1, DS_CT, -1>(sm, tw, [&](int, int y) { return __ldg(col + y); });
-      if (!live) continue;
+    ip_pass1<P0, 1, T, -1, false>(sm, [&](int, int j, float2* v) {
 #pragma unroll
-      for (int j = 0; j < PER; j++) {
-        const int y = threadIdx.x + j * DS_CT;
-        accumulate(j, y, sm[pidx(y)]);
+      for (int r = 0; r < 16; r++) v[r] = __ldg(col + j + r * P::A1);
+    });
+    __syncthreads();
+    ip_pass2<P0, 1, T, -1, false>(sm, tw);
+    if (live && mine) {
+      float2 v[P::RL];
+      ip_last_load<P0, 1>(sm, 0, threadIdx.x, v);
+      ip_twiddle_last<P0, -1>(v, threadIdx.x, tw);
+      ip_dft<P::RL, -1>(v);
+#pragma unroll
+      for (int r = 0; r < P::RL; r++) {
+        const int y = threadIdx.x + r * P::NS;
+        const float filt = exp2f(cd * inv_crit[y]);
+        const float thres = exp2f(-LOG2E * exp2f(prm.cutoff_order * (lq[y] - ltq)));
+        const float w = thres * filt;
+        acc[r] = make_float2(acc[r].x + v[r].x * w, acc[r].y + v[r].y * w);
+        if (prm.normalize) fm[r] += w;
       }
     }
   }
+  if (!mine) return;
 #pragma unroll
-  for (int j = 0; j < PER; j++) {
-    const int y = threadIdx.x + j * DS_CT;
-    ACC[(size_t)kx * P0 + y] = acc[j];
-    if (prm.normalize) FM[(size_t)kx * P0 + y] = fm[j];
+  for (int r = 0; r < P::RL; r++) {
+    const size_t o = (size_t)kx * P0 + threadIdx.x + r * P::NS;
+    ACC[o] = acc[r];
+    if (prm.normalize) FM[o] = fm[r];
   }
 }
 
 // Inverse column pass, keeping rows [0, H).
 template <int P0>
-__global__ void __launch_bounds__(fft_threads(P0, ds_nbr(P0)), ds_minb(fft_threads(P0, ds_nbr(P0))))
+__global__ void __launch_bounds__(ip_threads(P0, ds_nbr(P0)), ds_minb(ip_threads(P0, ds_nbr(P0))))
     k_dose_icols(const float2* __restrict__ ACC, const float* __restrict__ FM, int normalize, int K4, int H,
                  float2* __restrict__ T2, const float2* __restrict__ tw) {
-  constexpr int T = fft_threads(P0, ds_nbr(P0));
-  constexpr int LD = ld_of(P0);
+  constexpr int NB = ds_nbr(P0);
+  constexpr int T = ip_threads(P0, NB);
+  using P = Ip<P0>;
   extern __shared__ float2 sm[];
-  const int k0 = blockIdx.x * ds_nbr(P0);
-  block_fft_from<P0, ds_nbr(P0), T, 1>(sm, tw, [&](int c, int y) {
-    float2 v = __ldg(ACC + (size_t)(k0 + c) * P0 + y);
-    if (normalize) {
-      const float s = 1.0f / (__ldg(FM + (size_t)(k0 + c) * P0 + y) + 1.0f);
-      v = make_float2(v.x * s, v.y * s);
+  const int k0 = blockIdx.x * NB;
+  ip_pass1<P0, NB, T, 1, false>(sm, [&](int c, int j, float2* v) {
+#pragma unroll
+    for (int r = 0; r < 16; r++) {
+      const size_t o = (size_t)(k0 + c) * P0 + j + r * P::A1;
+      v[r] = __ldg(ACC + o);
+      if (normalize) {
+        const float s = 1.0f / (__ldg(FM + o) + 1.0f);
+        v[r] = make_float2(v[r].x * s, v[r].y * s);
+      }
     }
-    return v;
   });
-  for (int e = threadIdx.x; e < H * ds_nbr(P0); e += T) {
-    const int y = e / ds_nbr(P0), c = e - y * ds_nbr(P0);
-    T2[(size_t)y * K4 + k0 + c] = sm[c * LD + pidx(y)];
-  }
+  __syncthreads();
+  ip_pass2<P0, NB, T, 1, false>(sm, tw);
+  ip_last<P0, NB, T, 1, true>(sm, tw, [&](int c, int k, const float2* v) {
+#pragma unroll
+    for (int r = 0; r < P::RL; r++) {
+      const int y = k + r * P::NS;
+      if (y < H) T2[(size_t)y * K4 + k0 + c] = v[r];
+    }
+  });
 }
 
 // Real-output inverse row pass (two rows per complex FFT), |.|, crop, scale.
 template <int P1>
-__global__ void __launch_bounds__(fft_threads(P1, 2), fft_minblocks(P1))
+__global__ void __launch_bounds__(ip_threads(P1, 2), ds_minb(ip_threads(P1, 2)))
     k_dose_irows(const float2* __restrict__ T2, int K4, int H, int W, float scale, float* __restrict__ out,
                  const float2* __restrict__ tw) {
-  constexpr int T = fft_threads(P1, 2);
-  constexpr int LD = ld_of(P1);
+  constexpr int T = ip_threads(P1, 2);
+  using P = Ip<P1>;
   extern __shared__ float2 sm[];
   const int y0 = blockIdx.x * 4;
-  block_fft_from<P1, 2, T, 1>(sm, tw, [&](int p, int i) {
+  ip_pass1<P1, 2, T, 1, false>(sm, [&](int p, int j, float2* v) {
     const int a0 = y0 + 2 * p, a1 = a0 + 1;
-    return packed_rows<P1>(a0 < H ? T2 + (size_t)a0 * K4 : nullptr, a1 < H ? T2 + (size_t)a1 * K4 : nullptr, i);
+    const float2* r0 = a0 < H ? T2 + (size_t)a0 * K4 : nullptr;
+    const float2* r1 = a1 < H ? T2 + (size_t)a1 * K4 : nullptr;
+#pragma unroll
+    for (int r = 0; r < 16; r++) v[r] = packed_rows<P1>(r0, r1, j + r * P::A1);
   });
-  for (int e = threadIdx.x; e < 4 * W; e += T) {
-    const int q = e / W, x = e - q * W;
-    const int y = y0 + q;
-    if (y >= H) continue;
-    const float2 v = sm[(q >> 1) * LD + pidx(x)];
-    out[(size_t)y * W + x] = fabsf(((q & 1) ? v.y : v.x) * scale);
-  }
+  __syncthreads();
+  ip_pass2<P1, 2, T, 1, false>(sm, tw);
+  ip_last<P1, 2, T, 1, false>(sm, tw, [&](int p, int k, const float2* v) {
+    const int y = y0 + 2 * p;
+    float* o = out + (size_t)y * W;
+#pragma unroll
+    for (int r = 0; r < P::RL; r++) {
+      const int x = k + r * P::NS;
+      if (x >= W) continue;
+      if (y < H) o[x] = fabsf(v[r].x * scale);
+      if (y + 1 < H) o[W + x] = fabsf(v[r].y * scale);
+    }
+  });
 }
 
 template <int P>
@@ -254,9 +289,9 @@ static int set_smem(const void* fn, size_t smem) {
 template <int P1>
 static int dose_rows(const float* img, int N, int H, int W, int f0, int npairs, int K4, int P0, float2* RW,
                      const float2* tw, cudaStream_t st) {
-  const size_t smem = (size_t)ds_nbr(P1) * ld_of(P1) * sizeof(float2);
+  const size_t smem = (size_t)ds_nbr(P1) * ip_ld(P1, ds_nbr(P1)) * sizeof(float2);
   ZR_TRY(set_smem<P1>((const void*)k_dose_rows<P1>, smem));
-  k_dose_rows<P1><<<dim3(P0 / ds_nbr(P1), npairs), fft_threads(P1, ds_nbr(P1)), smem, st>>>(img, N, H, W, f0, K4, P0,
+  k_dose_rows<P1><<<dim3(P0 / ds_nbr(P1), npairs), ip_threads(P1, ds_nbr(P1)), smem, st>>>(img, N, H, W, f0, K4, P0,
                                                                                             RW, tw);
   return launched("k_dose_rows");
 }
@@ -265,27 +300,27 @@ template <int P0>
 static int dose_cols(const float2* RW, int f0, int nfr, int K4, int P1, const zr_dose_params_t& prm,
                      const float* tq, const float* de, int first, float2* ACC, float* FM, const float2* tw,
                      cudaStream_t st) {
-  const size_t smem = (size_t)ld_of(P0) * sizeof(float2) + (size_t)2 * P0 * sizeof(float);
+  const size_t smem = (size_t)ip_ld(P0, 1) * sizeof(float2) + (size_t)2 * P0 * sizeof(float);
   ZR_TRY(set_smem<P0>((const void*)k_dose_cols<P0>, smem));
-  k_dose_cols<P0><<<K4, DS_CT, smem, st>>>(RW, f0, nfr, K4, P1, prm, tq, de, first, ACC, FM, tw);
+  k_dose_cols<P0><<<K4, ds_ct(P0), smem, st>>>(RW, f0, nfr, K4, P1, prm, tq, de, first, ACC, FM, tw);
   return launched("k_dose_cols");
 }
 
 template <int P0>
 static int dose_icols(const float2* ACC, const float* FM, int normalize, int K4, int H, float2* T2, const float2* tw,
                       cudaStream_t st) {
-  const size_t smem = (size_t)ds_nbr(P0) * ld_of(P0) * sizeof(float2);
+  const size_t smem = (size_t)ds_nbr(P0) * ip_ld(P0, ds_nbr(P0)) * sizeof(float2);
   ZR_TRY(set_smem<P0>((const void*)k_dose_icols<P0>, smem));
-  k_dose_icols<P0><<<K4 / ds_nbr(P0), fft_threads(P0, ds_nbr(P0)), smem, st>>>(ACC, FM, normalize, K4, H, T2, tw);
+  k_dose_icols<P0><<<K4 / ds_nbr(P0), ip_threads(P0, ds_nbr(P0)), smem, st>>>(ACC, FM, normalize, K4, H, T2, tw);
   return launched("k_dose_icols");
 }
 
 template <int P1>
 static int dose_irows(const float2* T2, int K4, int H, int W, float scale, float* out, const float2* tw,
                       cudaStream_t st) {
-  const size_t smem = (size_t)2 * ld_of(P1) * sizeof(float2);
+  const size_t smem = (size_t)2 * ip_ld(P1, 2) * sizeof(float2);
   ZR_TRY(set_smem<P1>((const void*)k_dose_irows<P1>, smem));
-  k_dose_irows<P1><<<(H + 3) / 4, fft_threads(P1, 2), smem, st>>>(T2, K4, H, W, scale, out, tw);
+  k_dose_irows<P1><<<(H + 3) / 4, ip_threads(P1, 2), smem, st>>>(T2, K4, H, W, scale, out, tw);
   return launched("k_dose_irows");
 }
 
