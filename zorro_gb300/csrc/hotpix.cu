@@ -12,25 +12,50 @@
 
 namespace zr {
 
+// A running sum of floats as an unevaluated pair hi + lo (Knuth's two-sum:
+// exact error of every addition), so that a thread's share of the float64
+// total needs no float64 operation per pixel: a converted addition a pixel
+// kept the float64 pipe (2 lanes an SM) 79 % busy and bound the frame sum.
+// The terms are scaled by 2^-10 (exact) so that no sum of a few hundred of
+// them overflows.
+struct PairSum {
+  float hi = 0.0f, lo = 0.0f;
+  __device__ __forceinline__ void add(float v) {
+    v *= 0.0009765625f;
+    const float t = __fadd_rn(hi, v), b = __fsub_rn(t, hi);
+    lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(hi, __fsub_rn(t, b)), __fsub_rn(v, b)));
+    hi = t;
+  }
+  // (an infinite or NaN sum has no error term)
+  __device__ __forceinline__ double value() const {
+    return 1024.0 * (fabsf(hi) < INFINITY ? (double)hi + (double)lo : (double)hi);
+  }
+};
+
+// Adds the CTA's share to the total.
+__device__ __forceinline__ void add_total(double part, double* __restrict__ total) {
+  for (int o = 16; o > 0; o >>= 1) part += __shfl_down_sync(0xffffffffu, part, o);
+  __shared__ double red[32];
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = part;
+  __syncthreads();
+  if (threadIdx.x == 0 && total) {
+    double v = 0.0;
+    for (int i = 0; i < (int)(blockDim.x >> 5); i++) v += red[i];
+    atomicAdd(total, v);
+  }
+}
+
 __global__ void k_gain_sum(FrameSrc f, float* __restrict__ sum, double* __restrict__ total) {
   const long long npix = (long long)f.H * f.W;
-  double part = 0.0;
+  PairSum part;
   for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < npix; p += (long long)gridDim.x * blockDim.x) {
     const int y = (int)(p / f.W), x = (int)(p - (long long)y * f.W);
     float s = 0.0f;
     for (int n = 0; n < f.N; n++) s = __fadd_rn(s, load_corrected(f, n, y, x));
     sum[p] = s;
-    part += (double)s;
+    part.add(s);
   }
-  for (int o = 16; o > 0; o >>= 1) part += __shfl_down_sync(0xffffffffu, part, o);
-  __shared__ double red[32];
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = part;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    double v = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0.0;
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    if (threadIdx.x == 0 && total) atomicAdd(total, v);
-  }
+  add_total(part.value(), total);
 }
 
 // Same sum, four pixels per thread (H*W % 4 == 0, aligned vector loads), the
@@ -41,41 +66,42 @@ constexpr int GS_FRAMES = 8;
 template <int TYPE>
 __global__ void __launch_bounds__(256, 3) k_gain_sum_q(FrameSrc f, float* __restrict__ sum, double* __restrict__ total) {
   const long long n4 = (long long)f.H * f.W / 4;
-  double part = 0.0;
+  PairSum part;
   for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < n4; q += (long long)gridDim.x * blockDim.x) {
     const long long p = 4 * q;
     float4 g = make_float4(1.f, 1.f, 1.f, 1.f);
     if (f.gain) g = __ldg(reinterpret_cast<const float4*>(f.gain + p));
     float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int n0 = 0; n0 < f.N; n0 += GS_FRAMES) {
-      uint4 r[GS_FRAMES];
+    auto add = [&](const uint4& r) {
+      float4 v = quad_value<TYPE>(r);
+      if (f.gain) v = make_float4(__fmul_rn(g.x, v.x), __fmul_rn(g.y, v.y), __fmul_rn(g.z, v.z), __fmul_rn(g.w, v.w));
+      if (f.gdiv != 0.0f)
+        v = make_float4(__fdiv_rn(v.x, f.gdiv), __fdiv_rn(v.y, f.gdiv), __fdiv_rn(v.z, f.gdiv), __fdiv_rn(v.w, f.gdiv));
+      s = make_float4(__fadd_rn(s.x, v.x), __fadd_rn(s.y, v.y), __fadd_rn(s.z, v.z), __fadd_rn(s.w, v.w));
+    };
+    uint4 r[GS_FRAMES];
+    int n0 = 0;
+    for (; n0 + GS_FRAMES <= f.N; n0 += GS_FRAMES) {
+#pragma unroll
+      for (int j = 0; j < GS_FRAMES; j++) r[j] = raw_quad<TYPE>(f.raw, (long long)(n0 + j) * f.fstride + p);
+#pragma unroll
+      for (int j = 0; j < GS_FRAMES; j++) add(r[j]);
+    }
+    if (n0 < f.N) {
 #pragma unroll
       for (int j = 0; j < GS_FRAMES; j++)  // past the last frame: a repeated load, not added
         r[j] = raw_quad<TYPE>(f.raw, (long long)min(n0 + j, f.N - 1) * f.fstride + p);
 #pragma unroll
-      for (int j = 0; j < GS_FRAMES; j++) {
-        if (n0 + j < f.N) {
-          float4 v = quad_value<TYPE>(r[j]);
-          if (f.gain) v = make_float4(__fmul_rn(g.x, v.x), __fmul_rn(g.y, v.y), __fmul_rn(g.z, v.z), __fmul_rn(g.w, v.w));
-          if (f.gdiv != 0.0f)
-            v = make_float4(__fdiv_rn(v.x, f.gdiv), __fdiv_rn(v.y, f.gdiv), __fdiv_rn(v.z, f.gdiv),
-                            __fdiv_rn(v.w, f.gdiv));
-          s = make_float4(__fadd_rn(s.x, v.x), __fadd_rn(s.y, v.y), __fadd_rn(s.z, v.z), __fadd_rn(s.w, v.w));
-        }
-      }
+      for (int j = 0; j < GS_FRAMES; j++)
+        if (n0 + j < f.N) add(r[j]);
     }
     reinterpret_cast<float4*>(sum)[q] = s;
-    part += (double)s.x + (double)s.y + (double)s.z + (double)s.w;
+    part.add(s.x);
+    part.add(s.y);
+    part.add(s.z);
+    part.add(s.w);
   }
-  for (int o = 16; o > 0; o >>= 1) part += __shfl_down_sync(0xffffffffu, part, o);
-  __shared__ double red[32];
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = part;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    double v = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0.0;
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    if (threadIdx.x == 0 && total) atomicAdd(total, v);
-  }
+  add_total(part.value(), total);
 }
 
 __global__ void k_histogram(const float* __restrict__ v, long long n, double e0, int nbins, unsigned int* __restrict__ counts) {
@@ -101,88 +127,110 @@ __global__ void k_histogram(const float* __restrict__ v, long long n, double e0,
 // (v - floor(v) is exact for every float32 except just below zero, where the
 // rounding cannot cross 1/2), and v equals the last edge exactly when that
 // index is nbins and v - floor(v) is 1/2.
-__global__ void k_histogram_half(const float* __restrict__ v, long long n, int k, int nbins,
-                                 unsigned int* __restrict__ counts) {
+// Each warp counts in one of ``copies`` histograms in shared memory, which
+// keeps the warps off each other's counters (a movie's sums fill a few tens
+// of bins), and a thread reads 16 pixels before it counts any.
+__global__ void __launch_bounds__(512) k_histogram_half(const float* __restrict__ v, long long n, int k, int nbins,
+                                                        int copies, unsigned int* __restrict__ counts) {
   extern __shared__ unsigned int hist[];
-  for (int i = threadIdx.x; i < nbins; i += blockDim.x) hist[i] = 0;
+  for (int i = threadIdx.x; i < nbins * copies; i += blockDim.x) hist[i] = 0;
   __syncthreads();
-  for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x) {
-    const float x = __ldg(v + p);
-    if (!(fabsf(x) < 1073741824.0f)) continue;  // NaN, inf and values far outside every bin
+  unsigned int* mine = hist + (threadIdx.x >> 5) % copies * nbins;
+  auto count = [&](float x) {
+    if (!(fabsf(x) < 1073741824.0f)) return;  // NaN, inf and values far outside every bin
     const float c = floorf(x);
     const float fr = x - c;
     int b = (int)c + (fr >= 0.5f ? 1 : 0) - k;
-    if (b < 0 || b > nbins) continue;
+    if (b < 0 || b > nbins) return;
     if (b == nbins) {
-      if (fr != 0.5f) continue;
+      if (fr != 0.5f) return;
       b = nbins - 1;  // the last bin is closed on the right
     }
-    atomicAdd(&hist[b], 1u);
+    atomicAdd(mine + b, 1u);
+  };
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
+  if (((uintptr_t)v & 15) == 0) {
+    const float4* q = reinterpret_cast<const float4*>(v);
+    const long long n4 = n / 4;
+    for (long long p = t; p < n4; p += 4 * step) {
+      float4 x[4];
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+        if (p + i * step < n4) x[i] = __ldg(q + p + i * step);
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+        if (p + i * step < n4) {
+          count(x[i].x);
+          count(x[i].y);
+          count(x[i].z);
+          count(x[i].w);
+        }
+    }
+    if (t < n - 4 * n4) count(__ldg(v + 4 * n4 + t));
+  } else {
+    for (long long p = t; p < n; p += step) count(__ldg(v + p));
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < nbins; i += blockDim.x)
-    if (hist[i]) atomicAdd(counts + i, hist[i]);
-}
-
-// logisticMask (written as the map a) and 1 - logisticMask; dead/hot counts.
-// The logistic exponents K (sigma - c relax), sigma = (s - mu) / sigma_fit,
-// are evaluated in float64 as one fused multiply-add each, A s + Cc with
-// A = K / sigma_fit and Cc = -K c relax - A mu folded on the host (within a
-// few units in the last float64 place of the step-by-step value; the
-// exponents are rounded to float32), or step by step as K ((s - mu) rsig -
-// c relax) when sigma_fit is 0.  The counts compare the float32 sum with
-// s_dead / s_hot, the float32 values where the float64 quotient crosses the
-// cut-offs (found on the host with the same float64 operations), which gives
-// the counts of the quotient itself without a float64 division per pixel.
-__global__ void __launch_bounds__(256) k_hot_lm(const float* __restrict__ sum, long long npix, zr_hotpix_params_t p,
-                                                double rsig, double A, double C1, double C2, float s_dead, float s_hot,
-                                                float* __restrict__ LM, float* __restrict__ CONV,
-                                                unsigned int* __restrict__ counts) {
-  unsigned int dead = 0, hot = 0;
-  const double lrel = (double)(p.cutoff_lower * p.relax), urel = (double)(p.cutoff_upper * p.relax);
-  const double K = (double)p.logistic_k;
-  const bool folded = rsig < INFINITY;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < npix; i += (long long)gridDim.x * blockDim.x) {
-    const float s = sum[i];
-    dead += s < s_dead;
-    hot += s >= s_hot;
-    float x1, x2;
-    if (folded) {
-      x1 = (float)fma(A, (double)s, C1);
-      x2 = (float)fma(A, (double)s, C2);
-    } else {
-      const double sg = ((double)s - p.mu) * rsig;
-      x1 = (float)(K * (sg - lrel));
-      x2 = (float)(K * (sg - urel));
-    }
-    const float e1 = expf(x1);
-    const float e2 = expf(x2);
-    const float s1 = 1.0f / (1.0f + e1);
-    const float lm = (1.0f - s1) / (1.0f + e2);
-    float conv;
-    if (lm < 0.5f || isinf(e2)) conv = 1.0f - lm;
-    else conv = (e2 + s1) / (1.0f + e2);
-    LM[i] = lm;
-    CONV[i] = conv;
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    dead += __shfl_down_sync(0xffffffffu, dead, o);
-    hot += __shfl_down_sync(0xffffffffu, hot, o);
-  }
-  if ((threadIdx.x & 31) == 0) {
-    if (dead) atomicAdd(counts + 0, dead);
-    if (hot) atomicAdd(counts + 1, hot);
+  for (int i = threadIdx.x; i < nbins; i += blockDim.x) {
+    unsigned int c = 0;
+    for (int j = 0; j < copies; j++) c += hist[j * nbins + i];
+    if (c) atomicAdd(counts + i, c);
   }
 }
 
 __device__ __forceinline__ int rfl(int i, int n) { return i < 0 ? -i - 1 : (i >= n ? 2 * n - i - 1 : i); }
 
-// The PSF fill of singleton outliers, the neighbourly-outlier mask and
-// neighbourFilt (zorro.py:2614-2649) for one HF_TY x HF_TX tile of the map b.
+// The logistic exponents K (sigma - c relax), sigma = (s - mu) / sigma_fit, as
+// A s + C with A = K / sigma_fit and C = -K c relax - A mu folded on the host
+// in float64.  A pixel evaluates them with A and C split into float pairs (the
+// product's and the sum's rounding errors kept: 2^-47 of the larger term,
+// before the rounding to float32 that the float64 form ends with too); a
+// float64 multiply-add and its conversions kept the float64 pipe 85 % busy.
+// Sums or constants too large for the float products go through float64, step
+// by step when sigma_fit is 0.
+struct HotConst {
+  double rsig, A, C1, C2;
+  float Ah, Al, C1h, C1l, C2h, C2l;
+  float s_max;  // |s| below which the float pairs serve (0: none)
+};
+
+__device__ __forceinline__ float pair_fma(float Ah, float Al, float Ch, float Cl, float s) {
+  const float p = __fmul_rn(Ah, s);
+  const float e = __fmaf_rn(Al, s, __fmaf_rn(Ah, s, -p));
+  const float t = __fadd_rn(p, Ch), b = __fsub_rn(t, p);
+  const float r = __fadd_rn(__fsub_rn(p, __fsub_rn(t, b)), __fsub_rn(Ch, b));
+  return __fadd_rn(t, __fadd_rn(r, __fadd_rn(e, Cl)));
+}
+
+// logisticMask and 1 - logisticMask of one pixel of the sum.
+__device__ __forceinline__ void hot_mask(float s, const zr_hotpix_params_t& p, const HotConst& h, float& lm,
+                                         float& conv) {
+  float x1, x2;
+  if (fabsf(s) < h.s_max) {
+    x1 = pair_fma(h.Ah, h.Al, h.C1h, h.C1l, s);
+    x2 = pair_fma(h.Ah, h.Al, h.C2h, h.C2l, s);
+  } else if (h.rsig < INFINITY) {
+    x1 = (float)fma(h.A, (double)s, h.C1);
+    x2 = (float)fma(h.A, (double)s, h.C2);
+  } else {
+    const double sg = ((double)s - p.mu) * h.rsig, K = (double)p.logistic_k;
+    x1 = (float)(K * (sg - (double)(p.cutoff_lower * p.relax)));
+    x2 = (float)(K * (sg - (double)(p.cutoff_upper * p.relax)));
+  }
+  const float e1 = expf(x1);
+  const float e2 = expf(x2);
+  const float s1 = 1.0f / (1.0f + e1);
+  lm = (1.0f - s1) / (1.0f + e2);
+  if (lm < 0.5f || isinf(e2)) conv = 1.0f - lm;
+  else conv = (e2 + s1) / (1.0f + e2);
+}
+
+// The maps for one tile of HF_TY x HF_TX pixels: a = logisticMask, and b, the
+// PSF fill of singleton outliers plus neighbourFilt (zorro.py:2614-2649).
 // Shared memory holds 1 - logisticMask on the tile and a two-pixel ring, the
-// per-frame mean (sum / n_frames) and the mask on a one-pixel ring; positions
-// outside the image hold the values at the reflected positions, as
-// scipy.ndimage.convolve(mode='reflect') reads them.
+// per-frame mean (sum / n_frames) and the neighbourly-outlier mask on a
+// one-pixel ring; positions outside the image hold the values at the
+// reflected positions, as scipy.ndimage.convolve(mode='reflect') reads them.
 //   b = (1 - lm) * [nom <= thres] * psf(mean),  nom = (1 - lm) * psf(1 - lm),
 // then for pixels with nom > thres the neighbour term is added: the mean of
 // the per-frame means of the in-image 3 x 3 neighbours that are not in the
@@ -190,87 +238,132 @@ __device__ __forceinline__ int rfl(int i, int n) { return i < 0 ? -i - 1 : (i >=
 // times 1 - lm, or bestMean when more than 66 % (or none but the pixel itself
 // at 0.1 %) of the window is in the mask; float32 throughout, as np.mean of
 // the float32 means and the float32 neighbourFilt array of the reference.
-// The PSF sums keep the order of a per-pixel loop (taps row by row).
-constexpr int HF_TX = 32, HF_TY = 32;
+// The PSF sums keep the order of a per-pixel loop (taps row by row); a thread
+// slides them down a strip of rows of one column.
+// The dead and hot counts compare the float32 sum with s_dead / s_hot, the
+// float32 values where the float64 quotient crosses the cut-offs (found on the
+// host with the same float64 operations).
+//
+// Fused: the mask used to be a pass of its own (139 us for a K2 frame, bound
+// by the float64 pipe) whose 1 - lm the fill read back per 32 x 32 tile (129
+// us, 83 % of issue slots); together they take 160 us.
+constexpr int HF_TX = 64, HF_TY = 32;
 constexpr int HF_CW = HF_TX + 4, HF_CH = HF_TY + 4;  // 1 - lm, two-pixel ring
 constexpr int HF_MW = HF_TX + 2, HF_MH = HF_TY + 2;  // mean and mask, one-pixel ring
+constexpr int HF_T = 256;
 
-__global__ void __launch_bounds__(256) k_hot_fill(const float* __restrict__ CONV, const float* __restrict__ sum,
-                                                  int H, int W, int nfr, zr_hotpix_params_t p,
-                                                  float* __restrict__ B, unsigned int* __restrict__ counts) {
+// 3 x 3 sums down a column: ``psf_strip`` calls f(row, sum) for rows r0 .. r0 +
+// n - 1, the sum of psf[3 a + b] src[row + 2 - a][col + 2 - b] in that order.
+template <int PITCH, typename F>
+__device__ __forceinline__ void psf_strip(const float* __restrict__ src, int r0, int n, const float (&k)[9], F f) {
+  const float* q = src + r0 * PITCH;
+  float t0 = q[2], t1 = q[1], t2 = q[0];                          // row r
+  float m0 = q[PITCH + 2], m1 = q[PITCH + 1], m2 = q[PITCH];      // row r + 1
+  for (int r = r0; r < r0 + n; r++) {
+    q = src + (r + 2) * PITCH;
+    const float u0 = q[2], u1 = q[1], u2 = q[0];
+    float c = fmaf(k[0], u0, 0.0f);
+    c = fmaf(k[1], u1, c);
+    c = fmaf(k[2], u2, c);
+    c = fmaf(k[3], m0, c);
+    c = fmaf(k[4], m1, c);
+    c = fmaf(k[5], m2, c);
+    c = fmaf(k[6], t0, c);
+    c = fmaf(k[7], t1, c);
+    c = fmaf(k[8], t2, c);
+    f(r, c);
+    t0 = m0; t1 = m1; t2 = m2;
+    m0 = u0; m1 = u1; m2 = u2;
+  }
+}
+
+__global__ void __launch_bounds__(HF_T) k_hot_maps(const float* __restrict__ sum, int H, int W, int nfr,
+                                                   zr_hotpix_params_t p, HotConst h, float s_dead, float s_hot,
+                                                   float* __restrict__ LM, float* __restrict__ B,
+                                                   unsigned int* __restrict__ counts) {
   __shared__ float cv[HF_CH][HF_CW];
   __shared__ float mn[HF_MH][HF_MW];
   __shared__ uint8_t nm[HF_MH][HF_MW];
   const int ty0 = blockIdx.y * HF_TY, tx0 = blockIdx.x * HF_TX;
   const float fn = (float)nfr;
   const float bm = (float)p.best_mean;
-  for (int e = threadIdx.x; e < HF_CH * HF_CW; e += blockDim.x) {
+  unsigned int dead = 0, hot = 0, nb = 0;
+  float k[9];
+#pragma unroll
+  for (int i = 0; i < 9; i++) k[i] = p.psf[i];
+  for (int e = threadIdx.x; e < HF_CH * HF_CW; e += HF_T) {
     const int ey = e / HF_CW, ex = e - (e / HF_CW) * HF_CW;
-    const int gy = rfl(min(ty0 + ey - 2, H + 1), H), gx = rfl(min(tx0 + ex - 2, W + 1), W);
-    cv[ey][ex] = __ldg(CONV + (size_t)gy * W + gx);
-  }
-  for (int e = threadIdx.x; e < HF_MH * HF_MW; e += blockDim.x) {
-    const int ey = e / HF_MW, ex = e - (e / HF_MW) * HF_MW;
-    const int gy = rfl(min(ty0 + ey - 1, H), H), gx = rfl(min(tx0 + ex - 1, W), W);
-    mn[ey][ex] = __ldg(sum + (size_t)gy * W + gx) / fn;
+    const int y = ty0 + ey - 2, x = tx0 + ex - 2;
+    const int gy = rfl(min(y, H + 1), H), gx = rfl(min(x, W + 1), W);
+    const size_t g = (size_t)gy * W + gx;
+    const float s = __ldg(sum + g);
+    float lm, conv;
+    hot_mask(s, p, h, lm, conv);
+    cv[ey][ex] = conv;
+    if (ey >= 1 && ey <= HF_MH && ex >= 1 && ex <= HF_MW) mn[ey - 1][ex - 1] = s / fn;
+    if (ey >= 2 && ey < HF_TY + 2 && ex >= 2 && ex < HF_TX + 2 && y < H && x < W) {
+      LM[g] = lm;
+      dead += s < s_dead;
+      hot += s >= s_hot;
+    }
   }
   __syncthreads();
   // the mask on the tile and its ring (in-image positions only)
-  for (int e = threadIdx.x; e < HF_MH * HF_MW; e += blockDim.x) {
-    const int ey = e / HF_MW, ex = e - (e / HF_MW) * HF_MW;
-    const int gy = ty0 + ey - 1, gx = tx0 + ex - 1;
-    uint8_t m = 0;
-    if (gy >= 0 && gy < H && gx >= 0 && gx < W) {
-      float cc = 0.0f;
-#pragma unroll
-      for (int a = 0; a < 3; a++)
-#pragma unroll
-        for (int b = 0; b < 3; b++) cc = fmaf(p.psf[a * 3 + b], cv[ey + 2 - a][ex + 2 - b], cc);
-      m = (cv[ey + 1][ex + 1] * cc) > p.neighbour_thres;
-    }
-    nm[ey][ex] = m;
+  constexpr int S1 = 3, N1 = (HF_MH + S1 - 1) / S1;  // strips of rows
+  for (int e = threadIdx.x; e < HF_MW * S1; e += HF_T) {
+    const int st = e / HF_MW, ex = e - st * HF_MW;
+    const int gx = tx0 + ex - 1;
+    psf_strip<HF_CW>(&cv[0][ex], st * N1, min(N1, HF_MH - st * N1), k, [&](int ey, float cc) {
+      const int gy = ty0 + ey - 1;
+      nm[ey][ex] = gy >= 0 && gy < H && gx >= 0 && gx < W && (cv[ey + 1][ex + 1] * cc) > p.neighbour_thres;
+    });
   }
   __syncthreads();
-  unsigned int nb = 0;
-  for (int e = threadIdx.x; e < HF_TY * HF_TX; e += blockDim.x) {
-    const int ly = e / HF_TX, lx = e - (e / HF_TX) * HF_TX;
-    const int y = ty0 + ly, x = tx0 + lx;
-    if (y >= H || x >= W) continue;
-    float pm = 0.0f;
-#pragma unroll
-    for (int a = 0; a < 3; a++)
-#pragma unroll
-      for (int b = 0; b < 3; b++) pm = fmaf(p.psf[a * 3 + b], mn[ly + 2 - a][lx + 2 - b], pm);
-    const float conv = cv[ly + 2][lx + 2];
-    const bool neigh = nm[ly + 1][lx + 1] != 0;
-    const float single = neigh ? 0.0f : conv;
-    float bv = single * pm;
-    if (neigh) {
-      nb++;
-      float nf;
-      if (y == 0 || x == 0) {
-        nf = bm;
-      } else {
-        const int y1 = min(y + 2, H), x1 = min(x + 2, W);
-        int cnt = 0, size = 0, nk = 0;
-        float sm = 0.0f;
-        for (int yy = y - 1; yy < y1; yy++)
-          for (int xx = x - 1; xx < x1; xx++) {
-            size++;
-            if (nm[yy - ty0 + 1][xx - tx0 + 1]) cnt++;
-            else { sm += mn[yy - ty0 + 1][xx - tx0 + 1]; nk++; }
-          }
-        // cnt / size > 0.66 or <= 0.001 as integers: with size <= 9 no ratio
-        // lies within 1/450 of 0.66, and cnt >= 1 (the pixel itself)
-        if (50 * cnt > 33 * size || 1000 * cnt <= size) nf = bm;
-        else nf = conv * (sm / (float)nk);
+  constexpr int N2 = HF_TY / (HF_T / HF_TX);  // rows a thread
+  const int lx = threadIdx.x % HF_TX, x = tx0 + lx;
+  if (x < W) {
+    const int r0 = threadIdx.x / HF_TX * N2;
+    psf_strip<HF_MW>(&mn[0][lx], r0, max(0, min(N2, H - ty0 - r0)), k, [&](int ly, float pm) {
+      const int y = ty0 + ly;
+      const float conv = cv[ly + 2][lx + 2];
+      const bool neigh = nm[ly + 1][lx + 1] != 0;
+      const float single = neigh ? 0.0f : conv;
+      float bv = single * pm;
+      if (neigh) {
+        nb++;
+        float nf;
+        if (y == 0 || x == 0) {
+          nf = bm;
+        } else {
+          const int y1 = min(y + 2, H), x1 = min(x + 2, W);
+          int cnt = 0, size = 0, nk = 0;
+          float sm = 0.0f;
+          for (int yy = y - 1; yy < y1; yy++)
+            for (int xx = x - 1; xx < x1; xx++) {
+              size++;
+              if (nm[yy - ty0 + 1][xx - tx0 + 1]) cnt++;
+              else { sm += mn[yy - ty0 + 1][xx - tx0 + 1]; nk++; }
+            }
+          // cnt / size > 0.66 or <= 0.001 as integers: with size <= 9 no ratio
+          // lies within 1/450 of 0.66, and cnt >= 1 (the pixel itself)
+          if (50 * cnt > 33 * size || 1000 * cnt <= size) nf = bm;
+          else nf = conv * (sm / (float)nk);
+        }
+        bv = bv + nf;
       }
-      bv = bv + nf;
-    }
-    B[(size_t)y * W + x] = bv;
+      B[(size_t)y * W + x] = bv;
+    });
   }
-  for (int o = 16; o > 0; o >>= 1) nb += __shfl_down_sync(0xffffffffu, nb, o);
-  if ((threadIdx.x & 31) == 0 && nb) atomicAdd(counts + 2, nb);
+  for (int o = 16; o > 0; o >>= 1) {
+    dead += __shfl_down_sync(0xffffffffu, dead, o);
+    hot += __shfl_down_sync(0xffffffffu, hot, o);
+    nb += __shfl_down_sync(0xffffffffu, nb, o);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    if (dead) atomicAdd(counts + 0, dead);
+    if (hot) atomicAdd(counts + 1, hot);
+    if (nb) atomicAdd(counts + 2, nb);
+  }
 }
 
 // The float32 value t where the float64 test pred(s) = fn((double)s) changes
@@ -346,9 +439,11 @@ extern "C" int zr_histogram(const float* values, long long n, double first_edge,
   const size_t smem = (size_t)nbins * sizeof(unsigned int);
   const double k = first_edge + 0.5;
   if (k == floor(k) && fabs(k) < 4194304.0) {
-    ZR_TRY(cuda_check(cudaFuncSetAttribute(k_histogram_half, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                      "hist attr"));
-    k_histogram_half<<<blocks, 512, smem, (cudaStream_t)stream>>>(values, n, (int)k, nbins, counts);
+    // as many copies as 48 KB of shared memory holds, one a warp at most
+    const int copies = smem * 16 <= 48 * 1024 ? 16 : (smem >= 48 * 1024 ? 1 : (int)(48 * 1024 / smem));
+    ZR_TRY(cuda_check(cudaFuncSetAttribute(k_histogram_half, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)(smem * copies)), "hist attr"));
+    k_histogram_half<<<blocks, 512, smem * copies, (cudaStream_t)stream>>>(values, n, (int)k, nbins, copies, counts);
     return launched("k_histogram_half");
   }
   ZR_TRY(cuda_check(cudaFuncSetAttribute(k_histogram, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "hist attr"));
@@ -386,20 +481,24 @@ extern "C" int zr_hotpix_maps(const float* unaligned_sum, int height, int width,
   const zr_hotpix_params_t p = *params;
   float s_dead = 0.0f, s_hot = 0.0f;
   ZR_TRY(zr_hotpix_thresholds(p.mu, p.sigma, p.cutoff_lower, p.cutoff_upper, &s_dead, &s_hot));
-  const double mu = p.mu, sigma = p.sigma;
-  const double rsig = 1.0 / sigma;
+  HotConst h;
   const double Kd = (double)p.logistic_k;
-  const double A = Kd * rsig;
-  const double C1 = -(Kd * (double)(p.cutoff_lower * p.relax)) - A * mu;
-  const double C2 = -(Kd * (double)(p.cutoff_upper * p.relax)) - A * mu;
-  const long long npix = (long long)height * width;
-  float* CONV = (float*)work;
-  int blocks = (int)((npix + 255) / 256);
-  if (blocks > 152 * 16) blocks = 152 * 16;
-  cudaStream_t st = (cudaStream_t)stream;
-  k_hot_lm<<<blocks, 256, 0, st>>>(unaligned_sum, npix, p, rsig, A, C1, C2, s_dead, s_hot, hot_a, CONV, counts3);
-  ZR_TRY(launched("k_hot_lm"));
+  h.rsig = 1.0 / p.sigma;
+  h.A = Kd * h.rsig;
+  h.C1 = -(Kd * (double)(p.cutoff_lower * p.relax)) - h.A * p.mu;
+  h.C2 = -(Kd * (double)(p.cutoff_upper * p.relax)) - h.A * p.mu;
+  auto split = [](double v, float& hi, float& lo) {
+    hi = (float)v;
+    lo = (float)(v - (double)hi);
+  };
+  split(h.A, h.Ah, h.Al);
+  split(h.C1, h.C1h, h.C1l);
+  split(h.C2, h.C2h, h.C2l);
+  // the float pairs hold their errors for |A s| and |C| well inside float's range
+  const double big = 1e18, amax = fabs(h.A);
+  h.s_max = h.rsig < INFINITY && amax < big && fabs(h.C1) < big && fabs(h.C2) < big ? 1e15f : 0.0f;
   const dim3 tiles((width + HF_TX - 1) / HF_TX, (height + HF_TY - 1) / HF_TY);
-  k_hot_fill<<<tiles, 256, 0, st>>>(CONV, unaligned_sum, height, width, n_frames, p, hot_b, counts3);
-  return launched("k_hot_fill");
+  k_hot_maps<<<tiles, HF_T, 0, (cudaStream_t)stream>>>(unaligned_sum, height, width, n_frames, p, h, s_dead, s_hot,
+                                                       hot_a, hot_b, counts3);
+  return launched("k_hot_maps");
 }
