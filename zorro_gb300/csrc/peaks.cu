@@ -18,28 +18,22 @@
 //     (zorro.py:1180-1216), or the integer fallback at the window edge.
 // Filtered values are recomputed on the fly in blocks of rows, so the CTA
 // needs only the window and one row block of shared memory.
+#include <cooperative_groups.h>
 #include <math.h>
+
+#include <type_traits>
 
 #include "common.cuh"
 #include "internal.h"
 
 namespace zr {
 
-// Threads of a peak-search CTA, and rows per thread of the vectorised filter
-// pass (register blocking of its vertical taps: the R rows of a thread share
-// each 16-byte row load).
-#ifndef ZR_PK_T
-#define ZR_PK_T 1024
-#endif
-#ifndef ZR_PK_VR
-#define ZR_PK_VR 2
-#endif
+namespace cg = cooperative_groups;
 
-constexpr int PK_T = ZR_PK_T;
+constexpr int PK_T = 1024;       // threads of a peak-search CTA
 constexpr int PK_NW = PK_T / 32;  // warps
-constexpr int PK_RB = PK_T / 64;  // rows per block of the scalar filter pass
-constexpr int PK_MAXR = 64;    // largest filter radius
-constexpr int PK_SUBR = 8;     // +/- patch half-size (zorro.py:619)
+constexpr int PK_MAXR = 64;       // largest filter radius
+constexpr int PK_SUBR = 8;        // +/- patch half-size (zorro.py:619)
 
 // The bounded Brent search's state.  It lives in shared memory and only
 // thread 0 touches it, so none of it stays in registers across the filter
@@ -50,7 +44,6 @@ struct BrentState {
 };
 
 struct PkShared {
-  double gw[2 * PK_MAXR + 1];
   alignas(16) float wy[2 * PK_MAXR + 4];  // 16-byte aligned: read four taps at a time
   alignas(16) float wx[2 * PK_MAXR + 4];
   double red[PK_NW][3];
@@ -60,11 +53,9 @@ struct PkShared {
   int wcnt[PK_NW];
   double bc[4];
   int bi[2];
-  double st_s1, st_s2;  // block totals of the filter statistics
-  float st_mx;
-  int st_n;
-  double x;             // the Brent search's next abscissa (thread 0 -> all)
+  double x;             // the Brent search's next abscissa
   int go;               // 1 while the search continues
+  int r;                // filter radius of the current sigma
   BrentState bs;        // the search's state (thread 0 only)
 };
 
@@ -77,30 +68,36 @@ __device__ __forceinline__ int reflect_idx(int i, int n) {
 }
 
 // Gaussian weights exp(-0.5 k^2 / sigma^2), normalised (double, then float).
-// Every thread computes some of the exponentials; thread 0 sums them in
-// order.  All threads must call (with the same sigma).
-__device__ int gauss_weights(double sigma, float* w, PkShared& sh) {
+// One warp calls; returns the radius.  A dependent float64 operation takes 59
+// cycles here, a division 570, a square root 590 and an exponential 1100, so
+// what counts is the length of the chain: one exponential and one division
+// for both taps +/- k, side by side on the lanes, and a shuffle tree for the
+// sum (2 r + 1 additions in a row took up to 3400 cycles).
+__device__ int gauss_weights(double sigma, float* w) {
+  const int lane = threadIdx.x & 31;
   if (!(sigma > 1e-15)) {
-    if (threadIdx.x == 0) w[0] = 1.0f;
+    if (lane == 0) w[0] = 1.0f;
     return 0;
   }
   int r = (int)(4.0 * sigma + 0.5);
   if (r > PK_MAXR) r = PK_MAXR;
   const double c = -0.5 / (sigma * sigma);
-  __syncthreads();  // a previous call may still be reading sh.gw
-  for (int i = threadIdx.x; i <= 2 * r; i += blockDim.x) {
-    const int k = i - r;
-    sh.gw[i] = exp(c * (double)k * (double)k);
+  double e[(PK_MAXR + 32) / 32], s = 0.0;
+#pragma unroll
+  for (int i = 0; i < (PK_MAXR + 32) / 32; i++) {
+    const int k = lane + 32 * i;
+    e[i] = 0.0;
+    if (32 * i <= r) {
+      e[i] = k <= r ? exp(c * (double)k * (double)k) : 0.0;
+      s += k == 0 ? e[i] : 2.0 * e[i];
+    }
   }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double s = 0.0;
-    for (int i = 0; i <= 2 * r; i++) s += sh.gw[i];
-    sh.bc[0] = s;
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+#pragma unroll
+  for (int i = 0; i < (PK_MAXR + 32) / 32; i++) {
+    const int k = lane + 32 * i;
+    if (k <= r) w[r - k] = w[r + k] = (float)(e[i] / s);
   }
-  __syncthreads();
-  const double s = sh.bc[0];
-  for (int i = threadIdx.x; i <= 2 * r; i += blockDim.x) w[i] = (float)(sh.gw[i] / s);
   return r;
 }
 
@@ -163,12 +160,9 @@ struct FiltStats {
   int n;
 };
 
-// Block totals of the per-thread filter statistics: float sums within each
-// warp (a shuffle tree), the warps' partials summed in double by warp 0 in a
-// fixed order; the count exactly, the maximum.  All threads must call; every
-// thread receives the totals.  (The float64 pipe only sees one warp's worth
-// of additions.)
-__device__ void block_stats(PkShared& sh, float s1, float s2, int cnt, float mx, FiltStats& st) {
+// Warp sums of the per-thread filter statistics (a shuffle tree in float),
+// left in shared memory for stats_total.  All threads call.
+__device__ __forceinline__ void stats_warps(PkShared& sh, float s1, float s2, int cnt, float mx) {
   for (int o = 16; o > 0; o >>= 1) {
     s1 += __shfl_down_sync(0xffffffffu, s1, o);
     s2 += __shfl_down_sync(0xffffffffu, s2, o);
@@ -177,360 +171,427 @@ __device__ void block_stats(PkShared& sh, float s1, float s2, int cnt, float mx,
   }
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (lane == 0) { sh.ws1[wid] = s1; sh.ws2[wid] = s2; sh.wcnt[wid] = cnt; sh.wmx[wid] = mx; }
-  __syncthreads();
-  if (wid == 0) {
-    double a = lane < PK_NW ? (double)sh.ws1[lane] : 0.0;
-    double b = lane < PK_NW ? (double)sh.ws2[lane] : 0.0;
-    int n = lane < PK_NW ? sh.wcnt[lane] : 0;
-    float m = lane < PK_NW ? sh.wmx[lane] : -INFINITY;
-    for (int o = 16; o > 0; o >>= 1) {
-      a += __shfl_down_sync(0xffffffffu, a, o);
-      b += __shfl_down_sync(0xffffffffu, b, o);
-      n += __shfl_down_sync(0xffffffffu, n, o);
-      m = fmaxf(m, __shfl_down_sync(0xffffffffu, m, o));
-    }
-    if (lane == 0) { sh.st_s1 = a; sh.st_s2 = b; sh.st_n = n; sh.st_mx = m; }
-  }
-  __syncthreads();
-  st.s1 = sh.st_s1;
-  st.s2 = sh.st_s2;
-  st.n = sh.st_n;
-  st.mx = sh.st_mx;
-  __syncthreads();  // the totals are read before any later call writes them
 }
 
-constexpr int PK_TX = 64;            // column lanes of the filter passes
-constexpr int PK_TY = PK_T / PK_TX;  // rows per block (== PK_RB)
-static_assert(PK_TY == PK_RB, "row block must match the thread layout");
+// Their totals, the warps' partials summed in double in a fixed order (the
+// float64 pipe only sees one warp's worth of additions).  Warp 0 calls, after
+// a barrier; lane 0 holds the result.
+__device__ __forceinline__ FiltStats stats_total(PkShared& sh) {
+  const int lane = threadIdx.x & 31;
+  FiltStats st;
+  st.s1 = lane < PK_NW ? (double)sh.ws1[lane] : 0.0;
+  st.s2 = lane < PK_NW ? (double)sh.ws2[lane] : 0.0;
+  st.n = lane < PK_NW ? sh.wcnt[lane] : 0;
+  st.mx = lane < PK_NW ? sh.wmx[lane] : -INFINITY;
+  for (int o = 16; o > 0; o >>= 1) {
+    st.s1 += __shfl_down_sync(0xffffffffu, st.s1, o);
+    st.s2 += __shfl_down_sync(0xffffffffu, st.s2, o);
+    st.n += __shfl_down_sync(0xffffffffu, st.n, o);
+    st.mx = fmaxf(st.mx, __shfl_down_sync(0xffffffffu, st.mx, o));
+  }
+  return st;
+}
 
-// Visit every filtered value of the window.  MODE 0: statistics of all
-// values.  MODE 1: masked statistics plus argmax of (mask ? f : 0).  rtab[i +
-// PK_MAXR] is the 'reflect' index of i for i in [-PK_MAXR, w + PK_MAXR).
-template <int MODE>
-__device__ void filter_pass(const float* C, float* V, const int* rtab, int w, int mS, int ry, int rx,
-                            const float* wy, const float* wx, float c, PkShared& sh, bool use_mask, FiltStats& st,
-                            float& amax, int& aidx) {
-  const int tx = threadIdx.x & (PK_TX - 1), ty = threadIdx.x / PK_TX;
-  float s1 = 0.0f, s2 = 0.0f, mx = -INFINITY;
-  float bv = -INFINITY;
-  int bi = 0x7fffffff;
-  int cnt = 0;
-  for (int y0 = 0; y0 < w; y0 += PK_RB) {
-    const int y = y0 + ty;
-    if (y < w) {
-      for (int x = tx; x < w; x += PK_TX) {
-        float acc = 0.0f;
-        if (ry == 0) {
-          acc = C[y * w + x];
-        } else if (y >= ry && y + ry < w) {
-          const float* p = C + (y - ry) * w + x;
-          for (int k = 0; k <= 2 * ry; k++) acc = fmaf(wy[k], p[k * w], acc);
-        } else {
-          const int* rt = rtab + PK_MAXR + y - ry;
-          for (int k = 0; k <= 2 * ry; k++) acc = fmaf(wy[k], C[rt[k] * w + x], acc);
+// How the window's rows are laid out over the CTAs of a window's cluster and
+// over their filter blocks, and which pixels each statistics thread sums.
+//
+// The statistics are float sums over the pixels of 1024 threads, in a fixed
+// order that is part of the results (the Brent search takes its decisions on
+// them): with w % 4 == 0 thread (ty, tx) = (t / (w/4), t % (w/4)) owns columns
+// 4 tx .. 4 tx + 3 of the rows y with y mod (2 RB) = 2 ty, 2 ty + 1 (RB = 1024
+// / (w/4)), otherwise thread (t / 64, t % 64) the columns tx + 64 i of the rows
+// y mod 16 = ty; rows ascending, then columns.  A cluster of S CTAs gives
+// each CTA a range of ty, hence runs of ``len`` rows from ``off`` in every
+// ``period`` rows.  A single CTA takes blocks of consecutive rows.
+struct PkRows {
+  int w, period, off, len;  // row of run i, place j: i period + off + j
+  int nruns, rpb;            // runs, runs per filter block
+  int ty0, nty;              // ty range of this CTA
+  int rb;                    // ty values (all CTAs)
+  int cols;                  // tx values
+  bool quad;                 // the w % 4 == 0 ownership
+  bool direct;               // a block is one period of rows, a statistics thread's pixels are
+                             // those of its horizontal unit and its neighbour's (w % 8 == 0)
+  int pad, vp;               // reflected columns on each side of V, pitch of V
+};
+
+// V rows of a filter block: at most ``ROUNDS`` horizontal units (8 columns of
+// a row) a thread, and what the shared memory beside the window holds.
+__host__ __device__ inline int pk_vrows(int w, int vp, int rounds, int vfloats) {
+  const int a = 2 * (rounds * PK_T / (2 * ((w + 7) / 8))), b = vfloats / vp;
+  return a < b ? a : b;
+}
+
+__host__ __device__ inline bool pk_quad(int w) { return (w & 3) == 0 && w >= 16 && w <= 256; }
+__host__ __device__ inline int pk_ty(int w) { return pk_quad(w) ? PK_T / (w / 4) : 16; }
+
+template <int S>
+__device__ __forceinline__ PkRows pk_rows(int w, int pad, int vfloats, int rank) {
+  PkRows L;
+  L.w = w;
+  L.quad = pk_quad(w);
+  L.rb = pk_ty(w);
+  L.cols = L.quad ? w / 4 : 64;
+  L.pad = pad;
+  L.vp = ((w + 7) & ~7) + 2 * pad + 12;
+  if (S == 1) {
+    int nr = pk_vrows(w, L.vp, 1, vfloats);
+    L.direct = L.quad && (w & 7) == 0 && nr >= min(2 * L.rb, w);
+    if (L.direct) nr = 2 * L.rb;
+    else if (nr > 8) nr &= ~7;
+    if (nr > w) nr = w;
+    L.period = L.len = nr;
+    L.off = 0;
+    L.nruns = (w + nr - 1) / nr;
+    L.rpb = 1;
+    L.ty0 = 0;
+    L.nty = L.rb;
+  } else {
+    L.direct = false;
+    const int m = L.quad ? 2 : 1;
+    L.ty0 = rank * L.rb / S;
+    L.nty = (rank + 1) * L.rb / S - L.ty0;
+    L.period = m * L.rb;
+    L.off = m * L.ty0;
+    L.len = m * L.nty;
+    L.nruns = (w + L.period - 1) / L.period;
+    const int fit = pk_vrows(w, L.vp, 2, vfloats) / (m * ((L.rb + S - 1) / S));
+    L.rpb = fit < L.nruns ? fit : L.nruns;
+  }
+  return L;
+}
+
+// R rows of one column through the vertical taps: acc[j] = sum_k wy[k]
+// C[reflect(y + j + k - r)][x], k ascending.  The thread slides a window of R
+// inputs: one 4-byte load (consecutive lanes, consecutive columns) and a
+// broadcast weight (two in one load) feed R multiply-adds.
+template <int R>
+__device__ __forceinline__ void vcol(const float* __restrict__ C, int w, int x, int y, int r,
+                                     const float* __restrict__ wy, float (&acc)[R]) {
+  static_assert(R % 2 == 0, "weights are read in pairs");
+  const int K = 2 * r + 1;
+#pragma unroll
+  for (int j = 0; j < R; j++) acc[j] = 0.0f;
+  float d[R];
+  auto taps = [&](auto in) {
+#pragma unroll
+    for (int j = 0; j < R - 1; j++) d[j] = in(j);
+    auto tap = [&](int s, int k, float wk) {
+      d[(s + R - 1) % R] = in(k + R - 1);
+#pragma unroll
+      for (int j = 0; j < R; j++) acc[j] = fmaf(wk, d[(s + j) % R], acc[j]);
+    };
+    int k = 0;
+    for (; k + R <= K; k += R) {
+#pragma unroll
+      for (int s = 0; s < R; s += 2) {
+        const float2 W = *reinterpret_cast<const float2*>(wy + k + s);
+        tap(s, k + s, W.x);
+        tap(s + 1, k + s + 1, W.y);
+      }
+    }
+#pragma unroll
+    for (int s = 0; s < R - 1; s++) {
+      if (k + s >= K) break;
+      tap(s, k + s, wy[k + s]);
+    }
+  };
+  if (y >= r && y + R - 1 + r < w) {
+    const float* p = C + (y - r) * w + x;
+    taps([&](int i) { return p[i * w]; });
+  } else if (r + R <= w) {  // one reflection at either edge
+    taps([&](int i) {
+      int q = y - r + i;
+      q = q < 0 ? -1 - q : q;
+      q = q < w ? q : 2 * w - 1 - q;
+      return C[q * w + x];
+    });
+  } else {
+    taps([&](int i) { return C[reflect_idx(y - r + i, w) * w + x]; });
+  }
+}
+
+// 8 consecutive outputs of a filtered row: p + OFF is the input of tap 0 of
+// output 0, p 16-byte aligned; taps in order.  A ring of 16 inputs in
+// registers: one 16-byte load and four broadcast weights per 32
+// multiply-adds.
+template <int OFF>
+__device__ __forceinline__ void hrow8(const float* __restrict__ p, const float* __restrict__ wx, int K, float (&f)[8]) {
+  float v[16];
+  auto load = [&](int at, const float* q) {
+    const float4 t = *reinterpret_cast<const float4*>(q);
+    v[at] = t.x;
+    v[at + 1] = t.y;
+    v[at + 2] = t.z;
+    v[at + 3] = t.w;
+  };
+  load(0, p);
+  load(4, p + 4);
+  load(8, p + 8);
+  auto taps = [&](int g, int q, float w) {  // tap 4 g + q of the ring's current turn
+#pragma unroll
+    for (int j = 0; j < 8; j++) f[j] = fmaf(w, v[(4 * g + OFF + q + j) % 16], f[j]);
+  };
+  int k = 0;
+  for (; k + 16 <= K; k += 16) {
+#pragma unroll
+    for (int g = 0; g < 4; g++) {
+      load((4 * g + 12) % 16, p + k + 4 * g + 12);
+      const float4 W = *reinterpret_cast<const float4*>(wx + k + 4 * g);
+      taps(g, 0, W.x);
+      taps(g, 1, W.y);
+      taps(g, 2, W.z);
+      taps(g, 3, W.w);
+    }
+  }
+#pragma unroll
+  for (int g = 0; g < 4; g++) {
+    if (k + 4 * g >= K) break;
+    load((4 * g + 12) % 16, p + k + 4 * g + 12);
+    const float4 W = *reinterpret_cast<const float4*>(wx + k + 4 * g);
+    const int n = K - k - 4 * g;
+    taps(g, 0, W.x);
+    if (n > 1) taps(g, 1, W.y);
+    if (n > 2) taps(g, 2, W.z);
+    if (n > 3) taps(g, 3, W.w);
+  }
+}
+
+// Vertical pass of a filter block (runs [r0, r0 + nr)) into V, with the
+// columns that the horizontal taps reach beyond the edges written as their
+// reflections.
+template <int R>
+__device__ __forceinline__ void vert_unit(const float* C, float* V, const PkRows& L, int r0, int run, int gg, int x,
+                                          int ry, int rx, const float* wy) {
+  const int w = L.w, y = (r0 + run) * L.period + L.off + gg * R;
+  if (y >= w) return;
+  float acc[R];
+  vcol<R>(C, w, x, y, ry, wy, acc);
+  float* out = V + (run * L.len + gg * R) * L.vp + L.pad + x;
+  const int n = min(R, min(L.len - gg * R, w - y));
+#pragma unroll
+  for (int j = 0; j < R; j++)
+    if (j < n) out[j * L.vp] = acc[j];
+  auto mirror = [&](int q) {  // column q holds the same values
+#pragma unroll
+    for (int j = 0; j < R; j++)
+      if (j < n) out[j * L.vp + q - x] = acc[j];
+  };
+  if (rx <= w) {
+    if (x < rx) mirror(-1 - x);
+    if (x >= w - rx) mirror(2 * w - 1 - x);
+  } else {
+    for (int m = -1 - rx / (2 * w); m <= 1 + rx / (2 * w); m++)
+      for (int h = 0; h < 2; h++) {
+        const int q = (h ? -1 - x : x) + 2 * w * m;  // reflect_idx(q) == x
+        if (q != x && q >= -rx && q < w + rx) mirror(q);
+      }
+  }
+}
+
+template <int R>
+__device__ __forceinline__ void vert_block(const float* C, float* V, const PkRows& L, int r0, int nr, int ry, int rx,
+                                           const float* wy) {
+  const int G = (L.len + R - 1) / R, units = L.w * G * nr;
+  for (int u = threadIdx.x; u < units; u += PK_T) {
+    const int g = u / L.w, x = u - g * L.w, run = g / G;
+    vert_unit<R>(C, V, L, r0, run, g - run * G, x, ry, rx, wy);
+  }
+}
+
+// Visit every filtered value of this CTA's rows.  MODE 0: statistics of all
+// values.  MODE 1: masked statistics plus the argmax of (mask ? f : 0), first
+// index on ties.  Each filter block of rows is filtered vertically into V,
+// horizontally into registers, written over V as F and summed from there by
+// the statistics threads in their own order.  Returns this statistics
+// thread's sums.
+struct PkSums {
+  float s1, s2, mx, bv;
+  int cnt, bi;
+};
+
+template <int MODE, int ROUNDS>
+__device__ PkSums filter_rows(const float* C, float* V, const PkRows& L, int mS, int ry, int rx, const float* wy,
+                              const float* wx, float c, bool use_mask) {
+  const int w = L.w, U = (w + 7) / 8, K = 2 * rx + 1, OFF = (-rx) & 3;
+  const int fp = 8 * U + 4;  // pitch of F
+  PkSums a{0.0f, 0.0f, -INFINITY, -INFINITY, 0, 0x7fffffff};
+  const int tl = threadIdx.x, tyl = tl / L.cols, tx = tl - tyl * L.cols, ty = L.ty0 + tyl;
+  const bool owner = tyl < L.nty;
+  // one pixel into the sums
+  auto add = [&](int y, int x, float v) {
+    bool in = true;
+    if (MODE == 1) {
+      const int dy = y - mS, dx = x - mS;
+      in = !use_mask || (dy * dy + dx * dx < mS * mS);
+      const float mv = in ? v : 0.0f;
+      const int idx = y * w + x;
+      if (mv > a.bv || (mv == a.bv && idx < a.bi)) { a.bv = mv; a.bi = idx; }
+      a.cnt += in;
+    }
+    if (in) {
+      const float d = v - c;
+      a.s1 += d;
+      a.s2 = fmaf(d, d, a.s2);
+      a.mx = fmaxf(a.mx, v);
+    }
+  };
+  auto horizontal = [&](int m, int x, float (&f)[8]) {
+    const float* p = V + m * L.vp + L.pad + x - rx - OFF;
+    switch (OFF) {
+      case 0: hrow8<0>(p, wx, K, f); break;
+      case 1: hrow8<1>(p, wx, K, f); break;
+      case 2: hrow8<2>(p, wx, K, f); break;
+      default: hrow8<3>(p, wx, K, f); break;
+    }
+  };
+  if (ROUNDS == 1 && L.direct) {
+    // thread t filters row 2 ty + (t & 1), columns 8 (tx / 2) .. + 7, and sums
+    // rows 2 ty, 2 ty + 1, columns 4 tx .. + 3: half of what its lane
+    // neighbour t ^ 1 holds, exchanged in registers
+    const int G = (L.len + 7) / 8;
+    const bool r8 = w * G <= PK_T;  // rows a thread filters vertically: 8, or 10 where that takes one round
+    const int vg = threadIdx.x / w, vx = threadIdx.x - vg * w;
+    const int m = 2 * ty + (tx & 1), x8 = 8 * (tx >> 1), odd = tx & 1;
+    for (int r0 = 0; r0 < L.nruns; r0++) {
+      if (r8) {
+        if (vg < G) vert_unit<8>(C, V, L, r0, 0, vg, vx, ry, rx, wy);
+      } else if (vg < (L.len + 9) / 10) {
+        vert_unit<10>(C, V, L, r0, 0, vg, vx, ry, rx, wy);
+      }
+      __syncthreads();
+      const int y0 = r0 * L.len;
+      float f[8];
+#pragma unroll
+      for (int j = 0; j < 8; j++) f[j] = 0.0f;
+      if (owner && y0 + m < w) horizontal(m, x8, f);
+      float fr[2][4];
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        const float got = __shfl_xor_sync(0xffffffffu, odd ? f[q] : f[4 + q], 1);
+        fr[0][q] = odd ? got : f[q];
+        fr[1][q] = odd ? f[4 + q] : got;
+      }
+      if (owner) {
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+          const int y = y0 + 2 * ty + j;
+          if (y >= w) break;
+#pragma unroll
+          for (int q = 0; q < 4; q++) add(y, 4 * tx + q, fr[j][q]);
         }
-        V[ty * w + x] = acc;
+      }
+      if (r0 + 1 < L.nruns) __syncthreads();  // V is read before it is written again
+    }
+    if (MODE == 0) a.cnt = threadIdx.x == 0 ? w * w : 0;
+    return a;
+  }
+  for (int r0 = 0; r0 < L.nruns; r0 += L.rpb) {
+    const int nr = min(L.rpb, L.nruns - r0);
+    // rows a thread filters vertically: what splits the runs evenly
+    const int e6 = (L.len + 5) / 6 * 6, e8 = (L.len + 7) / 8 * 8, e10 = (L.len + 9) / 10 * 10;
+    if (ROUNDS == 1 || (e8 <= e6 && e8 <= e10)) vert_block<8>(C, V, L, r0, nr, ry, rx, wy);
+    else if (e10 <= e6) vert_block<10>(C, V, L, r0, nr, ry, rx, wy);
+    else vert_block<6>(C, V, L, r0, nr, ry, rx, wy);
+    __syncthreads();
+    // unit u: row 2 (u / 2U) + (u & 1), columns 8 ((u / 2) mod U) ...: neighbouring
+    // lanes read rows whose pitch is 16 bytes mod 32, which spreads the
+    // 32-byte column steps of the others over all banks
+    const int rows = nr * L.len, units = ((rows + 1) & ~1) * U;
+    float f[ROUNDS][8];
+    auto unit = [&](int i, int& m, int& x) {
+      const int u = threadIdx.x + i * PK_T, pr = (u >> 1) / U;
+      m = 2 * pr + (u & 1);
+      x = 8 * ((u >> 1) - pr * U);
+      return u < units && m < rows;
+    };
+#pragma unroll
+    for (int i = 0; i < ROUNDS; i++) {
+      int m, x;
+#pragma unroll
+      for (int j = 0; j < 8; j++) f[i][j] = 0.0f;
+      if (unit(i, m, x)) horizontal(m, x, f[i]);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < ROUNDS; i++) {
+      int m, x;
+      if (unit(i, m, x)) {
+        float4* F = reinterpret_cast<float4*>(V + m * fp + x);
+        F[0] = make_float4(f[i][0], f[i][1], f[i][2], f[i][3]);
+        F[1] = make_float4(f[i][4], f[i][5], f[i][6], f[i][7]);
       }
     }
     __syncthreads();
-    if (y < w) {
-      const float* vr = V + ty * w;
-      for (int x = tx; x < w; x += PK_TX) {
-        float f = 0.0f;
-        if (rx == 0) {
-          f = vr[x];
-        } else if (x >= rx && x + rx < w) {
-          const float* p = vr + x - rx;
-          for (int k = 0; k <= 2 * rx; k++) f = fmaf(wx[k], p[k], f);
-        } else {
-          const int* rt = rtab + PK_MAXR + x - rx;
-          for (int k = 0; k <= 2 * rx; k++) f = fmaf(wx[k], vr[rt[k]], f);
-        }
-        bool in = true;
-        if (MODE == 1) {
-          const int dy = y - mS, dx = x - mS;
-          in = !use_mask || (dy * dy + dx * dx < mS * mS);
-          const float mv = in ? f : 0.0f;
-          const int idx = y * w + x;
-          if (mv > bv || (mv == bv && idx < bi)) { bv = mv; bi = idx; }
-        }
-        if (in) {
-          const float d = f - c;
-          s1 += d;
-          s2 = fmaf(d, d, s2);
-          mx = fmaxf(mx, f);
-          cnt++;
-        }
+    auto sum_row = [&](int y, int m) {  // row y, at row m of F
+      const float* F = V + m * fp;
+      if (L.quad) {
+        const float4 v = *reinterpret_cast<const float4*>(F + 4 * tx);
+        add(y, 4 * tx, v.x);
+        add(y, 4 * tx + 1, v.y);
+        add(y, 4 * tx + 2, v.z);
+        add(y, 4 * tx + 3, v.w);
+      } else {
+        for (int x = tx; x < w; x += 64) add(y, x, F[x]);
+      }
+    };
+    if (owner) {
+      const int per = L.quad ? 2 * L.rb : L.rb, n = L.quad ? 2 : 1;
+      if (ROUNDS == 1) {  // rows y of [y0, y1) with y mod per in n ty .. n ty + n - 1
+        const int y0 = r0 * L.len, y1 = min(w, y0 + L.len);
+        for (int yb = y0 - y0 % per; yb < y1; yb += per)
+          for (int j = 0; j < n; j++) {
+            const int y = yb + n * ty + j;
+            if (y >= y0 && y < y1) sum_row(y, y - y0);
+          }
+      } else {
+        for (int i = 0; i < nr; i++)
+          for (int j = 0; j < n; j++) {
+            const int y = (r0 + i) * per + n * ty + j;
+            if (y < w) sum_row(y, i * L.len + n * tyl + j);
+          }
       }
     }
-    __syncthreads();
+    if (r0 + L.rpb < L.nruns) __syncthreads();  // F is read before V is written again
   }
-  block_stats(sh, s1, s2, cnt, mx, st);
-  if (MODE == 1) {
-    block_argmax(sh, bv, bi);
-    amax = bv;
-    aidx = bi;
-  }
-}
-
-// The same visit for w % 4 == 0 with the work vectorised: each thread
-// filters 4 consecutive columns; the vertical taps are float4 loads, the
-// horizontal taps slide a 4-wide register window one column at a time.
-// Rows per thread of the vectorised filter pass (register blocking of the
-// vertical pass): 2 by default, which keeps a thread within the 64
-// registers of a 1024-thread CTA.  The thread layout fixes the order in
-// which the filter statistics are summed, so it is part of the results.
-__host__ __device__ constexpr int pk_vec_rows(int) { return ZR_PK_VR; }
-__host__ __device__ constexpr int pk_vec_pitch(int w) { return w + 8; }
-
-// Horizontal pass of one row for 4 consecutive outputs x0..x0+3 away from
-// the borders: 16-byte loads of the row (p = row + x0 - rx - OFF is 16-byte
-// aligned), taps in order, the same fused multiply-adds as the scalar form.
-// Taps k0..k0+3 of the four outputs from the 12 values s = (A, B, Cn) that
-// start at tap k0's first input, weights W = wx[k0..k0+3].
-template <int OFF>
-__device__ __forceinline__ void taps4(const float4& A, const float4& B, const float4& Cn, const float4& W, float& f0,
-                                      float& f1, float& f2, float& f3) {
-  const float sv[12] = {A.x, A.y, A.z, A.w, B.x, B.y, B.z, B.w, Cn.x, Cn.y, Cn.z, Cn.w};
-  const float wv[4] = {W.x, W.y, W.z, W.w};
-#pragma unroll
-  for (int q = 0; q < 4; q++) {
-    f0 = fmaf(wv[q], sv[OFF + q], f0);
-    f1 = fmaf(wv[q], sv[OFF + q + 1], f1);
-    f2 = fmaf(wv[q], sv[OFF + q + 2], f2);
-    f3 = fmaf(wv[q], sv[OFF + q + 3], f3);
-  }
-}
-
-template <int OFF>
-__device__ __forceinline__ void hrow4(const float* __restrict__ p, const float* __restrict__ wx, int rx, float& f0,
-                                      float& f1, float& f2, float& f3) {
-  const int K = 2 * rx;  // last tap
-  float4 A = *reinterpret_cast<const float4*>(p), B = *reinterpret_cast<const float4*>(p + 4);
-  int k0 = 0;
-  // eight taps a step while they are all there: no per-tap tests, the weights
-  // four at a time, the row chunks renamed rather than moved
-  for (; k0 + 7 <= K; k0 += 8) {
-    const float4 Cn = *reinterpret_cast<const float4*>(p + k0 + 8);
-    taps4<OFF>(A, B, Cn, *reinterpret_cast<const float4*>(wx + k0), f0, f1, f2, f3);
-    const float4 Dn = *reinterpret_cast<const float4*>(p + k0 + 12);
-    taps4<OFF>(B, Cn, Dn, *reinterpret_cast<const float4*>(wx + k0 + 4), f0, f1, f2, f3);
-    A = Cn;
-    B = Dn;
-  }
-  for (; k0 <= K; k0 += 4) {
-    const float4 Cn = *reinterpret_cast<const float4*>(p + k0 + 8);
-    const float sv[12] = {A.x, A.y, A.z, A.w, B.x, B.y, B.z, B.w, Cn.x, Cn.y, Cn.z, Cn.w};
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-      if (k0 + q <= K) {
-        const float wk = wx[k0 + q];
-        f0 = fmaf(wk, sv[OFF + q], f0);
-        f1 = fmaf(wk, sv[OFF + q + 1], f1);
-        f2 = fmaf(wk, sv[OFF + q + 2], f2);
-        f3 = fmaf(wk, sv[OFF + q + 3], f3);
-      }
-    }
-    A = B;
-    B = Cn;
-  }
-}
-
-__device__ __forceinline__ float4 fma4(float w, const float4& v, float4 a) {
-  a.x = fmaf(w, v.x, a.x);
-  a.y = fmaf(w, v.y, a.y);
-  a.z = fmaf(w, v.z, a.z);
-  a.w = fmaf(w, v.w, a.w);
+  if (MODE == 0) a.cnt = owner && tx == 0 && tyl == 0 && L.ty0 == 0 ? w * w : 0;
   return a;
 }
 
-// Vectorised form for w % 4 == 0: w/4 column lanes of 4 columns, RB lanes of
-// R rows each per block of RB*R rows.  The vertical pass slides over the
-// input rows once per thread (R outputs share each 16-byte row load), the
-// horizontal pass reads 16-byte chunks of the filtered rows; every output
-// still accumulates its taps in order with fmaf, as the scalar form does.
-template <int MODE, int R>
-__device__ void filter_pass4(const float* C, float* V, const int* rtab, int w, int mS, int ry, int rx,
-                             const float* wy, const float* wx, float c, PkShared& sh, bool use_mask, FiltStats& st,
-                             float& amax, int& aidx) {
-  const int w4 = w >> 2;
-  const int RB = PK_T / w4;
-  const int VP = pk_vec_pitch(w);
-  const int tx = threadIdx.x % w4, ty = threadIdx.x / w4;
-  const int x0 = tx << 2;
-  float s1 = 0.0f, s2 = 0.0f, mx = -INFINITY;
-  float bv = -INFINITY;
-  int bi = 0x7fffffff;
-  int cnt = 0;
-  const int OFF = (-rx) & 3;
-  const bool xin = (x0 >= rx && x0 + 3 + rx < w);
-  for (int yb = 0; yb < w; yb += RB * R) {
-    const int y = yb + ty * R;  // first of this thread's R rows
-    const bool act = ty < RB && y < w;
-    if (act) {
-      float4 acc[R];
-#pragma unroll
-      for (int j = 0; j < R; j++) acc[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-      const bool yin = (y >= ry && y + R - 1 + ry < w);
-      const int* rt = rtab + PK_MAXR + y - ry;
-      float wr[R];
-#pragma unroll
-      for (int j = 0; j < R; j++) wr[j] = 0.0f;
-      if (R == 2 && yin) {
-        // rows y and y + 1 away from the borders: input row y - ry + t adds
-        // wy[t] to row y and wy[t - 1] to row y + 1, taps in order (as below),
-        // two input rows a step with no per-tap tests
-        const float* pr = C + (y - ry) * w + x0;
-        const int K = 2 * ry;
-        float4 a0 = acc[0], a1 = acc[R - 1];
-        float wp = wy[0];
-        a0 = fma4(wp, *reinterpret_cast<const float4*>(pr), a0);
-        int t = 1;
-        for (; t + 1 <= K; t += 2) {
-          const float4 va = *reinterpret_cast<const float4*>(pr + t * w);
-          const float4 vb = *reinterpret_cast<const float4*>(pr + (t + 1) * w);
-          const float wa = wy[t], wb = wy[t + 1];
-          a0 = fma4(wa, va, a0);
-          a1 = fma4(wp, va, a1);
-          a0 = fma4(wb, vb, a0);
-          a1 = fma4(wa, vb, a1);
-          wp = wb;
-        }
-        if (t <= K) {
-          const float4 va = *reinterpret_cast<const float4*>(pr + t * w);
-          const float wa = wy[t];
-          a0 = fma4(wa, va, a0);
-          a1 = fma4(wp, va, a1);
-          wp = wa;
-        }
-        a1 = fma4(wp, *reinterpret_cast<const float4*>(pr + (K + 1) * w), a1);
-        acc[0] = a0;
-        acc[R - 1] = a1;
-      } else
-      for (int t = 0; t <= 2 * ry + R - 1; t++) {
-        // wr[j] = wy[t - j]
-#pragma unroll
-        for (int j = R - 1; j > 0; j--) wr[j] = wr[j - 1];
-        wr[0] = t <= 2 * ry ? wy[t] : 0.0f;
-        const int row = yin ? (y - ry + t) : rt[t];
-        const float4 v = *reinterpret_cast<const float4*>(C + row * w + x0);
-#pragma unroll
-        for (int j = 0; j < R; j++) {
-          if (t - j >= 0 && t - j <= 2 * ry) {
-            const float wk = wr[j];
-            acc[j].x = fmaf(wk, v.x, acc[j].x); acc[j].y = fmaf(wk, v.y, acc[j].y);
-            acc[j].z = fmaf(wk, v.z, acc[j].z); acc[j].w = fmaf(wk, v.w, acc[j].w);
-          }
-        }
-      }
-#pragma unroll
-      for (int j = 0; j < R; j++)
-        if (y + j < w) *reinterpret_cast<float4*>(V + (ty * R + j) * VP + x0) = acc[j];
-    }
-    __syncthreads();
-    if (act) {
-      // the horizontal taps of the thread's R rows, then their statistics
-      float fr[R][4];
-#pragma unroll
-      for (int j = 0; j < R; j++) {
-        fr[j][0] = fr[j][1] = fr[j][2] = fr[j][3] = 0.f;
-        if (y + j >= w) break;
-        const float* vr = V + (ty * R + j) * VP;
-        float& f0 = fr[j][0];
-        float& f1 = fr[j][1];
-        float& f2 = fr[j][2];
-        float& f3 = fr[j][3];
-        if (xin) {
-          const float* pp = vr + x0 - rx - OFF;
-          switch (OFF) {
-            case 0: hrow4<0>(pp, wx, rx, f0, f1, f2, f3); break;
-            case 1: hrow4<1>(pp, wx, rx, f0, f1, f2, f3); break;
-            case 2: hrow4<2>(pp, wx, rx, f0, f1, f2, f3); break;
-            default: hrow4<3>(pp, wx, rx, f0, f1, f2, f3); break;
-          }
-        } else {
-          const int* rt = rtab + PK_MAXR + x0 - rx;
-          float a0 = vr[rt[0]], a1 = vr[rt[1]], a2 = vr[rt[2]];
-          for (int k = 0; k <= 2 * rx; k++) {
-            const float a3 = vr[rt[k + 3]];
-            const float wk = wx[k];
-            f0 = fmaf(wk, a0, f0); f1 = fmaf(wk, a1, f1); f2 = fmaf(wk, a2, f2); f3 = fmaf(wk, a3, f3);
-            a0 = a1; a1 = a2; a2 = a3;
-          }
-        }
-      }
-#pragma unroll
-      for (int j = 0; j < R; j++) {
-        const int yy = y + j;
-        if (yy >= w) break;
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-          const float f = fr[j][q];
-          const int x = x0 + q;
-          bool in = true;
-          if (MODE == 1) {
-            const int dy = yy - mS, dx = x - mS;
-            in = !use_mask || (dy * dy + dx * dx < mS * mS);
-            const float mv = in ? f : 0.0f;
-            const int idx = yy * w + x;
-            if (mv > bv || (mv == bv && idx < bi)) { bv = mv; bi = idx; }
-          }
-          if (in) {
-            const float d = f - c;
-            s1 += d;
-            s2 = fmaf(d, d, s2);
-            mx = fmaxf(mx, f);
-            cnt++;
-          }
-        }
-      }
-    }
-    __syncthreads();
-  }
-  block_stats(sh, s1, s2, cnt, mx, st);
-  if (MODE == 1) {
-    block_argmax(sh, bv, bi);
-    amax = bv;
-    aidx = bi;
-  }
+// a / b from a reciprocal r of b good to a few units in the last place: the
+// quotient's remainder folded back once, which rounds it correctly.
+__device__ __forceinline__ double div_by(double a, double b, double r) {
+  const double q = a * r;
+  return fma(fma(-q, b, a), r, q);
 }
 
-template <int MODE>
-__device__ void filter_any(const float* C, float* V, const int* rtab, int w, int mS, int ry, int rx, const float* wy,
-                           const float* wx, float c, PkShared& sh, bool use_mask, FiltStats& st, float& amax,
-                           int& aidx) {
-  if ((w & 3) == 0 && w >= 16 && w <= 4 * PK_TX)
-    filter_pass4<MODE, pk_vec_rows(0)>(C, V, rtab, w, mS, ry, rx, wy, wx, c, sh, use_mask, st, amax, aidx);
-  else
-    filter_pass<MODE>(C, V, rtab, w, mS, ry, rx, wy, wx, c, sh, use_mask, st, amax, aidx);
-}
-
-// std(G_sigma * C) / (max - mean) of the filtered window (zorro.py:1108-
-// 1121).  All threads filter; the value is formed by thread 0 only (the
-// others return 0).
-__device__ double objective(const float* C, float* V, const int* rtab, int w, int mS, double sigma, float c,
-                            PkShared& sh) {
-  const int r = gauss_weights(sigma, sh.wy, sh);
-  __syncthreads();
-  FiltStats st;
-  float am;
-  int ai;
-  filter_any<0>(C, V, rtab, w, mS, r, r, sh.wy, sh.wy, c, sh, false, st, am, ai);
-  if (threadIdx.x != 0) return 0.0;
-  const double n = (double)st.n;
-  const double m1 = st.s1 / n;
-  const double var = st.s2 / n - m1 * m1;
+// std(G_sigma * C) / (max - mean) from the statistics (zorro.py:1108-1121).
+// The warp that holds them calls, lane 0 gets the value.  The square root of
+// the variance and the division by the difference start from two reciprocal
+// square roots side by side on lanes 0 and 1 (1 / |d| = rsqrt(d d)), and the
+// divisions by n (rn = 1 / n) from rn: 1400 cycles instead of four operations
+// of 570 to 590 in a row, the same roundings.
+__device__ __forceinline__ double objective(const FiltStats& st, float c, double n, double rn) {
+  const double m1 = div_by(st.s1, n, rn);
+  const double var = div_by(st.s2, n, rn) - m1 * m1;
   const double mean = (double)c + m1;
-  return sqrt(var > 0.0 ? var : 0.0) / ((double)st.mx - mean);
+  const double d = __shfl_sync(0xffffffffu, (double)st.mx - mean, 0);
+  const double v = __shfl_sync(0xffffffffu, var > 0.0 ? var : 0.0, 0);
+  const double q = rsqrt((threadIdx.x & 31) == 0 ? v : d * d);
+  const double rd = copysign(__shfl_sync(0xffffffffu, q, 1), d);
+  double sd = v * q;  // sqrt(v), one correction
+  sd = fma(fma(-sd, sd, v), 0.5 * q, sd);
+  const double f = div_by(sd, d, rd);
+  return fabs(f) < INFINITY ? f : sqrt(v) / d;  // zero, infinite or NaN terms
 }
 
 __device__ __forceinline__ double sgn1(double v) { return v > 0.0 ? 1.0 : (v < 0.0 ? -1.0 : 1.0); }
 
-// Bounded Brent minimisation (FMM FMIN).  Returns the abscissa of the best
-// value (to every thread); *nfev receives the number of function values.
-// The search's scalar state lives in thread 0, which decides each next
-// abscissa and whether to go on and hands them to the CTA through shared
-// memory; all threads evaluate the objective.
+// Bounded Brent minimisation (FMM FMIN).  The search's state lives in shared
+// memory and one thread steps it (brent_begin, brent_step): it leaves the next
+// abscissa in sh.x with sh.go = 1, or the best one with sh.go = 0 and the
+// number of function values in sh.bi[1].
+
 // Thread 0: the next abscissa of the search (sh.x, sh.go = 1), or its end
 // (sh.go = 0).
 __device__ void brent_next(BrentState& S, PkShared& sh) {
@@ -567,80 +628,57 @@ __device__ void brent_next(BrentState& S, PkShared& sh) {
   sh.go = 1;
 }
 
-// Bounded Brent minimisation (FMM FMIN).  Returns the abscissa of the best
-// value (to every thread); *nfev receives the number of function values.
-// Thread 0 runs the search (its state in shared memory), decides each next
-// abscissa and whether to go on and hands them to the CTA through shared
-// memory; all threads evaluate the objective.
-__device__ double fmin_bounded(const float* C, float* V, const int* rtab, int w, int mS, float c, PkShared& sh,
-                               double lo, double hi, double xatol, int maxfun, int* nfev) {
-  const bool lead = threadIdx.x == 0;
-  const double sqrt_eps = sqrt(2.2e-16);
-  const double golden = 0.5 * (3.0 - sqrt(5.0));
-  const double x0 = lo + golden * (hi - lo);
-  const double f0 = objective(C, V, rtab, w, mS, x0, c, sh);
-  if (lead) {
-    BrentState S;
-    S.a = lo;
-    S.b = hi;
-    S.fulc = x0;
-    S.nfc = x0;
-    S.xf = x0;
-    S.rat = 0.0;
-    S.e = 0.0;
-    S.x = x0;
-    S.fx = f0;
-    S.num = 1;
-    S.ffulc = f0;
-    S.fnfc = f0;
-    S.xm = 0.5 * (lo + hi);
-    S.tol1 = sqrt_eps * fabs(x0) + xatol / 3.0;
-    S.tol2 = 2.0 * S.tol1;
-    brent_next(S, sh);
-    if (!sh.go) {  // the search ended before its first step
-      sh.x = S.xf;
-      sh.bi[1] = S.num;
-    }
-    sh.bs = S;
+__device__ double brent_first(double lo, double hi) { return lo + 0.5 * (3.0 - sqrt(5.0)) * (hi - lo); }
+
+__device__ __forceinline__ void brent_tols(BrentState& S, double xatol3) {
+  S.tol1 = sqrt(2.2e-16) * fabs(S.xf) + xatol3;
+  S.tol2 = 2.0 * S.tol1;
+}
+
+__device__ void brent_begin(PkShared& sh, double lo, double hi, double xatol3, double x0, double f0) {
+  BrentState S;
+  S.a = lo;
+  S.b = hi;
+  S.fulc = S.nfc = S.xf = S.x = x0;
+  S.rat = S.e = 0.0;
+  S.fx = S.ffulc = S.fnfc = f0;
+  S.num = 1;
+  S.xm = 0.5 * (lo + hi);
+  brent_tols(S, xatol3);
+  brent_next(S, sh);
+  if (!sh.go) {  // the search ended before its first step
+    sh.x = S.xf;
+    sh.bi[1] = S.num;
   }
-  __syncthreads();
-  while (sh.go) {
-    const double xe = sh.x;
-    const double fu = objective(C, V, rtab, w, mS, xe, c, sh);  // barriers: every thread has read sh.x, sh.go
-    if (lead) {
-      BrentState S = sh.bs;
-      S.num += 1;
-      if (fu <= S.fx) {
-        if (S.x >= S.xf) S.a = S.xf; else S.b = S.xf;
-        S.fulc = S.nfc; S.ffulc = S.fnfc;
-        S.nfc = S.xf; S.fnfc = S.fx;
-        S.xf = S.x; S.fx = fu;
-      } else {
-        if (S.x < S.xf) S.a = S.x; else S.b = S.x;
-        if ((fu <= S.fnfc) || (S.nfc == S.xf)) {
-          S.fulc = S.nfc; S.ffulc = S.fnfc;
-          S.nfc = S.x; S.fnfc = fu;
-        } else if ((fu <= S.ffulc) || (S.fulc == S.xf) || (S.fulc == S.nfc)) {
-          S.fulc = S.x; S.ffulc = fu;
-        }
-      }
-      S.xm = 0.5 * (S.a + S.b);
-      S.tol1 = sqrt_eps * fabs(S.xf) + xatol / 3.0;
-      S.tol2 = 2.0 * S.tol1;
-      if (S.num >= maxfun) sh.go = 0;
-      else brent_next(S, sh);
-      if (!sh.go) {
-        sh.x = S.xf;
-        sh.bi[1] = S.num;
-      }
-      sh.bs = S;
+  sh.bs = S;
+}
+
+__device__ void brent_step(PkShared& sh, double xatol3, int maxfun, double fu) {
+  BrentState S = sh.bs;
+  S.num += 1;
+  if (fu <= S.fx) {
+    if (S.x >= S.xf) S.a = S.xf; else S.b = S.xf;
+    S.fulc = S.nfc; S.ffulc = S.fnfc;
+    S.nfc = S.xf; S.fnfc = S.fx;
+    S.xf = S.x; S.fx = fu;
+  } else {
+    if (S.x < S.xf) S.a = S.x; else S.b = S.x;
+    if ((fu <= S.fnfc) || (S.nfc == S.xf)) {
+      S.fulc = S.nfc; S.ffulc = S.fnfc;
+      S.nfc = S.x; S.fnfc = fu;
+    } else if ((fu <= S.ffulc) || (S.fulc == S.xf) || (S.fulc == S.nfc)) {
+      S.fulc = S.x; S.ffulc = fu;
     }
-    __syncthreads();
   }
-  const double best = sh.x;
-  *nfev = sh.bi[1];
-  __syncthreads();
-  return best;
+  S.xm = 0.5 * (S.a + S.b);
+  brent_tols(S, xatol3);
+  if (S.num >= maxfun) sh.go = 0;
+  else brent_next(S, sh);
+  if (!sh.go) {
+    sh.x = S.xf;
+    sh.bi[1] = S.num;
+  }
+  sh.bs = S;
 }
 
 // The sub-pixel step on a 16 x 16 filtered patch (zorro.py:1180-1216): its
@@ -707,19 +745,27 @@ __device__ void subpix_search(const float* patch, int sp, const float2* __restri
   block_argmax(sh, bv, bi);
 }
 
+// One window per cluster of S CTAs (S = 1: a plain CTA).  Every CTA holds the
+// whole window and filters its own rows; with S > 1 the statistics threads'
+// sums stay in the CTA that made them and CTA 0 gathers them through
+// distributed shared memory, steps the search and hands the next weights back:
+// two cluster barriers per function value.
+template <int S>
 __global__ void __launch_bounds__(PK_T, 1) k_peaks(const float* __restrict__ cwin, int mS, zr_peak_params_t p,
-                                               zr_peak_result_t* __restrict__ res, const float2* __restrict__ tw) {
-  extern __shared__ float smf[];
+                                               int pad, int vfloats, double xatol3, double rn, zr_peak_result_t* __restrict__ res,
+                                               const float2* __restrict__ tw) {
+  extern __shared__ __align__(16) float smf[];
   __shared__ PkShared sh;
   __shared__ float2 patchF[16 * 16];
-  __shared__ int rtab[2 * PK_MAXR + 2 * 112];
   const int w = 2 * mS;
   const int w2 = w * w;
+  const int win = blockIdx.x / S, rank = S > 1 ? blockIdx.x % S : 0;
+  const int warp = threadIdx.x >> 5;
   float* C = smf;
-  float* V = smf + w2;
-  const float* src = cwin + (size_t)blockIdx.x * w2;
+  float* V = smf + ((w2 + 3) & ~3);
+  const float* src = cwin + (size_t)win * w2;
   for (int e = threadIdx.x; e < w2; e += PK_T) C[e] = src[e];
-  for (int i = threadIdx.x; i < w + 2 * PK_MAXR; i += PK_T) rtab[i] = reflect_idx(i - PK_MAXR, w);
+  const PkRows lay = pk_rows<S>(w, pad, vfloats, rank);
   __syncthreads();
   const float origin = C[mS * w + mS];
   if (p.suppress_origin) {
@@ -741,26 +787,147 @@ __global__ void __launch_bounds__(PK_T, 1) k_peaks(const float* __restrict__ cwi
   // (any value near the mean serves; the statistics are exact sums around it)
   float ls = 0.0f;
   for (int e = threadIdx.x; e < w2; e += PK_T) ls += C[e];
-  FiltStats tot;
-  block_stats(sh, ls, 0.0f, 0, 0.0f, tot);
-  const float c = (float)(tot.s1 / (double)w2);
+  stats_warps(sh, ls, 0.0f, 0, 0.0f);
+  __syncthreads();
+  if (warp == 0) {
+    const FiltStats t = stats_total(sh);
+    if (threadIdx.x == 0) sh.bc[0] = t.s1;
+  }
+  __syncthreads();
+  const float c = (float)(sh.bc[0] / (double)w2);
 
-  double sigy = 0.0, sigx = 0.0, sig_opt = nan("");
+  // Statistics of one filter setting, in CTA 0 of the window: FiltStats on
+  // thread 0 of warp 0 (and, MODE 1, the argmax on every thread).
+  auto gather = [&](PkSums a, auto mode) {
+    constexpr int MODE = decltype(mode)::value;
+    if constexpr (S > 1) {
+      cg::cluster_group cl = cg::this_cluster();
+      const int nt = lay.nty * lay.cols;  // statistics threads of this CTA
+      __syncthreads();                // F has been read
+      float* Z = V;
+      if ((int)threadIdx.x < nt) {
+        Z[threadIdx.x] = a.s1;
+        Z[nt + threadIdx.x] = a.s2;
+        Z[2 * nt + threadIdx.x] = a.mx;
+        if (MODE == 1) {
+          Z[3 * nt + threadIdx.x] = a.bv;
+          Z[4 * nt + threadIdx.x] = __int_as_float(a.bi);
+          Z[5 * nt + threadIdx.x] = __int_as_float(a.cnt);
+        }
+      }
+      cl.sync();
+      if (rank != 0) return;
+      const int t = threadIdx.x, ty = t / lay.cols, tx = t - ty * lay.cols;
+      a = PkSums{0.0f, 0.0f, -INFINITY, -INFINITY, 0, 0x7fffffff};
+      if (ty < lay.rb) {
+        int o = 0;
+        while ((o + 1) * lay.rb / S <= ty) o++;  // the CTA that owns ty
+        const int t0 = o * lay.rb / S, n = ((o + 1) * lay.rb / S - t0) * lay.cols, i = (ty - t0) * lay.cols + tx;
+        const float* R = cl.map_shared_rank(V, o);
+        a.s1 = R[i];
+        a.s2 = R[n + i];
+        a.mx = R[2 * n + i];
+        if (MODE == 1) {
+          a.bv = R[3 * n + i];
+          a.bi = __float_as_int(R[4 * n + i]);
+          a.cnt = __float_as_int(R[5 * n + i]);
+        }
+      }
+      if (MODE == 0) a.cnt = t == 0 ? w2 : 0;
+    }
+    stats_warps(sh, a.s1, a.s2, a.cnt, a.mx);
+    if (MODE == 1) {
+      block_argmax(sh, a.bv, a.bi);
+      if (threadIdx.x == 0) {
+        sh.bc[1] = a.bv;
+        sh.bi[0] = a.bi;
+      }
+    }
+    __syncthreads();
+  };
+  // CTA 0's weights (wy, r and go) for every CTA of the window
+  auto share = [&]() {
+    if constexpr (S > 1) {
+      cg::cluster_group cl = cg::this_cluster();
+      cl.sync();
+      if (rank != 0) {
+        const PkShared* lead = cl.map_shared_rank(&sh, 0);
+        for (int i = threadIdx.x; i < 2 * PK_MAXR + 4; i += PK_T) {
+          sh.wy[i] = lead->wy[i];
+          sh.wx[i] = lead->wx[i];
+        }
+        if (threadIdx.x == 0) {
+          sh.r = lead->r;
+          sh.bi[0] = lead->bi[0];
+          sh.go = lead->go;
+        }
+      }
+      __syncthreads();
+    } else {
+      __syncthreads();
+    }
+  };
+  constexpr int ROUNDS = S > 1 ? 2 : 1;
+  using Mode0 = std::integral_constant<int, 0>;
+  using Mode1 = std::integral_constant<int, 1>;
+
+  double sig_opt = nan("");
   int nfev = 0;
   if (p.bmode == 1) {
-    sig_opt = fmin_bounded(C, V, rtab, w, mS, c, sh, p.opti_lo, p.opti_hi, p.opti_xatol, p.opti_maxiter, &nfev);
-    sigy = sigx = sig_opt;
-  } else if (p.bmode == 2) {
-    sigy = p.conv_sigma_y;
-    sigx = p.conv_sigma_x;
+    const double x0 = brent_first(p.opti_lo, p.opti_hi);
+    if (rank == 0 && warp == 0) {
+      const int r = gauss_weights(x0, sh.wy);
+      if (threadIdx.x == 0) {
+        sh.r = r;
+        sh.go = 1;
+      }
+    }
+    share();
+    for (bool first = true; sh.go; first = false) {
+      const int r = sh.r;
+      const PkSums a = filter_rows<0, ROUNDS>(C, V, lay, mS, r, r, sh.wy, sh.wy, c, false);
+      gather(a, Mode0());
+      if (rank == 0 && warp == 0) {
+        const FiltStats st = stats_total(sh);
+        const double f = objective(st, c, (double)w2, rn);
+        if (threadIdx.x == 0) {
+          if (first) brent_begin(sh, p.opti_lo, p.opti_hi, xatol3, x0, f);
+          else brent_step(sh, xatol3, p.opti_maxiter, f);
+        }
+        __syncwarp();
+        if (sh.go) {
+          const int rn = gauss_weights(sh.x, sh.wy);
+          if (threadIdx.x == 0) sh.r = rn;
+        }
+      }
+      share();
+    }
+    sig_opt = sh.x;  // CTA 0
+    nfev = sh.bi[1];
   }
-  const int ry = gauss_weights(sigy, sh.wy, sh);
-  const int rx = gauss_weights(sigx, sh.wx, sh);
+  if (rank == 0 && warp == 0) {
+    const double sy = p.bmode == 1 ? sig_opt : (p.bmode == 2 ? p.conv_sigma_y : 0.0);
+    const double sx = p.bmode == 1 ? sig_opt : (p.bmode == 2 ? p.conv_sigma_x : 0.0);
+    const int a = gauss_weights(sy, sh.wy);
+    const int b = gauss_weights(sx, sh.wx);
+    if (threadIdx.x == 0) {
+      sh.r = a;
+      sh.bi[0] = b;
+    }
+  }
+  share();
+  const int ry = sh.r, rx = sh.bi[0];
+  const PkSums sums = filter_rows<1, ROUNDS>(C, V, lay, mS, ry, rx, sh.wy, sh.wx, c, p.use_mask != 0);
+  gather(sums, Mode1());
+  if constexpr (S > 1) {
+    cg::this_cluster().sync();  // CTA 0 has read the others' sums
+    if (rank != 0) return;
+  }
+  FiltStats st{0.0, 0.0, 0.0f, 0};
+  if (warp == 0) st = stats_total(sh);
+  const float amax = (float)sh.bc[1];
+  const int aidx = sh.bi[0];
   __syncthreads();
-  FiltStats st;
-  float amax = 0.0f;
-  int aidx = 0;
-  filter_any<1>(C, V, rtab, w, mS, ry, rx, sh.wy, sh.wx, c, sh, p.use_mask != 0, st, amax, aidx);
   const int cy = aidx / w, cx = aidx - (aidx / w) * w;
   const float cval = C[cy * w + cx];
   float corr = cval;
@@ -784,7 +951,7 @@ __global__ void __launch_bounds__(PK_T, 1) k_peaks(const float* __restrict__ cwi
         float acc = 0.0f;
         if (ry == 0) acc = C[y * w + xx];
         else
-          for (int k = 0; k <= 2 * ry; k++) acc = fmaf(sh.wy[k], C[rtab[PK_MAXR + y - ry + k] * w + xx], acc);
+          for (int k = 0; k <= 2 * ry; k++) acc = fmaf(sh.wy[k], C[reflect_idx(y - ry + k, w) * w + xx], acc);
         V[e] = acc;
       }
       __syncthreads();
@@ -829,7 +996,7 @@ __global__ void __launch_bounds__(PK_T, 1) k_peaks(const float* __restrict__ cwi
     r.cx = cx;
     r.flags = flags;
     r.nfev = nfev;
-    res[blockIdx.x] = r;
+    res[win] = r;
   }
 }
 
@@ -1141,6 +1308,39 @@ __global__ void __launch_bounds__(PK_T, 1) k_full_finish(const float* __restrict
   }
 }
 
+constexpr int PK_SMS = 152;                    // SMs: one CTA each
+constexpr size_t PK_SMEM = (227 - 9) * 1024;  // dynamic shared memory beside the static arrays
+
+// Whether one run of rows of a window split over S CTAs fits V (at two
+// horizontal units a thread).
+template <int S>
+static bool pk_splits(int w, int vp, int vfloats) {
+  const int rb = pk_ty(w), len = (pk_quad(w) ? 2 : 1) * ((rb + S - 1) / S);
+  const int nt = ((rb + S - 1) / S) * (pk_quad(w) ? w / 4 : 64);
+  return rb >= S && pk_vrows(w, vp, 2, vfloats) >= len && 6 * nt <= vfloats;
+}
+
+template <int S>
+static int launch_peaks(const float* cwin, int M, int mS, const zr_peak_params_t& p, int pad, int vfloats, size_t smem,
+                        zr_peak_result_t* res, const float2* tw, cudaStream_t st) {
+  ZR_TRY(cuda_check(cudaFuncSetAttribute(k_peaks<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+                    "k_peaks attr"));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(M * S);
+  cfg.blockDim = dim3(PK_T);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = S;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = S > 1 ? 1 : 0;
+  ZR_TRY(cuda_check(cudaLaunchKernelEx(&cfg, k_peaks<S>, cwin, mS, p, pad, vfloats, p.opti_xatol / 3.0,
+                                       1.0 / (4.0 * mS * mS), res, tw), "k_peaks launch"));
+  return launched("k_peaks");
+}
+
 static int full_blocks(int C) { return ((C + FP_TX - 1) / FP_TX) * ((C + FP_RY - 1) / FP_RY); }
 
 }  // namespace zr
@@ -1162,21 +1362,35 @@ extern "C" int zr_locate_peaks(const float* cwin, int M, int max_shift, const zr
     return set_error(ZR_ESIZE, "zr_locate_peaks: opti sigma bound too large");
   const float2* tw = twiddles();
   if (!tw) return ZR_ECUDA;
-  // window + one block of filtered rows (RB lanes x pk_vec_rows rows at pitch
-  // w + 8 for the vectorised layout, PK_RB rows otherwise)
-  const bool vec = (w & 3) == 0 && w >= 16 && w <= 4 * PK_TX;
-  const size_t vrows = vec ? (size_t)(PK_T / (w / 4)) * pk_vec_rows(w) : (size_t)PK_RB;
-  size_t vbuf = vrows * (vec ? pk_vec_pitch(w) : w) * sizeof(float);
-  // the row block also holds the vertical pass of the 16 x 16 sub-pixel patch
-  const size_t pbuf = (size_t)16 * (16 + 2 * PK_MAXR) * sizeof(float);
-  if (vbuf < pbuf) vbuf = pbuf;
-  size_t smem = (size_t)w * w * sizeof(float) + vbuf;
+  // shared memory: the window, then V (the filter blocks; also the vertical
+  // pass of the 16 x 16 sub-pixel patch)
+  double smax = params->bmode == 1 ? params->opti_hi : 0.0;
+  if (params->bmode == 2) smax = fmax(params->conv_sigma_y, params->conv_sigma_x);
+  const int pad = ((int)(4.0 * fmax(smax, 0.0) + 0.5) + 3) & ~3;
+  const size_t win = (((size_t)w * w + 3) & ~(size_t)3) * sizeof(float);
   const size_t sub = (size_t)17 * 16 * params->sub_pix_reg * sizeof(float2);
-  if (params->sub_pix_reg > 1 && (size_t)w * w * sizeof(float) < sub) smem = sub + vbuf;
-  ZR_TRY(cuda_check(cudaFuncSetAttribute(k_peaks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                    "k_peaks attr"));
-  k_peaks<<<M, PK_T, smem, (cudaStream_t)stream>>>(cwin, max_shift, *params, results, tw);
-  return launched("k_peaks");
+  const size_t base = params->sub_pix_reg > 1 && win < sub ? sub : win;  // the sub-pixel step's scratch takes the window
+  const size_t vmin = (size_t)16 * (16 + 2 * PK_MAXR) * sizeof(float);
+  size_t vbytes = PK_SMEM > base + vmin ? PK_SMEM - base : vmin;
+  if (vbytes > (size_t)64 * 1024) vbytes = 64 * 1024;
+  const int vfloats = (int)(vbytes / sizeof(float));
+  cudaStream_t st = (cudaStream_t)stream;
+  // Full waves of one CTA per window and SM, then what is left with as many
+  // CTAs per window as fit the SMs
+  const int full = M / PK_SMS * PK_SMS, rest = M - full;
+  if (full) ZR_TRY(launch_peaks<1>(cwin, full, max_shift, *params, pad, vfloats, base + vbytes, results, tw, st));
+  cwin += (size_t)full * w * w;
+  results += full;
+  const int vp = ((w + 7) & ~7) + 2 * pad + 12;
+  if (rest == 0) return ZR_OK;
+  // (clusters sit within a GPC: not 19 of 8 CTAs fit at a time)
+  if (rest <= 8 && pk_splits<8>(w, vp, vfloats))
+    return launch_peaks<8>(cwin, rest, max_shift, *params, pad, vfloats, base + vbytes, results, tw, st);
+  if (rest <= 32 && pk_splits<4>(w, vp, vfloats))
+    return launch_peaks<4>(cwin, rest, max_shift, *params, pad, vfloats, base + vbytes, results, tw, st);
+  if (rest <= 72 && pk_splits<2>(w, vp, vfloats))
+    return launch_peaks<2>(cwin, rest, max_shift, *params, pad, vfloats, base + vbytes, results, tw, st);
+  return launch_peaks<1>(cwin, rest, max_shift, *params, pad, vfloats, base + vbytes, results, tw, st);
 }
 
 extern "C" int zr_full_prepare(float* planes, int n, int C, int suppress_origin, float* origin, float* mean,
