@@ -320,6 +320,31 @@ __device__ __forceinline__ void ip_pass1(float2* s, Load load) {
   }
 }
 
+// Pass 1 with butterflies j and j + 1 (j even) of one sequence in a thread, so
+// that the loader can read neighbouring elements in one access: ``load(b, j,
+// odd, v0, v1)`` fills v0 with butterfly j + odd and v1 with j + 1 - odd.
+// Every other eight lanes take the odd one first (odd = 1): each store of a
+// half-warp then covers all banks.
+template <int L, int NB, int T, int DIR, typename Load>
+__device__ __forceinline__ void ip_pass1_pairs(float2* s, Load load) {
+  using P = Ip<L>;
+  constexpr int NU = NB * (P::A1 / 2), LD = ip_ld(L, NB);
+  static_assert(P::A1 % 2 == 0, "whole pairs");
+  const int odd = (threadIdx.x >> 3) & 1;
+  for (int e = threadIdx.x; e < NU; e += T) {
+    const int b = e / (P::A1 / 2), j = 2 * (e - b * (P::A1 / 2));
+    float2 v0[16], v1[16];
+    load(b, j, odd, v0, v1);
+    float2* p = s + b * LD + j;
+    ip_dft<16, DIR>(v0);
+#pragma unroll
+    for (int r = 0; r < 16; r++) p[odd + r * P::S1] = v0[r];
+    ip_dft<16, DIR>(v1);
+#pragma unroll
+    for (int r = 0; r < 16; r++) p[1 - odd + r * P::S1] = v1[r];
+  }
+}
+
 // Pass 2 of a three-pass length, in place (nothing for a two-pass length).
 template <int L, int NB, int T, int DIR, bool BF>
 __device__ __forceinline__ void ip_pass2(float2* s, const float2* __restrict__ tw) {

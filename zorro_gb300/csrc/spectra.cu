@@ -6,10 +6,10 @@
 // Hermitian symmetry), only the C1/2+1 non-negative kx columns the crop keeps
 // are written, and the column pass keeps only the C0+1 cropped ky rows.
 //
-// Row-pass output layout (scratch): [frame][y/16][K4][y%16] complex (the last
-// group of a frame as many rows as it has, a multiple of 4), so that the row
-// pass (4 rows per CTA) writes whole 32-byte sectors and a warp of the column
-// pass reads 128-byte runs.
+// Row-pass output layout (scratch): [frame][y/8][K4][y%8] complex (the last
+// group of a frame as many rows as it has, a multiple of 4): the row pass's
+// stores of consecutive k lie close together, and two columns of 8 rows are
+// the 128-byte line that eight and eight lanes of the column pass read.
 #include <stdio.h>
 
 #include <type_traits>
@@ -20,20 +20,99 @@
 
 namespace zr {
 
-constexpr int NBR = 16;  // rows per group of the row-pass output layout
+constexpr int NBR = 8;  // rows per group of the row-pass output layout
 // Element (k, y) of one frame's row-pass output of 4 H4 rows.
 __device__ __forceinline__ int ru_rows(int y, int H4) { return min(NBR, 4 * H4 - (y & ~(NBR - 1))); }
 __device__ __forceinline__ size_t ru_at(int k, int y, int K4, int H4) {
   return (size_t)(y & ~(NBR - 1)) * K4 + (size_t)k * ru_rows(y, H4) + (y & (NBR - 1));
 }
-// rows per CTA of the row pass and columns per CTA of the column pass: the
-// defaults (the row pass's four rows fill whole sectors of its output, up to
-// 4096 points), or the planner's choice of 1, 2 or 4 per transform length
-// (tune_get)
+// Rows per CTA of the row pass and columns per CTA of the column pass: the
+// defaults, or the planner's choice of 1, 2 or 4 per transform length
+// (tune_get).  Two rows of 4096 points make two CTAs an SM, of which one loads
+// while the other transforms.  Spectra of eight K2 frames, microseconds, with
+// R rows and C columns a CTA and groups of G rows: 634 with R 4, C 1, G 16;
+// 639 with R 2, C 1, G 16; 630 with R 4, C 2, G 8; 589 with R 2, C 2, G 8; 595
+// with R 2, C 2, G 4; 780 with R 1 (8-byte stores).  Below 2048 points several
+// CTAs of four rows share an SM anyway: eight frames of 1000 x 1000, 43.6 with
+// R 2, 39.9 with R 4; of 2000 x 2000, 151 and 152.
 constexpr int FC_DEFAULT = 2;
-__host__ __device__ constexpr int fr_default(int P1) { return P1 > 4096 ? 2 : 4; }
+__host__ __device__ constexpr int fr_default(int P1) { return P1 >= 2048 ? 2 : 4; }
+__host__ __device__ constexpr int most_of(int P) { return P > 4096 ? 2 : 4; }  // that fit a CTA
 // CTAs per SM to ask the register allocator for: 128 registers a thread
 constexpr int minb_of(int T) { return sm_minb(T); }
+
+// corrected16 for x and x + 1 (x = j + r STEP, j even): u0 holds pixels x +
+// odd, u1 x + 1 - odd.  Needs even row lengths and frame strides and arrays
+// aligned to two elements (wide_pixels).  Half the loads of corrected16, which
+// waited for them: spectra of eight K2 frames 671 -> 645 us.
+template <int STEP, int FULL>
+__device__ __forceinline__ void corrected32(const FrameSrc& f, int n, int y, int j, int cols, int odd, float* u0,
+                                            float* u1) {
+  const int lim = cols - j;
+  const long long q = (long long)y * f.W + j;
+  const long long p = q + map_off(f, n);
+  const long long i = (long long)n * f.fstride + q;
+#define ZR_INSIDE(r) (r < FULL || r * STEP < lim)
+  float2 u[16];
+  if (f.type == ZR_U8) {
+    unsigned short bits[16];
+#pragma unroll
+    for (int r = 0; r < 16; r++)
+      bits[r] = ZR_INSIDE(r) ? __ldg((const unsigned short*)((const uint8_t*)f.raw + i + r * STEP)) : 0;
+#pragma unroll
+    for (int r = 0; r < 16; r++) u[r] = make_float2((float)(bits[r] & 255), (float)(bits[r] >> 8));
+  } else if (f.type == ZR_F32) {
+#pragma unroll
+    for (int r = 0; r < 16; r++)
+      u[r] = ZR_INSIDE(r) ? __ldg((const float2*)((const float*)f.raw + i + r * STEP)) : make_float2(0.0f, 0.0f);
+  } else {
+    unsigned int bits[16];
+#pragma unroll
+    for (int r = 0; r < 16; r++)
+      bits[r] = ZR_INSIDE(r) ? __ldg((const unsigned int*)((const uint16_t*)f.raw + i + r * STEP)) : 0u;
+#pragma unroll
+    for (int r = 0; r < 16; r++) {
+      if (f.type == ZR_F16)
+        u[r] = make_float2(__half2float(__ushort_as_half((unsigned short)(bits[r] & 0xffffu))),
+                           __half2float(__ushort_as_half((unsigned short)(bits[r] >> 16))));
+      else u[r] = make_float2((float)(bits[r] & 0xffffu), (float)(bits[r] >> 16));
+    }
+  }
+  auto map = [&](const float* m, int r) {
+    return ZR_INSIDE(r) ? __ldg((const float2*)(m + p + r * STEP)) : make_float2(0.0f, 0.0f);
+  };
+  if (f.gain) {
+    float2 g[16];
+#pragma unroll
+    for (int r = 0; r < 16; r++) g[r] = map(f.gain, r);
+#pragma unroll
+    for (int r = 0; r < 16; r++) u[r] = make_float2(__fmul_rn(g[r].x, u[r].x), __fmul_rn(g[r].y, u[r].y));
+  }
+  if (f.gdiv != 0.0f) {
+#pragma unroll
+    for (int r = 0; r < 16; r++) u[r] = make_float2(__fdiv_rn(u[r].x, f.gdiv), __fdiv_rn(u[r].y, f.gdiv));
+  }
+  if (f.ha) {
+#pragma unroll
+    for (int h = 0; h < 16; h += 8) {
+      float2 a[8], b[8];
+#pragma unroll
+      for (int r = 0; r < 8; r++) {
+        a[r] = map(f.ha, h + r);
+        b[r] = map(f.hb, h + r);
+      }
+#pragma unroll
+      for (int r = 0; r < 8; r++)
+        u[h + r] = make_float2(__fmaf_rn(a[r].x, u[h + r].x, b[r].x), __fmaf_rn(a[r].y, u[h + r].y, b[r].y));
+    }
+  }
+#undef ZR_INSIDE
+#pragma unroll
+  for (int r = 0; r < 16; r++) {
+    u0[r] = odd ? u[r].y : u[r].x;
+    u1[r] = odd ? u[r].x : u[r].y;
+  }
+}
 
 // Row pass: FR rows of one frame per CTA.  The first FFT pass reads the
 // pixels (consecutive lanes, consecutive pixels) and the last one untangles
@@ -42,7 +121,7 @@ constexpr int minb_of(int T) { return sm_minb(T); }
 template <int P1, int FR>
 __global__ void __launch_bounds__(ip_threads(P1, FR), minb_of(ip_threads(P1, FR)))
     k_fwd_rows(FrameSrc f, const float* __restrict__ mask, const double* __restrict__ mean_sub,
-               double inv_area, int frame0, int mode, int rows, int cols, int C1, int K4, int H4,
+               double inv_area, int frame0, int mode, int rows, int cols, int C1, int K4, int H4, bool wide,
                float2* __restrict__ RU, float2* __restrict__ RV, const float2* __restrict__ tw) {
   constexpr int T = ip_threads(P1, FR);
   using P = Ip<P1>;
@@ -54,7 +133,31 @@ __global__ void __launch_bounds__(ip_threads(P1, FR), minb_of(ip_threads(P1, FR)
   const int n = frame0 + nl;
   float mu = 0.0f;
   if (mode == 0 && mean_sub) mu = (float)(mean_sub[n] * inv_area);
-  if (mode == 0 && !mask) {
+  if (mode == 0 && !mask && wide) {
+    auto pixels = [&](auto full) {
+      constexpr int FULL = decltype(full)::value;
+      ip_pass1_pairs<P1, FR, T, -1>(sm, [&](int b, int j, int odd, float2* v0, float2* v1) {
+        const int y = y0 + b;
+        if (y >= rows) {
+#pragma unroll
+          for (int r = 0; r < 16; r++) v0[r] = v1[r] = make_float2(0.0f, 0.0f);
+          return;
+        }
+        float u0[16], u1[16];
+        corrected32<P::A1, FULL>(f, n, y, j, cols, odd, u0, u1);
+        const int lim = cols - j;
+#pragma unroll
+        for (int r = 0; r < 16; r++) {
+          const bool in = r < FULL || r * P::A1 < lim;
+          const float a = in ? u0[r] - mu : 0.0f, b = in ? u1[r] - mu : 0.0f;
+          v0[r] = make_float2(a, a * a);
+          v1[r] = make_float2(b, b * b);
+        }
+      });
+    };
+    if (cols >= 14 * P::A1) pixels(std::integral_constant<int, 14>());
+    else pixels(std::integral_constant<int, 0>());
+  } else if (mode == 0 && !mask) {
     auto pixels = [&](auto full) {
       constexpr int FULL = decltype(full)::value;
       ip_pass1<P1, FR, T, -1, false>(sm, [&](int b, int j, float2* v) {
@@ -145,8 +248,8 @@ __global__ void __launch_bounds__(ip_threads(P0, FC), minb_of(ip_threads(P0, FC)
   const int RP = C0 + 4;
   float2* out = (blockIdx.z == 0 ? G : S) + (size_t)nl * spec_elems + (size_t)k0 * RP;
   // (whole groups of rows and a butterfly step of whole groups: one stride)
-  const bool even = (H4 & 3) == 0 && P::A1 % NBR == 0;
-  ip_pass1<P0, FC, T, -1, false>(sm, [&](int c, int j, float2* v) {
+  const bool even = H4 % (NBR / 4) == 0 && P::A1 % NBR == 0;
+  ip_pass1<P0, FC, T, -1, true>(sm, [&](int c, int j, float2* v) {
     if (even) {
       const float2* src = R + (size_t)(j & ~(NBR - 1)) * K4 + (k0 + c) * NBR + (j & (NBR - 1));
       const size_t step = (size_t)P::A1 * K4;
@@ -206,6 +309,14 @@ __global__ void k_frame_sums(FrameSrc f, double* __restrict__ sums) {
   }
 }
 
+// Frames whose pixels can be read two at a time.
+static bool wide_pixels(const FrameSrc& f, int cols) {
+  const int esize = f.type == ZR_U8 ? 1 : (f.type == ZR_F32 ? 4 : 2);
+  const uintptr_t maps = (uintptr_t)f.gain | (uintptr_t)f.ha | (uintptr_t)f.hb;
+  return (f.W & 1) == 0 && (cols & 1) == 0 && (f.fstride & 1) == 0 && (f.mstride & 1) == 0 && (maps & 7) == 0 &&
+         (uintptr_t)f.raw % (2 * esize) == 0;
+}
+
 template <int P, int FR>
 static int launch_rows_v(const FrameSrc& f, const float* mask, const double* mean_sub, double inv_area,
                          int frame0, int nfr, int mode, int rows, int cols, int C1, int K4, int H4,
@@ -215,7 +326,8 @@ static int launch_rows_v(const FrameSrc& f, const float* mask, const double* mea
   ZR_TRY(cuda_check(cudaFuncSetAttribute(k_fwd_rows<P, FR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                     "k_fwd_rows attr"));
   k_fwd_rows<P, FR><<<dim3(nfr, (rows + FR - 1) / FR), T, smem, st>>>(f, mask, mean_sub, inv_area, frame0, mode,
-                                                                       rows, cols, C1, K4, H4, RU, RV, tw);
+                                                                       rows, cols, C1, K4, H4, wide_pixels(f, cols),
+                                                                       RU, RV, tw);
   return launched("k_fwd_rows");
 }
 
@@ -223,14 +335,14 @@ template <int P>
 static int launch_rows(const FrameSrc& f, const float* mask, const double* mean_sub, double inv_area,
                        int frame0, int nfr, int mode, int rows, int cols, int C1, int K4, int H4,
                        float2* RU, float2* RV, const float2* tw, cudaStream_t st) {
-  // 6144-point rows: at most two fit a CTA's shared memory and registers
-  constexpr int MOST = fr_default(P);
   switch (tune_get(TUNE_FWD_ROWS, P)) {
     case 1: return launch_rows_v<P, 1>(f, mask, mean_sub, inv_area, frame0, nfr, mode, rows, cols, C1, K4, H4, RU, RV, tw, st);
-    case 2: return launch_rows_v<P, 2>(f, mask, mean_sub, inv_area, frame0, nfr, mode, rows, cols, C1, K4, H4, RU, RV, tw, st);
+    case 4:
+      return launch_rows_v<P, most_of(P)>(f, mask, mean_sub, inv_area, frame0, nfr, mode, rows, cols, C1, K4, H4, RU, RV,
+                                          tw, st);
     default:
-      return launch_rows_v<P, MOST>(f, mask, mean_sub, inv_area, frame0, nfr, mode, rows, cols, C1, K4, H4, RU, RV, tw,
-                                    st);
+      return launch_rows_v<P, fr_default(P)>(f, mask, mean_sub, inv_area, frame0, nfr, mode, rows, cols, C1, K4, H4, RU, RV,
+                                          tw, st);
   }
 }
 
@@ -250,7 +362,7 @@ static int launch_cols(const float2* RU, const float2* RV, int rows, int C0, int
                        int nfr, int nz, float2* G, float2* S, const float2* tw, cudaStream_t st) {
   switch (tune_get(TUNE_FWD_COLS, P)) {
     case 1: return launch_cols_v<P, 1>(RU, RV, rows, C0, K4, H4, se, nfr, nz, G, S, tw, st);
-    case 4: return launch_cols_v<P, fr_default(P)>(RU, RV, rows, C0, K4, H4, se, nfr, nz, G, S, tw, st);
+    case 4: return launch_cols_v<P, most_of(P)>(RU, RV, rows, C0, K4, H4, se, nfr, nz, G, S, tw, st);
     default: return launch_cols_v<P, FC_DEFAULT>(RU, RV, rows, C0, K4, H4, se, nfr, nz, G, S, tw, st);
   }
 }
