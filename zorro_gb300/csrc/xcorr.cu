@@ -29,10 +29,12 @@
 namespace zr {
 
 // Column pass: columns per CTA (by default four, which write whole sectors of
-// the window rows, and two of the long 3072 and 4096 columns; the planner may
-// choose 1, 2 or 4 per length).  Row pass: packed row pairs per CTA (default
+// the window rows, and two from 2048 points on, where smaller CTAs overlap
+// better: terms and 190 pair windows at crop 2048, 1193 us with four, 1143 us
+// with two; at 1024, 608 and 615 us; the planner may choose 1, 2 or 4 per
+// length).  Row pass: packed row pairs per CTA (default
 // 2; the planner may choose 1, 2 or 4).
-__host__ __device__ constexpr int xc_nbc_default(int C0) { return C0 >= 3072 ? 2 : 4; }
+__host__ __device__ constexpr int xc_nbc_default(int C0) { return C0 >= 2048 ? 2 : 4; }
 constexpr int XC_NBR_DEFAULT = 2;
 
 struct XcJobs {
