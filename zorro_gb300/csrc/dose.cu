@@ -21,29 +21,42 @@
 
 namespace zr {
 
-// rows per CTA of the forward row pass and columns per CTA of the inverse
-// column pass
-#ifndef ZR_DS_NBR
-#define ZR_DS_NBR 4
-#endif
-constexpr int DS_NBR = ZR_DS_NBR;
-// rows (columns) per CTA for a transform of length L: two for the 6144-point
-// transforms, whose four-row tiles would not fit the register file
+// rows per CTA of the forward row pass, columns per CTA of the inverse column
+// pass
+__host__ __device__ constexpr int ds_rows(int P1) { return P1 >= 3072 ? 2 : 4; }
+constexpr int DS_NBR = 4;
+constexpr int DS_G = 8;  // rows per group of the row pass's output
+
+// Element (k, y) of one frame's row-pass output.
+__device__ __forceinline__ size_t rw_at(int k, int y, int K4) {
+  return ((size_t)(y / DS_G) * K4 + k) * DS_G + y % DS_G;
+}
+// columns per CTA for a transform of length L: two for the 6144-point
+// transforms, whose four-column tiles would not fit the register file
 __host__ __device__ constexpr int ds_nbr(int L) { return L > 4096 ? 2 : DS_NBR; }
 // CTAs per SM to ask the register allocator for: 128 registers a thread
 constexpr int ds_minb(int T) { return sm_minb(T); }
-
 
 __device__ __forceinline__ int sym_idx(int i, int n) {
   int m = i % (2 * n);
   return m < n ? m : 2 * n - 1 - m;
 }
 
+// Forward row pass: two or four rows of two frames per CTA, one complex
+// transform a row.  What bounds it: the latency of its loads and the scattered
+// stores (issue slots 35 % and shared-memory bandwidth 48 % used).  So a thread
+// loads two columns at a time, several CTAs share an SM (two of two rows from
+// 3072 points on), and a row's stores lie within DS_G rows of one another (as
+// columns of the whole height every 32 bytes went to a line 32 KB from the
+// last).  40 K2 frames, the whole filter: 2395 us with four rows a CTA, single
+// columns and whole columns; 2235 us so; 2330 us with four rows, 2359 us with
+// groups of four.  At 2048 points four rows take 324 us for 20 frames of 2000 x
+// 2000, two rows 364 us; at 1024, 93 us for 1000 x 1000 and 101 us.
 template <int P1>
-__global__ void __launch_bounds__(ip_threads(P1, ds_nbr(P1)), ds_minb(ip_threads(P1, ds_nbr(P1))))
-    k_dose_rows(const float* __restrict__ img, int N, int H, int W, int f0, int K4, int P0,
+__global__ void __launch_bounds__(ip_threads(P1, ds_rows(P1)), ds_minb(ip_threads(P1, ds_rows(P1))))
+    k_dose_rows(const float* __restrict__ img, int N, int H, int W, int f0, int K4, int P0, bool wide,
                 float2* __restrict__ RW, const float2* __restrict__ tw) {
-  constexpr int NB = ds_nbr(P1);
+  constexpr int NB = ds_rows(P1);
   constexpr int T = ip_threads(P1, NB);
   using P = Ip<P1>;
   extern __shared__ float2 sm[];
@@ -52,34 +65,55 @@ __global__ void __launch_bounds__(ip_threads(P1, ds_nbr(P1)), ds_minb(ip_threads
   const int na = f0 + 2 * pl, nb = na + 1;
   const float* ia = img + (size_t)na * H * W;
   const float* ib = img + (size_t)(nb < N ? nb : na) * H * W;
-  // element x of row b: the symmetric padding of the two frames' row.  The
-  // first FULL of a butterfly's columns lie inside the image for every j.
-  auto rows = [&](auto full) {
-    constexpr int FULL = decltype(full)::value;
-    ip_pass1<P1, NB, T, -1, false>(sm, [&](int b, int j, float2* v) {
-      const int yy = y0 + b;
-      const int ys = yy < H ? yy : (yy < 2 * H ? 2 * H - 1 - yy : sym_idx(yy, H));
-      const size_t row = (size_t)ys * W;
+  // row b: the symmetric padding of the two frames' row
+  auto source = [&](int b) {
+    const int yy = y0 + b;
+    return (size_t)(yy < H ? yy : (yy < 2 * H ? 2 * H - 1 - yy : sym_idx(yy, H))) * W;
+  };
+  auto column = [&](int x) { return x < W ? x : (x < 2 * W ? 2 * W - 1 - x : sym_idx(x, W)); };
+  if (wide && W >= 14 * P::A1) {  // two columns a load
+    ip_pass1_pairs<P1, NB, T, -1>(sm, [&](int b, int j, int odd, float2* v0, float2* v1) {
+      const size_t row = source(b);
       const float *pa = ia + row, *pb = ib + row;
+      float2 a[16], c[16];
 #pragma unroll
       for (int r = 0; r < 16; r++) {
         const int x = j + r * P::A1;
-        const int xs = r < FULL || x < W ? x : (x < 2 * W ? 2 * W - 1 - x : sym_idx(x, W));
+        if (r < 14 || x < W) {
+          a[r] = __ldg(reinterpret_cast<const float2*>(pa + x));
+          c[r] = nb < N ? __ldg(reinterpret_cast<const float2*>(pb + x)) : make_float2(0.0f, 0.0f);
+        } else {
+          const int x0 = column(x), x1 = column(x + 1);
+          a[r] = make_float2(__ldg(pa + x0), __ldg(pa + x1));
+          c[r] = nb < N ? make_float2(__ldg(pb + x0), __ldg(pb + x1)) : make_float2(0.0f, 0.0f);
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < 16; r++) {
+        v0[r] = odd ? make_float2(a[r].y, c[r].y) : make_float2(a[r].x, c[r].x);
+        v1[r] = odd ? make_float2(a[r].x, c[r].x) : make_float2(a[r].y, c[r].y);
+      }
+    });
+  } else {
+    ip_pass1<P1, NB, T, -1, false>(sm, [&](int b, int j, float2* v) {
+      const size_t row = source(b);
+      const float *pa = ia + row, *pb = ib + row;
+#pragma unroll
+      for (int r = 0; r < 16; r++) {
+        const int xs = column(j + r * P::A1);
         v[r] = make_float2(__ldg(pa + xs), nb < N ? __ldg(pb + xs) : 0.0f);
       }
     });
-  };
-  if (W >= 14 * P::A1) rows(std::integral_constant<int, 14>());
-  else rows(std::integral_constant<int, 0>());
+  }
   __syncthreads();
   ip_pass2<P1, NB, T, -1, false>(sm, tw);
-  // output: column-major per frame, [frame][kx][ky]; the last pass pairs X[k]
-  // with X[P1 - k] in registers
+  // output: [frame][ky / DS_G][kx][ky % DS_G]; the last pass pairs X[k] with
+  // X[P1 - k] in registers
   const size_t fa = (size_t)(2 * pl) * K4 * P0;
   const size_t fb = fa + (size_t)K4 * P0;
   ip_last_paired<P1, NB, T, -1>(sm, tw, [&](int r, int k0, const float2* x0, int k1, const float2* x1) {
     auto put = [&](int k, float2 zk, float2 zm) {
-      const size_t o = (size_t)k * P0 + y0 + r;
+      const size_t o = rw_at(k, y0 + r, K4);
       RW[fa + o] = make_float2(0.5f * (zk.x + zm.x), 0.5f * (zk.y - zm.y));
       if (nb < N) RW[fb + o] = make_float2(0.5f * (zk.y + zm.y), -0.5f * (zk.x - zm.x));
     };
@@ -93,7 +127,7 @@ __global__ void __launch_bounds__(ip_threads(P1, ds_nbr(P1)), ds_minb(ip_threads
   // the pitch's columns past P1/2 are zero
   for (int e = threadIdx.x; e < NB * (K4 - P1 / 2 - 1); e += T) {
     const int r = e % NB, k = P1 / 2 + 1 + e / NB;
-    const size_t o = (size_t)k * P0 + y0 + r;
+    const size_t o = rw_at(k, y0 + r, K4);
     RW[fa + o] = make_float2(0.0f, 0.0f);
     if (nb < N) RW[fb + o] = make_float2(0.0f, 0.0f);
   }
@@ -122,8 +156,9 @@ __device__ __forceinline__ void dose_weight(const zr_dose_params_t& p, int P0, i
 }
 
 // The whole filter of 40 K2 frames went from 2708 to 2395 us with the in-place
-// transforms (fft_inplace.cuh); the row and column passes' intermediates (2.7
-// GB each way) and the 2.3 GB of frames take 1130 us of it at copy bandwidth.
+// transforms (fft_inplace.cuh) and to 2235 us with the row pass above; the row
+// and column passes' intermediates (2.7 GB each way) and the 2.3 GB of frames
+// take 1130 us of it at copy bandwidth.
 //
 // One column kx per CTA: for every frame, the column's forward FFT, times the
 // frame's filter, accumulated in registers: thread k holds the rows k + r NS
@@ -158,36 +193,49 @@ __global__ void __launch_bounds__(ds_ct(P0), ds_minb(ds_ct(P0)))
     inv_crit[y] = 1.0f / crit;
     lq[y] = log2f(q);
   }
-  const bool mine = (int)threadIdx.x < P::NS;
-  float2 acc[P::RL];
-  float fm[P::RL];
+  // (256 points: 16 butterflies of 16 outputs, shared by 64 threads through
+  // shared memory)
+  constexpr bool SPREAD = P::NS < T;
+  constexpr int PER = SPREAD ? P0 / T : P::RL, STEP = SPREAD ? T : P::NS;
+  const bool mine = (int)threadIdx.x < STEP;
+  float2 acc[PER];
+  float fm[PER];
 #pragma unroll
-  for (int r = 0; r < P::RL; r++) {
-    const size_t o = (size_t)kx * P0 + threadIdx.x + r * P::NS;
+  for (int r = 0; r < PER; r++) {
+    const size_t o = (size_t)kx * P0 + threadIdx.x + r * STEP;
     acc[r] = first || !mine ? make_float2(0.0f, 0.0f) : ACC[o];
     fm[r] = (first || !mine || !prm.normalize) ? 0.0f : FM[o];
   }
   const float LOG2E = 1.4426950408889634f;
   for (int nl = 0; nl < nfr; nl++) {
-    const float2* col = RW + ((size_t)nl * K4 + kx) * P0;
+    const float2* col = RW + (size_t)nl * K4 * P0;
     // filt = exp(-0.5 D / crit), thres = exp(-(q / thresQ)^order)
     const float cd = (-0.5f * dose_end[f0 + nl]) * LOG2E;
     const float ltq = log2f(thres_q[f0 + nl]);
     __syncthreads();  // the previous frame's spectrum has been read
     ip_pass1<P0, 1, T, -1, false>(sm, [&](int, int j, float2* v) {
 #pragma unroll
-      for (int r = 0; r < 16; r++) v[r] = __ldg(col + j + r * P::A1);
+      for (int r = 0; r < 16; r++) v[r] = __ldg(col + rw_at(kx, j, K4) + (size_t)r * P::A1 * K4);
     });
     __syncthreads();
     ip_pass2<P0, 1, T, -1, false>(sm, tw);
+    if (SPREAD) {
+      ip_last_inplace<P0, 1, T, -1>(sm, tw);
+      __syncthreads();
+    }
     if (live && mine) {
-      float2 v[P::RL];
-      ip_last_load<P0, 1>(sm, 0, threadIdx.x, v);
-      ip_twiddle_last<P0, -1>(v, threadIdx.x, tw);
-      ip_dft<P::RL, -1>(v);
+      float2 v[PER];
+      if constexpr (SPREAD) {
 #pragma unroll
-      for (int r = 0; r < P::RL; r++) {
-        const int y = threadIdx.x + r * P::NS;
+        for (int r = 0; r < PER; r++) v[r] = sm[ip_at<P0>(threadIdx.x + r * STEP)];
+      } else {
+        ip_last_load<P0, 1>(sm, 0, threadIdx.x, v);
+        ip_twiddle_last<P0, -1>(v, threadIdx.x, tw);
+        ip_dft<P::RL, -1>(v);
+      }
+#pragma unroll
+      for (int r = 0; r < PER; r++) {
+        const int y = threadIdx.x + r * STEP;
         const float filt = exp2f(cd * inv_crit[y]);
         const float thres = exp2f(-LOG2E * exp2f(prm.cutoff_order * (lq[y] - ltq)));
         const float w = thres * filt;
@@ -198,8 +246,8 @@ __global__ void __launch_bounds__(ds_ct(P0), ds_minb(ds_ct(P0)))
   }
   if (!mine) return;
 #pragma unroll
-  for (int r = 0; r < P::RL; r++) {
-    const size_t o = (size_t)kx * P0 + threadIdx.x + r * P::NS;
+  for (int r = 0; r < PER; r++) {
+    const size_t o = (size_t)kx * P0 + threadIdx.x + r * STEP;
     ACC[o] = acc[r];
     if (prm.normalize) FM[o] = fm[r];
   }
@@ -289,10 +337,11 @@ static int set_smem(const void* fn, size_t smem) {
 template <int P1>
 static int dose_rows(const float* img, int N, int H, int W, int f0, int npairs, int K4, int P0, float2* RW,
                      const float2* tw, cudaStream_t st) {
-  const size_t smem = (size_t)ds_nbr(P1) * ip_ld(P1, ds_nbr(P1)) * sizeof(float2);
+  constexpr int T = ip_threads(P1, ds_rows(P1));
+  const size_t smem = (size_t)ds_rows(P1) * ip_ld(P1, ds_rows(P1)) * sizeof(float2);
+  const bool wide = (W & 1) == 0 && ((uintptr_t)img & 7) == 0;  // every row starts on 8 bytes
   ZR_TRY(set_smem<P1>((const void*)k_dose_rows<P1>, smem));
-  k_dose_rows<P1><<<dim3(P0 / ds_nbr(P1), npairs), ip_threads(P1, ds_nbr(P1)), smem, st>>>(img, N, H, W, f0, K4, P0,
-                                                                                            RW, tw);
+  k_dose_rows<P1><<<dim3(P0 / ds_rows(P1), npairs), T, smem, st>>>(img, N, H, W, f0, K4, P0, wide, RW, tw);
   return launched("k_dose_rows");
 }
 
