@@ -7,42 +7,61 @@
 // (scipy.ndimage.convolve: out[i] = sum_k w[k] in[i - k + 1], 'reflect'
 // borders of the rolled frame).  Sums run over frames in order in float32,
 // as np.sum(images, axis=0) does for a float32 stack.
+#include <type_traits>
+
 #include "common.cuh"
 #include "internal.h"
 
 namespace zr {
 
-#ifndef ZR_SS_MINB
-#define ZR_SS_MINB 6
-#endif
-#ifndef ZR_SS_R
-#define ZR_SS_R 2
-#endif
+constexpr int SS_MINB1 = 2;               // CTAs an SM of the kernel that loads ahead ...
+constexpr int SS_WAVE = SS_MINB1 * 152;   // ... and how many of them run at a time
 constexpr int SS_TX = 128, SS_THR = 256;  // tile columns (4 a lane), threads
 constexpr int SS_NCH = (SS_TX + 2 + 3 + 3) / 4;  // 4-pixel chunks that cover a halo row at any alignment
 constexpr int SS_TW = 4 * SS_NCH + 4;            // tile pitch: a guard column before the first chunk
+constexpr int SS_NQ = (SS_TX + 2 + 31) / 32;     // columns a lane reads of a row pixel by pixel
 // the corrections a frame's pixels take, resolved at compile time
 enum { SS_NONE = 0, SS_HOT = 1, SS_GAIN_HOT = 2, SS_ANY = 3 };
 
 __device__ __forceinline__ int refl1(int i, int n) { return i < 0 ? -i - 1 : (i >= n ? 2 * n - i - 1 : i); }
 
-// One raw value of the compile-time type TYPE, as float.
+// Raw values of the compile-time type TYPE: their array, their bits, as float.
 template <int TYPE>
-__device__ __forceinline__ float raw_at(const void* raw, long long idx) {
-  if constexpr (TYPE == ZR_U8) return (float)__ldg((const uint8_t*)raw + idx);
-  if constexpr (TYPE == ZR_U16) return (float)__ldg((const uint16_t*)raw + idx);
-  if constexpr (TYPE == ZR_F16) return __half2float(__ldg((const __half*)raw + idx));
-  return __ldg((const float*)raw + idx);
+__device__ __forceinline__ auto raw_ptr(const void* raw) {
+  if constexpr (TYPE == ZR_U8) return (const uint8_t*)raw;
+  else if constexpr (TYPE == ZR_F32) return (const unsigned int*)raw;
+  else return (const unsigned short*)raw;
+}
+template <int TYPE, typename T>
+__device__ __forceinline__ unsigned int raw_bits(const T* p) {
+  return __ldg(p);
+}
+template <int TYPE>
+__device__ __forceinline__ float bits_value(unsigned int b) {
+  if constexpr (TYPE == ZR_F32) return __uint_as_float(b);
+  else if constexpr (TYPE == ZR_F16) return __half2float(__ushort_as_half((unsigned short)b));
+  else return (float)b;
 }
 
 template <int TYPE>
 __device__ __forceinline__ float corrected_at(const FrameSrc& f, long long fo, long long p) {
-  float v = raw_at<TYPE>(f.raw, fo + p);
+  float v = bits_value<TYPE>(raw_bits<TYPE>(raw_ptr<TYPE>(f.raw) + fo + p));
   if (f.gain) v = __fmul_rn(__ldg(f.gain + p), v);
   if (f.gdiv != 0.0f) v = __fdiv_rn(v, f.gdiv);
   if (f.ha) v = __fmaf_rn(__ldg(f.ha + p), v, __ldg(f.hb + p));
   return v;
 }
+
+// A 4-pixel chunk's raw values and maps; a lane's columns of a row.
+struct SsChunk {
+  uint4 raw;
+  float4 g, A, B;
+};
+template <int NQ>
+struct SsRow {
+  unsigned int v[NQ];
+  float g[NQ], A[NQ], B[NQ];
+};
 
 // A CTA owns a 128 x 8R output tile and walks the frames in order.  For each
 // frame the corrected values of the tile and its one-pixel halo (at the
@@ -61,8 +80,17 @@ __device__ __forceinline__ float corrected_at(const FrameSrc& f, long long fo, l
 // pixels) is resolved where the row is read: two or three 16-byte loads and a
 // choice, the same for a whole warp, of which six of their values the four
 // columns take.  The chunks that hold the image's first and last column also
-// store its reflection beside it.  Wrapped tiles are read pixel by pixel.
-// Both paths apply the same operations to every pixel.
+// store its reflection beside it.  Wrapped tiles, and arrays not aligned so
+// (frames of odd width), are read pixel by pixel, a row a warp with all of a
+// lane's loads in flight: one at a time in a loop over the tile they took 654
+// us instead of 422 for 23 float32 frames of 1709 x 2859 with hot-pixel maps.
+// Every path applies the same operations to every pixel.
+//
+// R = 1 serves images whose 8-row tiles all run at once.  The walk over the
+// frames is what takes the time there, so the next frame's loads are in flight
+// while this one is filtered (registers for them: two CTAs an SM): 40 frames
+// of 512 x 512 with their aligned frames 100 us, 117 without; 27 of 302 x 114,
+// 53 and 70.
 //
 // What bounds it: issue slots.  The arithmetic is 6 operations a pixel, the
 // addressing was ten times that: so the rows' sources and alignments are
@@ -70,10 +98,10 @@ __device__ __forceinline__ float corrected_at(const FrameSrc& f, long long fo, l
 // frame ahead), and which corrections apply is a template argument.
 // 40 K2 frames (3838 x 3710 uint8, gain and hot-pixel maps) with their aligned
 // frames: 2135 us with 64 x 16 tiles whose chunks were stored and summed pixel
-// by pixel, 1438 us now; the half sums of 20 such frames 1071 -> 740 us.  Two
+// by pixel, 1365 us now; the half sums of 20 such frames 1071 -> 740 us.  Two
 // rows a thread (40 registers, six CTAs an SM) against four: 1438 and 1523 us.
 template <int TYPE, bool VEC, int MAPS, bool HALVES, int R>
-__global__ void __launch_bounds__(SS_THR, ZR_SS_MINB)
+__global__ void __launch_bounds__(SS_THR, R == 1 ? SS_MINB1 : (VEC && MAPS != SS_ANY ? 6 : 5))
     k_shift_sum(FrameSrc f, const zr_shift_t* __restrict__ sh, float* __restrict__ sum,
                 float* __restrict__ even, float* __restrict__ odd, float* __restrict__ aligned) {
   constexpr int TY = R * (SS_THR / 32), TH = TY + 2;
@@ -107,13 +135,12 @@ __global__ void __launch_bounds__(SS_THR, ZR_SS_MINB)
     const int c0 = xf - roll_x;
     return c0 < 0 ? c0 + W : c0;
   };
-  auto row_table = [&](int n) {
-    const int i = threadIdx.x;
-    if (i >= TH) return;
-    const int gy = y0 - 1 + i, c0 = first_col(sh[n].roll_x);
+  // where tile row i of a frame with shift t comes from: the row_table entry
+  auto row_source = [&](int i, const zr_shift_t& t) {
+    const int gy = y0 - 1 + i, c0 = first_col(t.roll_x);
     int2 r = make_int2(-1, 4 - edge);
     if (gy <= H) {
-      int sy = refl1(gy, H) - sh[n].roll_y;
+      int sy = refl1(gy, H) - t.roll_y;
       if (sy < 0) sy += H;
       if (VEC && c0 + ncol <= W) {
         const int p0 = sy * W + c0;
@@ -123,74 +150,154 @@ __global__ void __launch_bounds__(SS_THR, ZR_SS_MINB)
         r.x = sy;
       }
     }
-    rowt[n & 1][i] = r;
+    return r;
+  };
+  auto row_table = [&](int n) {
+    const int i = threadIdx.x;
+    if (i < TH) rowt[n & 1][i] = row_source(i, sh[n]);
   };
   row_table(0);
   __syncthreads();
   const int nrow = min(R, H - (y0 + ly0));              // output rows of this warp inside the image
   const bool pairs = x + 4 <= W && (W & 1) == 0;        // rows start on 8 bytes
+  constexpr int NR = (TH + 7) / 8;  // tile rows a warp reads
+  constexpr bool AHEAD = R == 1;    // loads a frame ahead
+  static_assert(!(AHEAD && VEC), "pixel by pixel");
+  const int extra = SS_THR - 1 - threadIdx.x;               // (from the last warp down: the first ones have the odd rows)
+  const bool gain = MAPS == SS_GAIN_HOT || (MAPS == SS_ANY && f.gain);
+  const bool hot = MAPS == SS_GAIN_HOT || MAPS == SS_HOT || (MAPS == SS_ANY && f.ha);
+  auto wraps = [&](const zr_shift_t& t) { return first_col(t.roll_x) + ncol > W; };
+  // first pixel of chunk k of a row with source r, -1 where the row does not reach it
+  auto first = [&](int2 r, int k) { return r.x < 0 || 4 * k >= r.y - 4 + edge + ncol ? -1 : r.x + 4 * k; };
+  auto fetch = [&](long long fo, int a, SsChunk& q) {
+    q.raw = raw_quad<TYPE>(f.raw, fo + a);
+    if (gain) q.g = __ldg(reinterpret_cast<const float4*>(f.gain + a));
+    if (hot) {
+      q.A = __ldg(reinterpret_cast<const float4*>(f.ha + a));
+      q.B = __ldg(reinterpret_cast<const float4*>(f.hb + a));
+    }
+  };
+  auto value = [&](const SsChunk& q) {
+    float4 r = quad_value<TYPE>(q.raw);
+    if (gain) r = make_float4(__fmul_rn(q.g.x, r.x), __fmul_rn(q.g.y, r.y), __fmul_rn(q.g.z, r.z), __fmul_rn(q.g.w, r.w));
+    if (MAPS == SS_ANY && f.gdiv != 0.0f)
+      r = make_float4(__fdiv_rn(r.x, f.gdiv), __fdiv_rn(r.y, f.gdiv), __fdiv_rn(r.z, f.gdiv), __fdiv_rn(r.w, f.gdiv));
+    if (hot)
+      r = make_float4(__fmaf_rn(q.A.x, r.x, q.B.x), __fmaf_rn(q.A.y, r.y, q.B.y), __fmaf_rn(q.A.z, r.z, q.B.z),
+                      __fmaf_rn(q.A.w, r.w, q.B.w));
+    return r;
+  };
+  auto tail = [&](long long fo, int a) {  // a chunk that runs past the end of the frame: its pixels inside
+    return make_float4(corrected_at<TYPE>(f, fo, a), a + 1 < HW ? corrected_at<TYPE>(f, fo, a + 1) : 0.0f,
+                       a + 2 < HW ? corrected_at<TYPE>(f, fo, a + 2) : 0.0f, 0.0f);
+  };
+  auto place = [&](int2 src, int i, int k, float4 r) {
+    float* dst = &tile[i][4 + 4 * k];
+    *reinterpret_cast<float4*>(dst) = r;
+    if (inner) return;
+    const int run = src.y - 4 + edge;  // misalignment s
+    if (edge && k == 0)  // column -1 reads column 0
+      dst[run - 1] = run == 0 ? r.x : (run == 1 ? r.y : (run == 2 ? r.z : r.w));
+    const int e = run + ncol - 1 - 4 * k;  // column W - 1, when this chunk holds it
+    if (last && e < 4) dst[e + 1] = e == 0 ? r.x : (e == 1 ? r.y : (e == 2 ? r.z : r.w));
+  };
+  // pixel (i, j) of the tile from its raw value and maps
+  auto put = [&](int i, int j, float r, float g, float A, float B) {
+    if (gain) r = __fmul_rn(g, r);
+    if (MAPS == SS_ANY && f.gdiv != 0.0f) r = __fdiv_rn(r, f.gdiv);
+    if (hot) r = __fmaf_rn(A, r, B);
+    tile[i][4 + j] = r;
+    if (edge && j == 0) tile[i][3] = r;
+    if (last && j == ncol - 1) tile[i][4 + j + 1] = r;
+  };
+  // A row pixel by pixel, wrapped or not: a lane takes every 32nd column (the
+  // first lanes the last two), NQ of them from column 32 q0 on
+  constexpr int NQ = VEC ? 2 : SS_NQ;  // (VEC: wrapped tiles are rare, registers are not)
+  auto row_fetch = [&](auto wrap, long long fo, int c0, int sy, int q0, SsRow<NQ>& q) {
+    const int m = sy < 0 ? 0 : ncol - lane - 32 * q0;  // columns lane + 32 (q0 + i), 32 i < m
+    const int c = c0 + lane + 32 * q0;
+    const long long p = (long long)sy * W + c;
+    const auto* vp = raw_ptr<TYPE>(f.raw) + fo + p;
+    const float *gp = f.gain + p, *ap = f.ha + p, *bp = f.hb + p;
+#pragma unroll
+    for (int i = 0; i < NQ; i++) {
+      const bool in = 32 * i < m;
+      const int o = decltype(wrap)::value && c + 32 * i >= W ? 32 * i - W : 32 * i;
+      q.v[i] = in ? raw_bits<TYPE>(vp + o) : 0u;
+      q.g[i] = in && gain ? __ldg(gp + o) : 0.0f;
+      q.A[i] = in && hot ? __ldg(ap + o) : 0.0f;
+      q.B[i] = in && hot ? __ldg(bp + o) : 0.0f;
+    }
+  };
+  auto row_place = [&](int sy, int i, int q0, const SsRow<NQ>& q) {
+    const int m = sy < 0 ? 0 : ncol - lane - 32 * q0;
+#pragma unroll
+    for (int j = 0; j < NQ; j++)
+      if (32 * j < m) put(i, lane + 32 * (q0 + j), bits_value<TYPE>(q.v[j]), q.g[j], q.A[j], q.B[j]);
+  };
+  SsRow<NQ> rw[AHEAD ? NR : 1];
+  auto load_ahead = [&](int n, const zr_shift_t& t) {
+#pragma unroll
+    for (int i = 0; i < NR; i++)
+      row_fetch(std::true_type(), (long long)n * f.fstride, first_col(t.roll_x),
+                wid + 8 * i < TH ? row_source(wid + 8 * i, t).x : -1, 0, rw[AHEAD ? i : 0]);
+  };
+  zr_shift_t t = sh[0], next = sh[min(1, f.N - 1)];
+  if constexpr (AHEAD) load_ahead(0, t);
   for (int n = 0; n < f.N; n++) {
-    const zr_shift_t t = sh[n];
+    if (!AHEAD) t = sh[n];
     const long long fo = (long long)n * f.fstride;
     const int c0 = first_col(t.roll_x);
     const int par = n & 1;
-    if (VEC && c0 + ncol <= W) {
-      auto chunk = [&](int i, int k) {
-        const int2 rt = rowt[par][i];
-        const int run = rt.y - 4 + edge;  // misalignment s
-        if (rt.x < 0 || 4 * k >= run + ncol) return;
-        const int a = rt.x + 4 * k;
+    if constexpr (AHEAD) {
+#pragma unroll
+      for (int i = 0; i < NR; i++) row_place(wid + 8 * i < TH ? rowt[par][wid + 8 * i].x : -1, wid + 8 * i, 0, rw[i]);
+    } else if (!VEC || wraps(t)) {
+      if (!VEC && wraps(t)) {
+        for (int e = threadIdx.x; e < TH * (SS_TX + 2); e += SS_THR) {
+          const int i = e / (SS_TX + 2), j = e - i * (SS_TX + 2);
+          const int sy = rowt[par][i].x;
+          if (sy < 0 || j >= ncol) continue;
+          const long long p = (long long)sy * W + (c0 + j >= W ? c0 + j - W : c0 + j);
+          put(i, j, bits_value<TYPE>(raw_bits<TYPE>(raw_ptr<TYPE>(f.raw) + fo + p)), gain ? __ldg(f.gain + p) : 0.0f,
+              hot ? __ldg(f.ha + p) : 0.0f, hot ? __ldg(f.hb + p) : 0.0f);
+        }
+      } else {
+#pragma unroll 1
+        for (int i = wid; i < TH; i += SS_THR / 32) {
+          const int sy = rowt[par][i].x;
+#pragma unroll 1
+          for (int q0 = 0; q0 < SS_NQ; q0 += NQ) {
+            row_fetch(std::integral_constant<bool, VEC>(), fo, c0, sy, q0, rw[0]);
+            row_place(sy, i, q0, rw[0]);
+          }
+        }
+      }
+    } else if constexpr (VEC) {
+      auto one = [&](int i, int k) {
+        const int2 src = rowt[par][i];
+        const int a = first(src, k);
+        if (a < 0) return;
         float4 r;
         if (a + 4 <= HW) {
-          r = quad_value<TYPE>(raw_quad<TYPE>(f.raw, fo + a));
-          if (MAPS == SS_GAIN_HOT || (MAPS == SS_ANY && f.gain)) {
-            const float4 g = __ldg(reinterpret_cast<const float4*>(f.gain + a));
-            r = make_float4(__fmul_rn(g.x, r.x), __fmul_rn(g.y, r.y), __fmul_rn(g.z, r.z), __fmul_rn(g.w, r.w));
-          }
-          if (MAPS == SS_ANY && f.gdiv != 0.0f)
-            r = make_float4(__fdiv_rn(r.x, f.gdiv), __fdiv_rn(r.y, f.gdiv), __fdiv_rn(r.z, f.gdiv),
-                            __fdiv_rn(r.w, f.gdiv));
-          if (MAPS == SS_GAIN_HOT || MAPS == SS_HOT || (MAPS == SS_ANY && f.ha)) {
-            const float4 A = __ldg(reinterpret_cast<const float4*>(f.ha + a));
-            const float4 B = __ldg(reinterpret_cast<const float4*>(f.hb + a));
-            r = make_float4(__fmaf_rn(A.x, r.x, B.x), __fmaf_rn(A.y, r.y, B.y), __fmaf_rn(A.z, r.z, B.z),
-                            __fmaf_rn(A.w, r.w, B.w));
-          }
-        } else {  // the chunk runs past the end of the frame: its pixels inside
-          r.x = corrected_at<TYPE>(f, fo, a);
-          r.y = a + 1 < HW ? corrected_at<TYPE>(f, fo, a + 1) : 0.0f;
-          r.z = a + 2 < HW ? corrected_at<TYPE>(f, fo, a + 2) : 0.0f;
-          r.w = 0.0f;
+          SsChunk q;
+          fetch(fo, a, q);
+          r = value(q);
+        } else {
+          r = tail(fo, a);
         }
-        float* dst = &tile[i][4 + 4 * k];
-        *reinterpret_cast<float4*>(dst) = r;
-        if (inner) return;
-        if (edge && k == 0)  // column -1 reads column 0
-          dst[run - 1] = run == 0 ? r.x : (run == 1 ? r.y : (run == 2 ? r.z : r.w));
-        const int e = run + ncol - 1 - 4 * k;  // column W - 1, when this chunk holds it
-        if (last && e < 4) dst[e + 1] = e == 0 ? r.x : (e == 1 ? r.y : (e == 2 ? r.z : r.w));
+        place(src, i, k, r);
       };
 #pragma unroll
-      for (int i = 0; i < (TH + 7) / 8; i++)
-        if (wid + 8 * i < TH) chunk(wid + 8 * i, lane);
-      // (from the last warp down: the first ones have the odd rows)
-      const int e = SS_THR - 1 - threadIdx.x;
-      if (e < 2 * TH) chunk(e >> 1, 32 + (e & 1));
-    } else {
-      for (int e = threadIdx.x; e < TH * (SS_TX + 2); e += SS_THR) {
-        const int i = e / (SS_TX + 2), j = e - i * (SS_TX + 2);
-        const int sy = rowt[par][i].x;
-        if (sy < 0 || j >= ncol) continue;
-        int sx = c0 + j;
-        if (sx >= W) sx -= W;
-        const float v = corrected_at<TYPE>(f, fo, (long long)sy * W + sx);
-        tile[i][4 + j] = v;
-        if (edge && j == 0) tile[i][3] = v;
-        if (last && j == ncol - 1) tile[i][4 + j + 1] = v;
-      }
+      for (int i = 0; i < NR; i++)
+        if (wid + 8 * i < TH) one(wid + 8 * i, lane);
+      if (extra < 2 * TH) one(extra >> 1, 32 + (extra & 1));
     }
     __syncthreads();
-    if (n + 1 < f.N) row_table(n + 1);
+    if (n + 1 < f.N) {
+      row_table(n + 1);
+      if constexpr (AHEAD) load_ahead(n + 1, next);
+    }
     // a function of columns x - 1 .. x + 4 of tile row ly0 + i
     auto six = [&](int i, auto g) {
       const int o = rowt[par][ly0 + i].y;
@@ -249,6 +356,10 @@ __global__ void __launch_bounds__(SS_THR, ZR_SS_MINB)
       for (int i = 0; i < R; i++)
         emit(i, six(i + 1, [](float, float b, float c, float d, float e, float) { return make_float4(b, c, d, e); }));
     }
+    if (AHEAD) {
+      t = next;
+      next = sh[min(n + 2, f.N - 1)];
+    }
     __syncthreads();
   }
 #pragma unroll
@@ -280,26 +391,20 @@ struct SsArgs {
 template <int TYPE, bool VEC, int MAPS, int R>
 static void launch_halves(const SsArgs& a, bool halves) {
   if (halves)
-    k_shift_sum<TYPE, VEC, MAPS, true, (R > 2 ? 2 : R)><<<a.grid, SS_THR, 0, a.st>>>(a.f, a.shifts, a.sum, a.even, a.odd,
-                                                                                  a.aligned);
+    k_shift_sum<TYPE, VEC, MAPS, true, R><<<a.grid, SS_THR, 0, a.st>>>(a.f, a.shifts, a.sum, a.even, a.odd, a.aligned);
   else
     k_shift_sum<TYPE, VEC, MAPS, false, R><<<a.grid, SS_THR, 0, a.st>>>(a.f, a.shifts, a.sum, a.even, a.odd, a.aligned);
 }
 
 template <int TYPE>
-static void launch_shift(const SsArgs& a, bool vec, bool tall, bool halves, int maps) {
-  constexpr int R = ZR_SS_R;
-  if (!vec) {
-    if (tall) launch_halves<TYPE, false, SS_ANY, R>(a, halves);
-    else launch_halves<TYPE, false, SS_ANY, 1>(a, halves);
-    return;
-  }
-  if (!tall) return launch_halves<TYPE, true, SS_ANY, 1>(a, halves);
+static void launch_shift(const SsArgs& a, bool vec, bool small, bool halves, int maps) {
+  if (small) return launch_halves<TYPE, false, SS_ANY, 1>(a, halves);
+  if (!vec) return launch_halves<TYPE, false, SS_ANY, 2>(a, halves);
   switch (maps) {
-    case SS_NONE: return launch_halves<TYPE, true, SS_NONE, R>(a, halves);
-    case SS_HOT: return launch_halves<TYPE, true, SS_HOT, R>(a, halves);
-    case SS_GAIN_HOT: return launch_halves<TYPE, true, SS_GAIN_HOT, R>(a, halves);
-    default: launch_halves<TYPE, true, SS_ANY, R>(a, halves);
+    case SS_NONE: return launch_halves<TYPE, true, SS_NONE, 2>(a, halves);
+    case SS_HOT: return launch_halves<TYPE, true, SS_HOT, 2>(a, halves);
+    case SS_GAIN_HOT: return launch_halves<TYPE, true, SS_GAIN_HOT, 2>(a, halves);
+    default: launch_halves<TYPE, true, SS_ANY, 2>(a, halves);
   }
 }
 
@@ -322,22 +427,20 @@ extern "C" int zr_shift_sum(const zr_frames_t* frames, const zr_shift_t* shifts,
   const bool vec = (long long)f.H * f.W < (1LL << 31) - 1024 && f.fstride % 4 == 0 && ((uintptr_t)f.raw % qbytes) == 0 && ((uintptr_t)f.gain & 15) == 0 &&
                    ((uintptr_t)f.ha & 15) == 0 && ((uintptr_t)f.hb & 15) == 0;
   const bool halves = even_sum || odd_sum;
-  // tiles of 32 rows (16 with the half sums, whose accumulators take shared
-  // memory); of 8 rows where those would leave the SMs short of CTAs (each
-  // CTA walks every frame, so a small image is bound by that walk)
+  // tiles of 16 rows; of 8, loading a frame ahead, where all of those run at
+  // once (above one wave they lose: 20 frames of 1536 x 1536 266 us against 168)
   const int nx = (f.W + SS_TX - 1) / SS_TX;
-  const int rows = halves ? 16 : 8 * ZR_SS_R;
-  const bool tall = (long long)nx * ((f.H + rows - 1) / rows) >= 2 * 152;
-  const dim3 grid(nx, tall ? (f.H + rows - 1) / rows : (f.H + 7) / 8);
+  const bool small = (long long)nx * ((f.H + 7) / 8) <= SS_WAVE;
+  const dim3 grid(nx, small ? (f.H + 7) / 8 : (f.H + 15) / 16);
   const int maps = f.gdiv != 0.0f ? SS_ANY
                    : f.gain       ? (f.ha ? SS_GAIN_HOT : SS_ANY)
                                   : (f.ha ? SS_HOT : SS_NONE);
   const SsArgs a{f, shifts, image_sum, even_sum, odd_sum, aligned, grid, st};
   switch (f.type) {
-    case ZR_U8: launch_shift<ZR_U8>(a, vec, tall, halves, maps); break;
-    case ZR_U16: launch_shift<ZR_U16>(a, vec, tall, halves, maps); break;
-    case ZR_F16: launch_shift<ZR_F16>(a, vec, tall, halves, maps); break;
-    case ZR_F32: launch_shift<ZR_F32>(a, vec, tall, halves, maps); break;
+    case ZR_U8: launch_shift<ZR_U8>(a, vec, small, halves, maps); break;
+    case ZR_U16: launch_shift<ZR_U16>(a, vec, small, halves, maps); break;
+    case ZR_F16: launch_shift<ZR_F16>(a, vec, small, halves, maps); break;
+    case ZR_F32: launch_shift<ZR_F32>(a, vec, small, halves, maps); break;
     default: return set_error(ZR_EINVAL, "zr_shift_sum: raw type %d", f.type);
   }
   return launched("k_shift_sum");
