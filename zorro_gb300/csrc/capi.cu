@@ -39,7 +39,7 @@ int launched(const char* what) {
 }
 
 // W_TWN^k = exp(-2 pi i k / TWN), then its contiguous copies per
-// sub-transform length (tw_compact_off) and the in-place transforms' tables
+// sub-transform length (TW_COMPACT) and the in-place transforms' tables
 // (ip_tw_off), one table per device.
 static __device__ float2 d_twiddle[TWN + TW_COMPACT + IP_TW];
 
@@ -60,11 +60,8 @@ static int init_device(int dev) {
     host[k] = make_float2((float)cos(a), (float)sin(a));
   }
   for (int k = 0; k < TW_COMPACT; k++) host[TWN + k] = make_float2(0.0f, 0.0f);
-  for (int M = 1; M <= 16384; M *= 2) {
-    for (int j = 0; j < M; j++) host[TWN + tw_compact_off(M) + j] = host[(size_t)j * (TWN / M)];
-    if (3 * M <= 12288)
-      for (int j = 0; j < 3 * M; j++) host[TWN + tw_compact_off(3 * M) + j] = host[(size_t)j * (TWN / (3 * M))];
-  }
+  for (int M = 1; M <= 16384; M *= 2)
+    for (int j = 0; j < M; j++) host[TWN + M + j] = host[(size_t)j * (TWN / M)];
   for (int i = 0; i <= IP_LENGTHS; i++) {
     const int L = ip_length(i);
     float2* t = host + TWN + TW_COMPACT + ip_tw_off(L);

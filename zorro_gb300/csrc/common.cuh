@@ -270,8 +270,6 @@ __device__ __forceinline__ void corrected16(const FrameSrc& f, int n, int y, int
   }
 }
 
-__device__ __forceinline__ int ilog2c(int v) { return 31 - __clz(v); }
-
 // Element i of the length-L complex sequence whose inverse FFT holds two real
 // rows (row a in the real part, row b in the imaginary part), from the rows'
 // half-plane spectra ``ra``/``rb`` (elements 0..L/2; null: a zero row):

@@ -31,14 +31,9 @@ inline int ilog2(long long v) {
 #ifndef ZR_FFT_EPT
 #define ZR_FFT_EPT 32
 #endif
-#ifndef ZR_FFT_MINB
-#define ZR_FFT_MINB 2
-#endif
 constexpr int fft_threads(int L, int NB, int ept = ZR_FFT_EPT) {
   return (NB * L / ept < 64) ? 64 : ((NB * L / ept > 512) ? 512 : NB * L / ept);
 }
-// Resident CTAs per SM to ask the register allocator for (short transforms).
-constexpr int fft_minblocks(int L) { return L <= 2048 ? ZR_FFT_MINB : 1; }
 // CTAs of T threads per SM to ask the register allocator for, so that
 // ZR_SM_THREADS threads fit an SM (512: up to 128 registers a thread).
 #ifndef ZR_SM_THREADS
