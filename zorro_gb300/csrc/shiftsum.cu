@@ -14,14 +14,14 @@
 
 namespace zr {
 
-constexpr int SS_MINB1 = 2;               // CTAs an SM of the kernel that loads ahead ...
-constexpr int SS_WAVE = SS_MINB1 * 152;   // ... and how many of them run at a time
+constexpr int SS_SMS = 152;
 constexpr int SS_TX = 128, SS_THR = 256;  // tile columns (4 a lane), threads
 constexpr int SS_NCH = (SS_TX + 2 + 3 + 3) / 4;  // 4-pixel chunks that cover a halo row at any alignment
 constexpr int SS_TW = 4 * SS_NCH + 4;            // tile pitch: a guard column before the first chunk
 constexpr int SS_NQ = (SS_TX + 2 + 31) / 32;     // columns a lane reads of a row pixel by pixel
 // the corrections a frame's pixels take, resolved at compile time
-enum { SS_NONE = 0, SS_HOT = 1, SS_GAIN_HOT = 2, SS_ANY = 3 };
+// (SS_BIG: any, and pixel offsets of more than 32 bits)
+enum { SS_NONE = 0, SS_HOT = 1, SS_GAIN_HOT = 2, SS_ANY = 3, SS_BIG = 4 };
 
 __device__ __forceinline__ int refl1(int i, int n) { return i < 0 ? -i - 1 : (i >= n ? 2 * n - i - 1 : i); }
 
@@ -83,14 +83,15 @@ struct SsRow {
 // store its reflection beside it.  Wrapped tiles, and arrays not aligned so
 // (frames of odd width), are read pixel by pixel, a row a warp with all of a
 // lane's loads in flight: one at a time in a loop over the tile they took 654
-// us instead of 422 for 23 float32 frames of 1709 x 2859 with hot-pixel maps.
+// us instead of 423 for 23 float32 frames of 1709 x 2859 with hot-pixel maps.
+// Their addresses are 32-bit byte offsets (64-bit ones were a quarter of the
+// instructions; SS_BIG keeps them for frames of 2^30 pixels and more).
 // Every path applies the same operations to every pixel.
 //
 // R = 1 serves images whose 8-row tiles all run at once.  The walk over the
 // frames is what takes the time there, so the next frame's loads are in flight
-// while this one is filtered (registers for them: two CTAs an SM): 40 frames
-// of 512 x 512 with their aligned frames 100 us, 117 without; 27 of 302 x 114,
-// 53 and 70.
+// while this one is filtered: 40 frames of 512 x 512 with their aligned frames
+// 83 us, 117 without; 27 of 302 x 114, 45 and 70.
 //
 // What bounds it: issue slots.  The arithmetic is 6 operations a pixel, the
 // addressing was ten times that: so the rows' sources and alignments are
@@ -98,10 +99,10 @@ struct SsRow {
 // frame ahead), and which corrections apply is a template argument.
 // 40 K2 frames (3838 x 3710 uint8, gain and hot-pixel maps) with their aligned
 // frames: 2135 us with 64 x 16 tiles whose chunks were stored and summed pixel
-// by pixel, 1365 us now; the half sums of 20 such frames 1071 -> 740 us.  Two
+// by pixel, 1360 us now; the half sums of 20 such frames 1071 -> 740 us.  Two
 // rows a thread (40 registers, six CTAs an SM) against four: 1438 and 1523 us.
-template <int TYPE, bool VEC, int MAPS, bool HALVES, int R>
-__global__ void __launch_bounds__(SS_THR, R == 1 ? SS_MINB1 : (VEC && MAPS != SS_ANY ? 6 : 5))
+template <int TYPE, bool VEC, int MAPS, bool HALVES, int R, int CTAS>
+__global__ void __launch_bounds__(SS_THR, CTAS)
     k_shift_sum(FrameSrc f, const zr_shift_t* __restrict__ sh, float* __restrict__ sum,
                 float* __restrict__ even, float* __restrict__ odd, float* __restrict__ aligned) {
   constexpr int TY = R * (SS_THR / 32), TH = TY + 2;
@@ -164,8 +165,8 @@ __global__ void __launch_bounds__(SS_THR, R == 1 ? SS_MINB1 : (VEC && MAPS != SS
   constexpr bool AHEAD = R == 1;    // loads a frame ahead
   static_assert(!(AHEAD && VEC), "pixel by pixel");
   const int extra = SS_THR - 1 - threadIdx.x;               // (from the last warp down: the first ones have the odd rows)
-  const bool gain = MAPS == SS_GAIN_HOT || (MAPS == SS_ANY && f.gain);
-  const bool hot = MAPS == SS_GAIN_HOT || MAPS == SS_HOT || (MAPS == SS_ANY && f.ha);
+  const bool gain = MAPS == SS_GAIN_HOT || (MAPS >= SS_ANY && f.gain);
+  const bool hot = MAPS == SS_GAIN_HOT || MAPS == SS_HOT || (MAPS >= SS_ANY && f.ha);
   auto wraps = [&](const zr_shift_t& t) { return first_col(t.roll_x) + ncol > W; };
   // first pixel of chunk k of a row with source r, -1 where the row does not reach it
   auto first = [&](int2 r, int k) { return r.x < 0 || 4 * k >= r.y - 4 + edge + ncol ? -1 : r.x + 4 * k; };
@@ -180,7 +181,7 @@ __global__ void __launch_bounds__(SS_THR, R == 1 ? SS_MINB1 : (VEC && MAPS != SS
   auto value = [&](const SsChunk& q) {
     float4 r = quad_value<TYPE>(q.raw);
     if (gain) r = make_float4(__fmul_rn(q.g.x, r.x), __fmul_rn(q.g.y, r.y), __fmul_rn(q.g.z, r.z), __fmul_rn(q.g.w, r.w));
-    if (MAPS == SS_ANY && f.gdiv != 0.0f)
+    if (MAPS >= SS_ANY && f.gdiv != 0.0f)
       r = make_float4(__fdiv_rn(r.x, f.gdiv), __fdiv_rn(r.y, f.gdiv), __fdiv_rn(r.z, f.gdiv), __fdiv_rn(r.w, f.gdiv));
     if (hot)
       r = make_float4(__fmaf_rn(q.A.x, r.x, q.B.x), __fmaf_rn(q.A.y, r.y, q.B.y), __fmaf_rn(q.A.z, r.z, q.B.z),
@@ -204,7 +205,7 @@ __global__ void __launch_bounds__(SS_THR, R == 1 ? SS_MINB1 : (VEC && MAPS != SS
   // pixel (i, j) of the tile from its raw value and maps
   auto put = [&](int i, int j, float r, float g, float A, float B) {
     if (gain) r = __fmul_rn(g, r);
-    if (MAPS == SS_ANY && f.gdiv != 0.0f) r = __fdiv_rn(r, f.gdiv);
+    if (MAPS >= SS_ANY && f.gdiv != 0.0f) r = __fdiv_rn(r, f.gdiv);
     if (hot) r = __fmaf_rn(A, r, B);
     tile[i][4 + j] = r;
     if (edge && j == 0) tile[i][3] = r;
@@ -214,26 +215,55 @@ __global__ void __launch_bounds__(SS_THR, R == 1 ? SS_MINB1 : (VEC && MAPS != SS
   // first lanes the last two), NQ of them from column 32 q0 on
   constexpr int NQ = VEC ? 2 : SS_NQ;  // (VEC: wrapped tiles are rare, registers are not)
   auto row_fetch = [&](auto wrap, long long fo, int c0, int sy, int q0, SsRow<NQ>& q) {
+    using Off = std::conditional_t<MAPS == SS_BIG, unsigned long long, unsigned int>;  // bytes
     const int m = sy < 0 ? 0 : ncol - lane - 32 * q0;  // columns lane + 32 (q0 + i), 32 i < m
     const int c = c0 + lane + 32 * q0;
-    const long long p = (long long)sy * W + c;
-    const auto* vp = raw_ptr<TYPE>(f.raw) + fo + p;
-    const float *gp = f.gain + p, *ap = f.ha + p, *bp = f.hb + p;
+    const Off row = (Off)sy * W + c;
+    const char* raw = reinterpret_cast<const char*>(raw_ptr<TYPE>(f.raw) + fo);
+    auto map = [&](const float* p, Off o) { return __ldg(reinterpret_cast<const float*>(reinterpret_cast<const char*>(p) + o)); };
 #pragma unroll
     for (int i = 0; i < NQ; i++) {
       const bool in = 32 * i < m;
-      const int o = decltype(wrap)::value && c + 32 * i >= W ? 32 * i - W : 32 * i;
-      q.v[i] = in ? raw_bits<TYPE>(vp + o) : 0u;
-      q.g[i] = in && gain ? __ldg(gp + o) : 0.0f;
-      q.A[i] = in && hot ? __ldg(ap + o) : 0.0f;
-      q.B[i] = in && hot ? __ldg(bp + o) : 0.0f;
+      const Off e = row + 32 * i - (decltype(wrap)::value && c + 32 * i >= W ? W : 0), o = 4 * e;
+      q.v[i] = in ? raw_bits<TYPE>(raw_ptr<TYPE>(raw + (Off)sizeof(*raw_ptr<TYPE>(nullptr)) * e)) : 0u;
+      q.g[i] = in && gain ? map(f.gain, o) : 0.0f;
+      q.A[i] = in && hot ? map(f.ha, o) : 0.0f;
+      q.B[i] = in && hot ? map(f.hb, o) : 0.0f;
     }
   };
   auto row_place = [&](int sy, int i, int q0, const SsRow<NQ>& q) {
     const int m = sy < 0 ? 0 : ncol - lane - 32 * q0;
+    if constexpr (VEC || AHEAD) {
 #pragma unroll
-    for (int j = 0; j < NQ; j++)
-      if (32 * j < m) put(i, lane + 32 * (q0 + j), bits_value<TYPE>(q.v[j]), q.g[j], q.A[j], q.B[j]);
+      for (int j = 0; j < NQ; j++)
+        if (32 * j < m) put(i, lane + 32 * (q0 + j), bits_value<TYPE>(q.v[j]), q.g[j], q.A[j], q.B[j]);
+    } else {  // one branch a correction (503 us for ten frames of 3838 x 3711, pixel by pixel 639)
+      float r[NQ];
+#pragma unroll
+      for (int j = 0; j < NQ; j++) r[j] = bits_value<TYPE>(q.v[j]);
+      if (gain) {
+#pragma unroll
+        for (int j = 0; j < NQ; j++) r[j] = __fmul_rn(q.g[j], r[j]);
+      }
+      if (MAPS >= SS_ANY && f.gdiv != 0.0f) {
+#pragma unroll
+        for (int j = 0; j < NQ; j++) r[j] = __fdiv_rn(r[j], f.gdiv);
+      }
+      if (hot) {
+#pragma unroll
+        for (int j = 0; j < NQ; j++) r[j] = __fmaf_rn(q.A[j], r[j], q.B[j]);
+      }
+      float* dst = &tile[i][4 + lane + 32 * q0];
+#pragma unroll
+      for (int j = 0; j < NQ; j++)
+        if (32 * j < m) dst[32 * j] = r[j];
+      if (edge && lane == 0 && q0 == 0 && m > 0) dst[-1] = r[0];  // column -1 reads column 0
+      if (last) {
+#pragma unroll
+        for (int j = 0; j < NQ; j++)
+          if (32 * j + 1 == m) dst[32 * j + 1] = r[j];  // column W reads column W - 1
+      }
+    }
   };
   SsRow<NQ> rw[AHEAD ? NR : 1];
   auto load_ahead = [&](int n, const zr_shift_t& t) {
@@ -388,23 +418,28 @@ struct SsArgs {
   cudaStream_t st;
 };
 
-template <int TYPE, bool VEC, int MAPS, int R>
+template <int TYPE, bool VEC, int MAPS, int R, int CTAS>
 static void launch_halves(const SsArgs& a, bool halves) {
   if (halves)
-    k_shift_sum<TYPE, VEC, MAPS, true, R><<<a.grid, SS_THR, 0, a.st>>>(a.f, a.shifts, a.sum, a.even, a.odd, a.aligned);
+    k_shift_sum<TYPE, VEC, MAPS, true, R, CTAS><<<a.grid, SS_THR, 0, a.st>>>(a.f, a.shifts, a.sum, a.even, a.odd,
+                                                                            a.aligned);
   else
-    k_shift_sum<TYPE, VEC, MAPS, false, R><<<a.grid, SS_THR, 0, a.st>>>(a.f, a.shifts, a.sum, a.even, a.odd, a.aligned);
+    k_shift_sum<TYPE, VEC, MAPS, false, R, CTAS><<<a.grid, SS_THR, 0, a.st>>>(a.f, a.shifts, a.sum, a.even, a.odd,
+                                                                             a.aligned);
 }
 
+// small: CTAs an SM of the kernel that loads a frame ahead, 0 for the other
 template <int TYPE>
-static void launch_shift(const SsArgs& a, bool vec, bool small, bool halves, int maps) {
-  if (small) return launch_halves<TYPE, false, SS_ANY, 1>(a, halves);
-  if (!vec) return launch_halves<TYPE, false, SS_ANY, 2>(a, halves);
+static void launch_shift(const SsArgs& a, bool vec, int small, bool halves, int maps) {
+  if (maps == SS_BIG) return launch_halves<TYPE, false, SS_BIG, 2, 5>(a, halves);
+  if (small == 2) return launch_halves<TYPE, false, SS_ANY, 1, 2>(a, halves);
+  if (small == 3) return launch_halves<TYPE, false, SS_ANY, 1, 3>(a, halves);
+  if (!vec) return launch_halves<TYPE, false, SS_ANY, 2, 5>(a, halves);
   switch (maps) {
-    case SS_NONE: return launch_halves<TYPE, true, SS_NONE, 2>(a, halves);
-    case SS_HOT: return launch_halves<TYPE, true, SS_HOT, 2>(a, halves);
-    case SS_GAIN_HOT: return launch_halves<TYPE, true, SS_GAIN_HOT, 2>(a, halves);
-    default: launch_halves<TYPE, true, SS_ANY, 2>(a, halves);
+    case SS_NONE: return launch_halves<TYPE, true, SS_NONE, 2, 6>(a, halves);
+    case SS_HOT: return launch_halves<TYPE, true, SS_HOT, 2, 6>(a, halves);
+    case SS_GAIN_HOT: return launch_halves<TYPE, true, SS_GAIN_HOT, 2, 6>(a, halves);
+    default: launch_halves<TYPE, true, SS_ANY, 2, 4>(a, halves);
   }
 }
 
@@ -424,17 +459,24 @@ extern "C" int zr_shift_sum(const zr_frames_t* frames, const zr_shift_t* shifts,
   // pixel index that is a multiple of 4
   const int qbytes = f.type == ZR_U8 ? 4 : (f.type == ZR_F32 ? 16 : 8);
   // (and pixel indices that fit an int)
-  const bool vec = (long long)f.H * f.W < (1LL << 31) - 1024 && f.fstride % 4 == 0 && ((uintptr_t)f.raw % qbytes) == 0 && ((uintptr_t)f.gain & 15) == 0 &&
+  const bool vec = f.fstride % 4 == 0 && ((uintptr_t)f.raw % qbytes) == 0 && ((uintptr_t)f.gain & 15) == 0 &&
                    ((uintptr_t)f.ha & 15) == 0 && ((uintptr_t)f.hb & 15) == 0;
   const bool halves = even_sum || odd_sum;
   // tiles of 16 rows; of 8, loading a frame ahead, where all of those run at
-  // once (above one wave they lose: 20 frames of 1536 x 1536 266 us against 168)
+  // once, two an SM (registers for the loads) or else three: 20 frames of 75 x
+  // 1031 34 us with two, 37 with three; 16 of 1665 x 167, 418 tiles, 43 us with
+  // three, 53 with two, 59 as 16-row tiles; above one wave they lose (20 frames
+  // of 1536 x 1536 266 us against 168)
   const int nx = (f.W + SS_TX - 1) / SS_TX;
-  const bool small = (long long)nx * ((f.H + 7) / 8) <= SS_WAVE;
+  const bool big = (long long)f.H * f.W >= (1LL << 30);
+  const long long tiles = (long long)nx * ((f.H + 7) / 8);
+  const int small = big ? 0 : (tiles <= 2 * SS_SMS ? 2 : (tiles <= 3 * SS_SMS ? 3 : 0));
   const dim3 grid(nx, small ? (f.H + 7) / 8 : (f.H + 15) / 16);
-  const int maps = f.gdiv != 0.0f ? SS_ANY
-                   : f.gain       ? (f.ha ? SS_GAIN_HOT : SS_ANY)
-                                  : (f.ha ? SS_HOT : SS_NONE);
+  // (byte offsets of pixels within 32 bits, for frames of less than 2^30)
+  const int maps = big              ? SS_BIG
+                   : f.gdiv != 0.0f ? SS_ANY
+                   : f.gain         ? (f.ha ? SS_GAIN_HOT : SS_ANY)
+                                    : (f.ha ? SS_HOT : SS_NONE);
   const SsArgs a{f, shifts, image_sum, even_sum, odd_sum, aligned, grid, st};
   switch (f.type) {
     case ZR_U8: launch_shift<ZR_U8>(a, vec, small, halves, maps); break;
