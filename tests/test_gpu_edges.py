@@ -1,0 +1,57 @@
+"""Calls at the edges of what the entry points take: buffers aligned to no
+more than an element, bounds in either order, every sub-pixel factor, the
+planner's choices, windows without a finite value, wide-ranging sums.
+
+What an input's alignment or the split between CTAs cannot change is held to
+equality; the other tolerances are derived at their tests."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from tests import gpu_helpers as gh
+from zorro_gb300 import _lib
+from zorro_gb300 import hostmath as hm
+
+pytestmark = pytest.mark.gpu
+
+
+def _init():
+    torch = gh.torch_mod()
+    _lib.call("zr_init", torch.cuda.current_device())
+    return torch, _lib.load()
+
+
+def _frames(raw, kind, maps=(None, None, None)):
+    N, H, W = raw.shape
+    return _lib.Frames(raw.data_ptr(), kind, *(None if m is None else m.data_ptr() for m in maps), 0.0, N, H, W, 0)
+
+
+@pytest.mark.parametrize("H,W", [(40, 130), (33, 258), (2600, 300), (50, 127)])
+@pytest.mark.parametrize("halves", [False, True])
+def test_shift_sum_aligned_frames_at_any_float(H, W, halves):
+    """The aligned frames go to any float-aligned buffer: one float past a
+    256-byte boundary they hold the same bits as on it (even widths, whose
+    rows are stored in pairs there, tiles of 8 and of 16 rows, and an odd
+    width)."""
+    torch, _ = _init()
+    rng = np.random.default_rng(H * W)
+    N = 3
+    raw = torch.from_numpy(rng.poisson(4.0, (N, H, W)).astype(np.uint8)).cuda()
+    fr = _frames(raw, _lib.ZR_U8)
+    t = np.round(16 * rng.uniform(-5, 5, (N, 2))) / 16
+    sh = torch.from_numpy(hm.shift_table(t, H, W).view(np.uint8)).cuda()
+    got = []
+    for skip in (0, 1):
+        arena = torch.full((N * H * W + 64,), 7.0, device="cuda")
+        assert arena.data_ptr() % 256 == 0
+        out = torch.empty(3, H, W, device="cuda")
+        even, odd = (out[1].data_ptr(), out[2].data_ptr()) if halves else (None, None)
+        _lib.call("zr_shift_sum", C.byref(fr), sh.data_ptr(), out[0].data_ptr(), even, odd,
+                  arena.data_ptr() + 4 * skip, gh.stream())
+        torch.cuda.synchronize()
+        rest = torch.cat([arena[:skip], arena[skip + N * H * W:]])
+        assert bool((rest == 7.0).all())
+        got.append((arena[skip:skip + N * H * W].clone(), out[:3 if halves else 1].clone()))
+    for a, b in zip(*got):
+        assert torch.equal(a, b)

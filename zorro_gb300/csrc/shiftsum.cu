@@ -160,7 +160,8 @@ __global__ void __launch_bounds__(SS_THR, CTAS)
   row_table(0);
   __syncthreads();
   const int nrow = min(R, H - (y0 + ly0));              // output rows of this warp inside the image
-  const bool pairs = x + 4 <= W && (W & 1) == 0;        // rows start on 8 bytes
+  // rows of the aligned frames start on 8 bytes (any float-aligned buffer is taken)
+  const bool pairs = x + 4 <= W && (W & 1) == 0 && (reinterpret_cast<uintptr_t>(aligned) & 7) == 0;
   constexpr int NR = (TH + 7) / 8;  // tile rows a warp reads
   constexpr bool AHEAD = R == 1;    // loads a frame ahead
   static_assert(!(AHEAD && VEC), "pixel by pixel");
