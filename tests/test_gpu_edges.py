@@ -55,3 +55,26 @@ def test_shift_sum_aligned_frames_at_any_float(H, W, halves):
         got.append((arena[skip:skip + N * H * W].clone(), out[:3 if halves else 1].clone()))
     for a, b in zip(*got):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("H,W,Hb,Wb", [(601, 640, 560, 562), (1100, 1024, 1026, 514), (2048, 3072, 1024, 1536)])
+def test_binning_work_at_any_element(H, W, Hb, Wb):
+    """``work`` holds complex floats and needs their alignment only: eight
+    bytes past a 256-byte boundary the binned frames are the same bits (odd
+    and even heights, chirp and direct sides), and nothing is written past
+    zr_bin_work_bytes."""
+    torch, lib = _init()
+    rng = np.random.default_rng(H)
+    raw = torch.from_numpy(rng.poisson(2.0, (2, H, W)).astype(np.uint8)).cuda()
+    fr = _frames(raw, _lib.ZR_U8)
+    wb = lib.zr_bin_work_bytes(H, W, Hb, Wb)
+    got = []
+    for skip in (0, 8):
+        arena = torch.full((wb + 256,), 165, dtype=torch.uint8, device="cuda")
+        assert arena.data_ptr() % 256 == 0
+        out = torch.empty(2, Hb, Wb, device="cuda")
+        _lib.call("zr_bin_fourier", C.byref(fr), Hb, Wb, out.data_ptr(), arena.data_ptr() + skip, wb, gh.stream())
+        torch.cuda.synchronize()
+        assert bool((arena[:skip] == 165).all()) and bool((arena[skip + wb:] == 165).all())
+        got.append(out)
+    assert torch.equal(*got)

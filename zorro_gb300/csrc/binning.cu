@@ -118,7 +118,9 @@ extern "C" int zr_bin_fourier(const zr_frames_t* frames, int Hb, int Wb, float* 
     return d;
   };
   const BnSide dw = side(W, 2 * b1 + 1), dh = side(H, 2 * b0 + 1), dhb = side(Hb, Hb), dwb = side(Wb, Wb);
-  auto even = [&](float2* p) { return p + ((p - (float2*)work) & 1); };  // 16-byte boundaries
+  // 16-byte boundaries of the address space (``work`` itself is aligned to a
+  // float2 only); zr_bin_work_bytes has the spare element of each
+  auto even = [](float2* p) { return p + (((uintptr_t)p & 15) != 0); };
   float2* Ct = even(w);
   float2* Cc = Ct + (size_t)H * Kb;
   float2* Ci = even(Cc + (size_t)(Hb + 1) * Kb);
