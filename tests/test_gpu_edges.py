@@ -78,3 +78,41 @@ def test_binning_work_at_any_element(H, W, Hb, Wb):
         assert bool((arena[:skip] == 165).all()) and bool((arena[skip + wb:] == 165).all())
         got.append(out)
     assert torch.equal(*got)
+
+
+def _windows(rng, M, mS):
+    """Noise with a broad peak off the centre."""
+    y = np.arange(2 * mS) - mS
+    at = rng.uniform(-0.3, 0.3, (M, 2)) * mS
+    r2 = (y[None, :, None] - at[:, 0, None, None]) ** 2 + (y[None, None, :] - at[:, 1, None, None]) ** 2
+    win = rng.normal(0, 1, (M, 2 * mS, 2 * mS)) + 8.0 * np.exp(-r2 / 18.0)
+    return (1e-3 * win).astype(np.float32)
+
+
+def _locate(win, mS, **kw):
+    torch, _ = _init()
+    p = dict(sub_pix_reg=16, bmode=1, suppress_origin=1, use_mask=1, conv_sigma_y=0.0, conv_sigma_x=0.0, opti_lo=0.0,
+             opti_hi=7.0, opti_xatol=0.01, opti_maxiter=15)
+    p.update(kw)
+    pp = _lib.PeakParams(**p)
+    dev = torch.from_numpy(np.ascontiguousarray(win, dtype=np.float32)).cuda()
+    out = torch.zeros((len(win), C.sizeof(_lib.PeakResult)), dtype=torch.uint8, device="cuda")
+    _lib.call("zr_locate_peaks", dev.data_ptr(), len(win), mS, C.byref(pp), out.data_ptr(), gh.stream())
+    torch.cuda.synchronize()
+    return np.frombuffer(out.cpu().numpy().tobytes(), dtype=gh.PEAK_DTYPE)
+
+
+@pytest.mark.parametrize("lo,hi", [(7.0, 0.0), (20.0, 1.0), (15.9, 15.8)])
+@pytest.mark.parametrize("mS,M", [(20, 3), (25, 3), (50, 20), (111, 2), (33, 160)])
+def test_opti_bounds_in_either_order(mS, M, lo, hi):
+    """With opti_lo > opti_hi the bounded search ends at its first abscissa
+    (FMM FMIN's test holds there), which may lie far above opti_hi: the records
+    are those of that sigma given to bmode 2."""
+    win = _windows(np.random.default_rng(mS), M, mS)
+    got = _locate(win, mS, opti_lo=lo, opti_hi=hi)
+    sigma = got["sigma"][0]
+    assert np.all(got["nfev"] == 1) and np.all(got["sigma"] == sigma)
+    assert abs(sigma - (lo + 0.5 * (3.0 - 5.0 ** 0.5) * (hi - lo))) < 1e-12
+    want = _locate(win, mS, bmode=2, conv_sigma_y=sigma, conv_sigma_x=sigma)
+    for k in ("sy", "sx", "corr", "peaksig", "origin", "cy", "cx", "flags"):
+        assert np.array_equal(got[k], want[k]), k

@@ -1455,9 +1455,11 @@ extern "C" int zr_locate_peaks(const float* cwin, int M, int max_shift, const zr
   if (!tw) return ZR_ECUDA;
   // shared memory: the window, then V (the filter blocks; also the vertical
   // pass of the 16 x 16 sub-pixel patch)
-  double smax = params->bmode == 1 ? params->opti_hi : 0.0;
+  // (every sigma of the bounded search lies between its bounds, in either order;
+  // gauss_weights cuts radii off at PK_MAXR)
+  double smax = params->bmode == 1 ? fmax(params->opti_lo, params->opti_hi) : 0.0;
   if (params->bmode == 2) smax = fmax(params->conv_sigma_y, params->conv_sigma_x);
-  const int pad = ((int)(4.0 * fmax(smax, 0.0) + 0.5) + 3) & ~3;
+  const int pad = ((int)fmin(4.0 * fmax(smax, 0.0) + 0.5, (double)PK_MAXR) + 3) & ~3;
   const size_t win = (((size_t)w * w + 3) & ~(size_t)3) * sizeof(float);
   const size_t sub = (size_t)17 * 16 * params->sub_pix_reg * sizeof(float2);
   const size_t base = params->sub_pix_reg > 1 && win < sub ? sub : win;  // the sub-pixel step's scratch takes the window
