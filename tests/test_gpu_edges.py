@@ -116,3 +116,34 @@ def test_opti_bounds_in_either_order(mS, M, lo, hi):
     want = _locate(win, mS, bmode=2, conv_sigma_y=sigma, conv_sigma_x=sigma)
     for k in ("sy", "sx", "corr", "peaksig", "origin", "cy", "cx", "flags"):
         assert np.array_equal(got[k], want[k]), k
+
+
+@pytest.mark.parametrize("sp", [3, 5, 6, 9, 12, 15, 20, 24, 30])
+@pytest.mark.parametrize("flat", [False, True])
+def test_subpixel_factors_that_are_no_power_of_two(sp, flat):
+    """Every sub-pixel factor that is taken finds the largest value of the
+    upsampled patch, by the quick search and term by term (a flat window):
+    within the 64 roundings of sum |F| that test_subpixel_maximum derives."""
+    rng = np.random.default_rng(sp)
+    mS, M, L = 14, 6, 16 * sp
+    win = _windows(rng, M, mS)
+    if flat:
+        win[:] = 1.0
+        win[:, mS, mS] = np.nextafter(np.float32(1.0), np.float32(2.0))
+    f = np.concatenate([np.arange(8), np.arange(-8, 0)])
+    E = np.exp(2j * np.pi * np.outer(np.arange(L), f) / L)
+    inside = 0
+    for k, r in enumerate(_locate(win, mS, sub_pix_reg=sp, bmode=0, suppress_origin=0)):
+        cy, cx = int(r["cy"]), int(r["cx"])
+        if not (8 <= cy <= 2 * mS - 8 and 8 <= cx <= 2 * mS - 8):
+            continue
+        inside += 1
+        F = np.fft.fft2(win[k, cy - 8:cy + 8, cx - 8:cx + 8].astype(np.float64))
+        V = np.abs(E @ F @ E.T)
+        tol = 64 * 2.0 ** -24 * np.abs(F).sum()
+        at = [(r[n] - (c - mS)) * sp + L / 2 - np.sign(c - mS) for n, c in (("sy", cy), ("sx", cx))]
+        sy, sx = (int(round(v)) for v in at)
+        assert np.allclose(at, (sy, sx), atol=1e-9) and 0 <= sy < L and 0 <= sx < L
+        assert V[sy, sx] >= V.max() - 2 * tol
+        assert abs(256 * float(r["corr"]) - V[sy, sx]) <= tol
+    assert inside >= 4

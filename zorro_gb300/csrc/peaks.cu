@@ -753,8 +753,9 @@ __device__ void subpix_search(const float* patch, int sp, const float2* __restri
   // frequencies f zero-padded to L are, for every a, a 16-point transform over
   // b of the inputs times exp(2 pi i f a / L).
   auto sixteenth = [&](const float2* in, int step, int a, float2 (&v)[16]) {
+    const int up = a > 0 ? L : 0;  // a < sp: |f a| < L
 #pragma unroll
-    for (int f = 0; f < 16; f++) v[f] = cmul(in[f * step], Wl[((f < 8 ? f : f - 16) * a) & (L - 1)]);
+    for (int f = 0; f < 16; f++) v[f] = cmul(in[f * step], Wl[f < 8 ? f * a : (f - 16) * a + up]);
     ip_dft<16, 1>(v);
   };
   if (threadIdx.x < 16 * sp) {
@@ -801,12 +802,19 @@ __device__ void subpix_search(const float* patch, int sp, const float2* __restri
     const float mag = sqrtf(fmaf(acc.x, acc.x, __fmul_rn(acc.y, acc.y)));
     if (mag > bv || (mag == bv && e < bi)) { bv = mag; bi = e; }
   };
+  // m mod L (L need not be a power of two: 16 sp divides TWN)
+  const bool pow2 = (L & (L - 1)) == 0;
+  auto turn = [&](int m) {
+    if (pow2) return m & (L - 1);
+    m %= L;
+    return m < 0 ? m + L : m;
+  };
   // row fyi of the intermediate, and the plane from it, term by term
   auto row_term = [&](int fyi, int nx) {
     float2 acc = make_float2(0.0f, 0.0f);
     for (int fxi = 0; fxi < 16; fxi++) {
       const int fx = fxi - 8;
-      acc = cadd(acc, cmul_rn(patchF[((fyi - 8) & 15) * 16 + (fx & 15)], Wl[(fx * nx) & (L - 1)]));
+      acc = cadd(acc, cmul_rn(patchF[((fyi - 8) & 15) * 16 + (fx & 15)], Wl[turn(fx * nx)]));
     }
     return acc;
   };
@@ -819,7 +827,7 @@ __device__ void subpix_search(const float* patch, int sp, const float2* __restri
       float2 acc = make_float2(0.0f, 0.0f);
       for (int fyi = 0; fyi < 16; fyi++) {
         const float2 r = make_float2(__shfl_sync(0xffffffffu, t.x, fyi), __shfl_sync(0xffffffffu, t.y, fyi));
-        acc = cadd(acc, cmul_rn(r, Wl[((fyi - 8) * ny) & (L - 1)]));
+        acc = cadd(acc, cmul_rn(r, Wl[turn((fyi - 8) * ny)]));
       }
       take(acc, e);
     }
@@ -829,7 +837,7 @@ __device__ void subpix_search(const float* patch, int sp, const float2* __restri
     for (int e = threadIdx.x; e < L * L; e += PK_T) {
       const int ny = e / L, nx = e - ny * L;
       float2 acc = make_float2(0.0f, 0.0f);
-      for (int fyi = 0; fyi < 16; fyi++) acc = cadd(acc, cmul_rn(Tx[fyi * L + nx], Wl[((fyi - 8) * ny) & (L - 1)]));
+      for (int fyi = 0; fyi < 16; fyi++) acc = cadd(acc, cmul_rn(Tx[fyi * L + nx], Wl[turn((fyi - 8) * ny)]));
       take(acc, e);
     }
   }
@@ -1446,7 +1454,7 @@ extern "C" int zr_locate_peaks(const float* cwin, int M, int max_shift, const zr
   if (max_shift < 8 || max_shift > 112)
     return set_error(ZR_ESIZE, "zr_locate_peaks: maxShift %d outside [8, 112]", max_shift);
   if (params->sub_pix_reg > 1 && (TWN % (16 * params->sub_pix_reg) != 0 || 16 * params->sub_pix_reg > 512))
-    return set_error(ZR_ESIZE, "zr_locate_peaks: subPixReg %d must be a power of two <= 32", params->sub_pix_reg);
+    return set_error(ZR_ESIZE, "zr_locate_peaks: subPixReg %d must be at most 32 and divide 2^10 * 3^2 * 5", params->sub_pix_reg);
   if (params->bmode == 2 && (4.0 * params->conv_sigma_y + 0.5 > PK_MAXR || 4.0 * params->conv_sigma_x + 0.5 > PK_MAXR))
     return set_error(ZR_ESIZE, "zr_locate_peaks: conv sigma too large");
   if (params->bmode == 1 && 4.0 * params->opti_hi + 0.5 > PK_MAXR)
@@ -1531,7 +1539,7 @@ extern "C" int zr_full_peaks(const float* planes, const float* filtered, int n_p
   if (n_sel <= 0) return ZR_OK;
   if (n_sel > n_planes || C < 32 || C > 8192 || max_shift <= 0) return set_error(ZR_EINVAL, "zr_full_peaks: bad sizes");
   if (sub_pix_reg > 1 && (TWN % (16 * sub_pix_reg) != 0 || 16 * sub_pix_reg > 512))
-    return set_error(ZR_ESIZE, "zr_full_peaks: subPixReg %d must be a power of two <= 32", sub_pix_reg);
+    return set_error(ZR_ESIZE, "zr_full_peaks: subPixReg %d must be at most 32 and divide 2^10 * 3^2 * 5", sub_pix_reg);
   if (work_bytes < zr_full_work_bytes(n_planes, C))
     return set_error(ZR_EWORK, "zr_full_peaks: work buffer %zu < %zu", work_bytes, zr_full_work_bytes(n_planes, C));
   const float2* tw = twiddles();
