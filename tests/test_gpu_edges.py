@@ -147,3 +147,41 @@ def test_subpixel_factors_that_are_no_power_of_two(sp, flat):
         assert V[sy, sx] >= V.max() - 2 * tol
         assert abs(256 * float(r["corr"]) - V[sy, sx]) <= tol
     assert inside >= 4
+
+
+@pytest.mark.parametrize("mS,M", [(20, 1), (20, 160), (25, 3)])
+@pytest.mark.parametrize("spike", [2.4e19, 1e20])
+def test_opti_search_avoids_infinite_statistics(mS, M, spike):
+    """Where the filtered window's sum of squares passes float32's range (the
+    sums are float32 within a warp of statistics threads, float64 across the
+    warps) its contrast is infinite and the search turns away from it: the
+    sigma found is that of the search over the float64 statistics with infinity
+    in those places.  (Both stop at the edge of that range; the abscissas there
+    lie within the search's xatol of 0.01 of one another, held to twice that.)"""
+    import scipy.ndimage
+    rng = np.random.default_rng(mS)
+    w = 2 * mS
+    win = 1e16 * rng.standard_normal((w, w))
+    win[mS + 1, mS - 2] = spike
+    win = win.astype(np.float32)
+    # the statistics thread of each pixel: rows 2 ty, 2 ty + 1 and columns 4 tx
+    # .. 4 tx + 3, or rows y mod 16 = ty and columns tx mod 64
+    y, x = np.mgrid[:w, :w]
+    warp = ((y // 2 % (4096 // w) * (w // 4) + x // 4) if w % 4 == 0 else (y % 16 * 64 + x % 64)) // 32
+    search = hm.brent_bounded(0.0, 7.0, 0.01, 15)
+    seen = []
+    s = next(search)
+    try:
+        while True:
+            F = scipy.ndimage.gaussian_filter(win.astype(np.float64), s)
+            d = F - win.mean(dtype=np.float64)
+            most = np.bincount(warp.ravel(), (d * d).ravel()).max()
+            f = np.sqrt(d.var()) / (F.max() - F.mean()) if most < 3.4028235e38 else np.inf
+            seen.append(f)
+            s = search.send(f)
+    except StopIteration as e:
+        sigma = e.value[0]
+    assert np.inf in seen
+    got = _locate(np.repeat(win[None], M, 0), mS, suppress_origin=0)
+    assert np.all(np.abs(got["sigma"] - sigma) <= 0.02), (got["sigma"][0], sigma)
+    assert np.all((got["cy"] == mS + 1) & (got["cx"] == mS - 2))

@@ -571,31 +571,17 @@ __device__ PkSums filter_rows(const float* C, float* V, const PkRows& L, int mS,
   return a;
 }
 
-// a / b from a reciprocal r of b good to a few units in the last place: the
-// quotient's remainder folded back once, which rounds it correctly.
-__device__ __forceinline__ double div_by(double a, double b, double r) {
-  const double q = a * r;
-  return fma(fma(-q, b, a), r, q);
-}
-
-// std(G_sigma * C) / (max - mean) from the statistics (zorro.py:1108-1121).
-// The warp that holds them calls, lane 0 gets the value.  The square root of
-// the variance and the division by the difference start from two reciprocal
-// square roots side by side on lanes 0 and 1 (1 / |d| = rsqrt(d d)), and the
-// divisions by n (rn = 1 / n) from rn: 1400 cycles instead of four operations
-// of 570 to 590 in a row, the same roundings.
-__device__ __forceinline__ double objective(const FiltStats& st, float c, double n, double rn) {
-  const double m1 = div_by(st.s1, n, rn);
-  const double var = div_by(st.s2, n, rn) - m1 * m1;
+// std(G_sigma * C) / (max - mean) from the statistics (zorro.py:1108-1121), in
+// float64's own divisions and square root: the search branches on the value,
+// and sums of squares beyond float32's range have to give infinity.  (Quotients
+// and the root from reciprocal square roots and one remainder step, which are
+// not always rounded so, took 149.0 us a lone window against 153.4, 643 against
+// 648 for 190 K2 windows.)
+__device__ __forceinline__ double objective(const FiltStats& st, float c, double n) {
+  const double m1 = st.s1 / n;
+  const double var = st.s2 / n - m1 * m1;
   const double mean = (double)c + m1;
-  const double d = __shfl_sync(0xffffffffu, (double)st.mx - mean, 0);
-  const double v = __shfl_sync(0xffffffffu, var > 0.0 ? var : 0.0, 0);
-  const double q = rsqrt((threadIdx.x & 31) == 0 ? v : d * d);
-  const double rd = copysign(__shfl_sync(0xffffffffu, q, 1), d);
-  double sd = v * q;  // sqrt(v), one correction
-  sd = fma(fma(-sd, sd, v), 0.5 * q, sd);
-  const double f = div_by(sd, d, rd);
-  return fabs(f) < INFINITY ? f : sqrt(v) / d;  // zero, infinite or NaN terms
+  return sqrt(var > 0.0 ? var : 0.0) / ((double)st.mx - mean);
 }
 
 __device__ __forceinline__ double sgn1(double v) { return v > 0.0 ? 1.0 : (v < 0.0 ? -1.0 : 1.0); }
@@ -851,7 +837,7 @@ __device__ void subpix_search(const float* patch, int sp, const float2* __restri
 // two cluster barriers per function value.
 template <int S>
 __global__ void __launch_bounds__(PK_T, 1) k_peaks(const float* __restrict__ cwin, int mS, zr_peak_params_t p,
-                                               int pad, int vfloats, double xatol3, double rn, zr_peak_result_t* __restrict__ res,
+                                               int pad, int vfloats, double xatol3, zr_peak_result_t* __restrict__ res,
                                                const float2* __restrict__ tw) {
   extern __shared__ __align__(16) float smf[];
   __shared__ PkShared sh;
@@ -988,15 +974,15 @@ __global__ void __launch_bounds__(PK_T, 1) k_peaks(const float* __restrict__ cwi
       gather(a, Mode0());
       if (rank == 0 && warp == 0) {
         const FiltStats st = stats_total(sh);
-        const double f = objective(st, c, (double)w2, rn);
         if (threadIdx.x == 0) {
+          const double f = objective(st, c, (double)w2);
           if (first) brent_begin(sh, p.opti_lo, p.opti_hi, xatol3, x0, f);
           else brent_step(sh, xatol3, p.opti_maxiter, f);
         }
         __syncwarp();
         if (sh.go) {
-          const int rn = gauss_weights(sh.x, sh.wy);
-          if (threadIdx.x == 0) sh.r = rn;
+          const int next = gauss_weights(sh.x, sh.wy);
+          if (threadIdx.x == 0) sh.r = next;
         }
       }
       share();
@@ -1436,7 +1422,7 @@ static int launch_peaks(const float* cwin, int M, int mS, const zr_peak_params_t
   cfg.attrs = at;
   cfg.numAttrs = S > 1 ? 1 : 0;
   ZR_TRY(cuda_check(cudaLaunchKernelEx(&cfg, k_peaks<S>, cwin, mS, p, pad, vfloats, p.opti_xatol / 3.0,
-                                       1.0 / (4.0 * mS * mS), res, tw), "k_peaks launch"));
+                                       res, tw), "k_peaks launch"));
   return launched("k_peaks");
 }
 
