@@ -185,3 +185,50 @@ def test_opti_search_avoids_infinite_statistics(mS, M, spike):
     got = _locate(np.repeat(win[None], M, 0), mS, suppress_origin=0)
     assert np.all(np.abs(got["sigma"] - sigma) <= 0.02), (got["sigma"][0], sigma)
     assert np.all((got["cy"] == mS + 1) & (got["cx"] == mS - 2))
+
+
+@pytest.mark.parametrize("mS,M", [(20, 1), (20, 160), (25, 3), (100, 9)])
+@pytest.mark.parametrize("bmode,use_mask", [(0, 0), (0, 1), (1, 0), (2, 0)])
+def test_windows_of_nan(mS, M, bmode, use_mask):
+    """A window without a number in it has its peak at np.argmax's index 0,
+    the window's corner, where there is no sub-pixel step; a patch with a NaN
+    has its sub-pixel maximum at index 0 too.  Windows beside them keep their
+    records."""
+    win = _windows(np.random.default_rng(mS), M, mS)
+    kw = dict(bmode=bmode, use_mask=use_mask, conv_sigma_y=1.3, conv_sigma_x=1.3, suppress_origin=0)
+    clean = _locate(win, mS, **kw)
+    win[0] = np.nan
+    got = _locate(win, mS, **kw)
+    assert (got["cy"][0], got["cx"][0], got["flags"][0]) == (0, 0, 1)
+    assert (got["sy"][0], got["sx"][0]) == (-mS, -mS)
+    assert np.isnan(got["corr"][0]) and np.isnan(got["peaksig"][0]) and np.isnan(got["origin"][0])
+    assert got[1:].tobytes() == clean[1:].tobytes()
+    if bmode == 0:
+        win[0] = 0.0
+        win[0, mS, mS + 1], win[0, mS + 3, mS + 3] = 1.0, np.nan
+        got = _locate(win, mS, **kw)[0]
+        assert (got["cy"], got["cx"], got["flags"]) == (mS, mS + 1, 0) and np.isnan(got["corr"])
+        assert (got["sy"], got["sx"]) == (-8.0, 1.0 + (1.0 - 128.0) / 16)
+
+
+def test_whole_planes_of_nan():
+    """The same for a plane that lies inside the search disc as a whole."""
+    torch, lib = _init()
+    n, Cc = 2, 32
+    P = torch.full((n, Cc, Cc), float("nan"), device="cuda")
+    P[1] = 0.0
+    P[1, 20, 12] = 1.0
+    wb = lib.zr_full_work_bytes(n, Cc)
+    work = torch.empty(wb, dtype=torch.uint8, device="cuda")
+    sel = torch.arange(n, dtype=torch.int32, device="cuda")
+    rolls = torch.zeros(n, 2, dtype=torch.int32, device="cuda")
+    mean, origin = torch.zeros(n, device="cuda"), torch.zeros(n, device="cuda")
+    sigma, nfev = torch.ones(n, dtype=torch.float64, device="cuda"), torch.ones(n, dtype=torch.int32, device="cuda")
+    out = torch.zeros((n, C.sizeof(_lib.PeakResult)), dtype=torch.uint8, device="cuda")
+    _lib.call("zr_full_peaks", P.data_ptr(), P.data_ptr(), n, Cc, sel.data_ptr(), n, 64, rolls.data_ptr(),
+              mean.data_ptr(), origin.data_ptr(), sigma.data_ptr(), nfev.data_ptr(), 16, out.data_ptr(),
+              work.data_ptr(), wb, gh.stream())
+    torch.cuda.synchronize()
+    r = np.frombuffer(out.cpu().numpy().tobytes(), dtype=gh.PEAK_DTYPE)
+    assert (r["cy"].tolist(), r["cx"].tolist(), r["flags"].tolist()) == ([0, 20], [0, 12], [1, 0])
+    assert np.isnan(r["corr"][0]) and abs(r["corr"][1] - 1.0) < 1e-5

@@ -129,7 +129,8 @@ __device__ double3 block_sum3(PkShared& sh, double a, double b, double c) {
   return r;
 }
 
-// max value with the smallest index among equal values
+// max value with the smallest index among equal values; where no thread has
+// one (all of them NaN), NaN and index 0, as np.argmax has it
 __device__ void block_argmax(PkShared& sh, float& v, int& idx) {
   for (int o = 16; o > 0; o >>= 1) {
     const float ov = __shfl_down_sync(0xffffffffu, v, o);
@@ -147,7 +148,11 @@ __device__ void block_argmax(PkShared& sh, float& v, int& idx) {
       const int oi = __shfl_down_sync(0xffffffffu, idx, o);
       if (ov > v || (ov == v && oi < idx)) { v = ov; idx = oi; }
     }
-    if (lane == 0) { sh.bc[3] = v; sh.bi[0] = idx; }
+    if (lane == 0) {
+      const bool none = idx == 0x7fffffff;
+      sh.bc[3] = none ? nan("") : (double)v;
+      sh.bi[0] = none ? 0 : idx;
+    }
   }
   __syncthreads();
   v = (float)sh.bc[3];
@@ -1345,6 +1350,10 @@ __global__ void __launch_bounds__(PK_T, 1) k_full_finish(const float* __restrict
       s1 += r[2];
       s2 += r[3];
       cnt += r[4];
+    }
+    if (bi == 0x7fffffff) {  // a plane of NaN, all of it inside the disc
+      bv = nan("");
+      bi = 0;
     }
     const double m1 = s1 / cnt;
     const double var = s2 / cnt - m1 * m1;
