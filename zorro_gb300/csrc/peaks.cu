@@ -47,6 +47,7 @@ struct BrentState {
 struct PkShared {
   alignas(16) float wy[2 * PK_MAXR + 4];  // 16-byte aligned: read four taps at a time
   alignas(16) float wx[2 * PK_MAXR + 4];
+  alignas(16) float ws[2 * PK_MAXR + 4];  // the search's weights, both axes
   double red[PK_NW][3];
   float redf[PK_NW];
   int redi[PK_NW];
@@ -57,6 +58,7 @@ struct PkShared {
   double x;             // the Brent search's next abscissa
   int go;               // 1 while the search continues
   int r;                // filter radius of the current sigma
+  int ry, rx;           // radii of the last filter
   BrentState bs;        // the search's state (thread 0 only)
 };
 
@@ -935,21 +937,31 @@ __global__ void __launch_bounds__(PK_T, 1) k_peaks(const float* __restrict__ cwi
     }
     __syncthreads();
   };
-  // CTA 0's weights (wy, r and go) for every CTA of the window
-  auto share = [&]() {
+  // CTA 0's weights and radii for every CTA of the window: the search's (ws, r
+  // and go) or the last filter's (wy, wx, ry, rx).  They are kept apart because
+  // CTA 0 writes the last filter's while the others still read the search's end.
+  auto share = [&](auto search) {
     if constexpr (S > 1) {
       cg::cluster_group cl = cg::this_cluster();
       cl.sync();
       if (rank != 0) {
         const PkShared* lead = cl.map_shared_rank(&sh, 0);
         for (int i = threadIdx.x; i < 2 * PK_MAXR + 4; i += PK_T) {
-          sh.wy[i] = lead->wy[i];
-          sh.wx[i] = lead->wx[i];
+          if constexpr (decltype(search)::value) {
+            sh.ws[i] = lead->ws[i];
+          } else {
+            sh.wy[i] = lead->wy[i];
+            sh.wx[i] = lead->wx[i];
+          }
         }
         if (threadIdx.x == 0) {
-          sh.r = lead->r;
-          sh.bi[0] = lead->bi[0];
-          sh.go = lead->go;
+          if constexpr (decltype(search)::value) {
+            sh.r = lead->r;
+            sh.go = lead->go;
+          } else {
+            sh.ry = lead->ry;
+            sh.rx = lead->rx;
+          }
         }
       }
       __syncthreads();
@@ -966,16 +978,16 @@ __global__ void __launch_bounds__(PK_T, 1) k_peaks(const float* __restrict__ cwi
   if (p.bmode == 1) {
     const double x0 = brent_first(p.opti_lo, p.opti_hi);
     if (rank == 0 && warp == 0) {
-      const int r = gauss_weights(x0, sh.wy);
+      const int r = gauss_weights(x0, sh.ws);
       if (threadIdx.x == 0) {
         sh.r = r;
         sh.go = 1;
       }
     }
-    share();
+    share(std::true_type());
     for (bool first = true; sh.go; first = false) {
       const int r = sh.r;
-      const PkSums a = filter_rows<0, ROUNDS>(C, V, lay, mS, r, r, sh.wy, sh.wy, c, false);
+      const PkSums a = filter_rows<0, ROUNDS>(C, V, lay, mS, r, r, sh.ws, sh.ws, c, false);
       gather(a, Mode0());
       if (rank == 0 && warp == 0) {
         const FiltStats st = stats_total(sh);
@@ -986,11 +998,11 @@ __global__ void __launch_bounds__(PK_T, 1) k_peaks(const float* __restrict__ cwi
         }
         __syncwarp();
         if (sh.go) {
-          const int next = gauss_weights(sh.x, sh.wy);
+          const int next = gauss_weights(sh.x, sh.ws);
           if (threadIdx.x == 0) sh.r = next;
         }
       }
-      share();
+      share(std::true_type());
     }
     sig_opt = sh.x;  // CTA 0
     nfev = sh.bi[1];
@@ -1001,12 +1013,12 @@ __global__ void __launch_bounds__(PK_T, 1) k_peaks(const float* __restrict__ cwi
     const int a = gauss_weights(sy, sh.wy);
     const int b = gauss_weights(sx, sh.wx);
     if (threadIdx.x == 0) {
-      sh.r = a;
-      sh.bi[0] = b;
+      sh.ry = a;
+      sh.rx = b;
     }
   }
-  share();
-  const int ry = sh.r, rx = sh.bi[0];
+  share(std::false_type());
+  const int ry = sh.ry, rx = sh.rx;
   const PkSums sums = filter_rows<1, ROUNDS>(C, V, lay, mS, ry, rx, sh.wy, sh.wx, c, p.use_mask != 0);
   gather(sums, Mode1());
   if constexpr (S > 1) {
