@@ -232,3 +232,14 @@ def test_whole_planes_of_nan():
     r = np.frombuffer(out.cpu().numpy().tobytes(), dtype=gh.PEAK_DTYPE)
     assert (r["cy"].tolist(), r["cx"].tolist(), r["flags"].tolist()) == ([0, 20], [0, 12], [1, 0])
     assert np.isnan(r["corr"][0]) and abs(r["corr"][1] - 1.0) < 1e-5
+
+
+@pytest.mark.parametrize("mS", [8, 9, 25, 47, 48])
+def test_one_windows_record_at_any_number(mS):
+    """Around a wave of 152 windows, and on both sides of the size from which
+    windows are split over CTAs, a window's record is the one it has alone."""
+    win = _windows(np.random.default_rng(mS), 154, mS)
+    whole = _locate(win, mS)
+    for k in (0, 1, 152, 153):
+        assert _locate(win[k:k + 1], mS).tobytes() == whole[k:k + 1].tobytes(), k
+    assert _locate(win[:153], mS).tobytes() == whole[:153].tobytes()

@@ -1483,8 +1483,13 @@ extern "C" int zr_locate_peaks(const float* cwin, int M, int max_shift, const zr
   if (vbytes > (size_t)64 * 1024) vbytes = 64 * 1024;
   const int vfloats = (int)(vbytes / sizeof(float));
   cudaStream_t st = (cudaStream_t)stream;
-  // Full waves of one CTA per window and SM, then what is left with as many
-  // CTAs per window as fit the SMs
+  // Windows below 96 pixels, each a CTA: two cluster barriers a function value
+  // take longer than the rows they share out (20 windows of 40 x 40 169 us, 193
+  // in clusters of two, 191 of four; of 82 x 82 201, 208 and 201; of 96 x 96
+  // 199, 197 and 181; of 100 x 100 208, 191 and 171).  Larger ones: full waves of
+  // one CTA per window and SM, then what is left with as many CTAs per window as
+  // fit the SMs.
+  if (w < 96) return launch_peaks<1>(cwin, M, max_shift, *params, pad, vfloats, base + vbytes, results, tw, st);
   const int full = M / PK_SMS * PK_SMS, rest = M - full;
   if (full) ZR_TRY(launch_peaks<1>(cwin, full, max_shift, *params, pad, vfloats, base + vbytes, results, tw, st));
   cwin += (size_t)full * w * w;
