@@ -243,3 +243,88 @@ def test_one_windows_record_at_any_number(mS):
     for k in (0, 1, 152, 153):
         assert _locate(win[k:k + 1], mS).tobytes() == whole[k:k + 1].tobytes(), k
     assert _locate(win[:153], mS).tobytes() == whole[:153].tobytes()
+
+
+class _KernelNode(C.Structure):
+    """CUDA_KERNEL_NODE_PARAMS of the driver API."""
+    _fields_ = [("func", C.c_void_p), ("grid", C.c_uint * 3), ("block", C.c_uint * 3), ("smem", C.c_uint),
+                ("params", C.c_void_p), ("extra", C.c_void_p), ("kern", C.c_void_p), ("ctx", C.c_void_p)]
+
+
+def _grids(calls):
+    """The grids of the two kernels that ``calls(stream)`` launches, in order,
+    from a captured graph (nothing runs)."""
+    torch = gh.torch_mod()
+    cu = C.CDLL("libcuda.so.1")
+    st = torch.cuda.Stream()
+    s = C.c_void_p(st.cuda_stream)
+    graph, n = C.c_void_p(), C.c_size_t(2)
+    assert cu.cuStreamBeginCapture_v2(s, 2) == 0
+    try:
+        calls(st.cuda_stream)
+    finally:
+        assert cu.cuStreamEndCapture(s, C.byref(graph)) == 0
+    nodes, root, one = (C.c_void_p * 2)(), (C.c_void_p * 1)(), C.c_size_t(1)
+    assert cu.cuGraphGetNodes(graph, nodes, C.byref(n)) == 0 and n.value == 2
+    assert cu.cuGraphGetRootNodes(graph, root, C.byref(one)) == 0 and one.value == 1
+    got = []
+    for node in [root[0]] + [v for v in nodes if v != root[0]]:
+        p = _KernelNode()
+        assert cu.cuGraphKernelNodeGetParams_v2(C.c_void_p(node), C.byref(p)) == 0
+        got.append(tuple(p.grid))
+    assert cu.cuGraphDestroy(graph) == 0
+    return got
+
+
+@pytest.mark.parametrize("P", [64, 128, 256, 512, 1024, 1536, 2048, 3072, 4096, 6144])
+def test_spectra_run_the_planned_sequences_per_cta(P):
+    """A choice of 1, 2 or 4 sequences per CTA is what runs, for every length
+    (a choice of 2 ran four rows below 2048 points, one of 4 two at 6144)."""
+    torch, lib = _init()
+    Cc, N, H = min(P, 1024), 3, P - 3
+    raw = torch.zeros(N, H, P, dtype=torch.uint8, device="cuda")
+    fr = _frames(raw, _lib.ZR_U8)
+    K4 = lib.zr_spectrum_pitch(Cc)
+    G = torch.empty(2, N, K4, Cc + 4, 2, device="cuda")
+    wb = lib.zr_spectra_work_bytes(H, N, Cc)
+    work = torch.empty(wb, dtype=torch.uint8, device="cuda")
+    shape = _lib.PlanShape(P, P, Cc, Cc, 8, 2)
+    try:
+        for rows in (1, 2, 4):
+            cols = {1: 2, 2: 4, 4: 1}[rows]
+            _lib.call("zr_plan_set", C.byref(shape), C.byref(_lib.PlanChoice(rows, cols, 0, 0)))
+            a, b = _grids(lambda st: _lib.call("zr_spectra", C.byref(fr), None, None, 0, N, 0, P, P, Cc, Cc,
+                                               G[0].data_ptr(), G[1].data_ptr(), work.data_ptr(), wb, st))
+            assert a == (N, -(-H // rows), 1) and b == (K4 // cols, N, 2)
+    finally:
+        _lib.call("zr_plan_set", C.byref(shape), C.byref(_lib.PlanChoice(0, 0, 0, 0)))
+
+
+@pytest.mark.parametrize("Cc", [64, 128, 256, 384, 512, 768, 1024, 1536, 2048, 3072, 4096])
+@pytest.mark.parametrize("half", [False, True])
+def test_windows_run_the_planned_sequences_per_cta(Cc, half):
+    """The same for the correlation windows, narrow ones and whole planes, from
+    float32 and from half-precision spectra."""
+    torch, lib = _init()
+    N, M = 2, 1
+    K4 = lib.zr_spectrum_pitch(Cc)
+    G = torch.empty(N, K4, Cc + 4, 2, dtype=torch.float16 if half else torch.float32, device="cuda")
+    sc = torch.ones(2 * N + 1, device="cuda")
+    pairs = torch.tensor([0, 1], dtype=torch.int32, device="cuda")
+    try:
+        for mS in (8, Cc // 2):
+            w = 2 * mS
+            terms, win = torch.empty(4 * N + 1, w, w, device="cuda"), torch.empty(M, w, w, device="cuda")
+            wb = lib.zr_xcorr_work_bytes(M, Cc, mS)
+            work = torch.empty(wb, dtype=torch.uint8, device="cuda")
+            shape = _lib.PlanShape(Cc, Cc, Cc, Cc, mS, 2)
+            for cols in (1, 2, 4):
+                rows = {1: 2, 2: 4, 4: 1}[cols]
+                _lib.call("zr_plan_set", C.byref(shape), C.byref(_lib.PlanChoice(0, 0, cols, rows)))
+                head = [G.data_ptr()] + ([sc.data_ptr()] if half else [])
+                a, b = _grids(lambda st: _lib.call("zr_xcorr_pairs_half" if half else "zr_xcorr_pairs", *head,
+                                                   terms.data_ptr(), pairs.data_ptr(), M, N, Cc, Cc, mS,
+                                                   win.data_ptr(), work.data_ptr(), wb, st))
+                assert a == (M, K4 // cols, 1) and b == (-(-w // (2 * rows)), M, 1)
+    finally:
+        _lib.call("zr_plan_set", C.byref(shape), C.byref(_lib.PlanChoice(0, 0, 0, 0)))

@@ -37,7 +37,6 @@ __device__ __forceinline__ size_t ru_at(int k, int y, int K4, int H4) {
 // R 2, 39.9 with R 4; of 2000 x 2000, 151 and 152.
 constexpr int FC_DEFAULT = 2;
 __host__ __device__ constexpr int fr_default(int P1) { return P1 >= 2048 ? 2 : 4; }
-__host__ __device__ constexpr int most_of(int P) { return P > 4096 ? 2 : 4; }  // that fit a CTA
 // CTAs per SM to ask the register allocator for: 128 registers a thread
 constexpr int minb_of(int T) { return sm_minb(T); }
 
@@ -337,9 +336,8 @@ static int launch_rows(const FrameSrc& f, const float* mask, const double* mean_
                        float2* RU, float2* RV, const float2* tw, cudaStream_t st) {
   switch (tune_get(TUNE_FWD_ROWS, P)) {
     case 1: return launch_rows_v<P, 1>(f, mask, mean_sub, inv_area, frame0, nfr, mode, rows, cols, C1, K4, H4, RU, RV, tw, st);
-    case 4:
-      return launch_rows_v<P, most_of(P)>(f, mask, mean_sub, inv_area, frame0, nfr, mode, rows, cols, C1, K4, H4, RU, RV,
-                                          tw, st);
+    case 2: return launch_rows_v<P, 2>(f, mask, mean_sub, inv_area, frame0, nfr, mode, rows, cols, C1, K4, H4, RU, RV, tw, st);
+    case 4: return launch_rows_v<P, 4>(f, mask, mean_sub, inv_area, frame0, nfr, mode, rows, cols, C1, K4, H4, RU, RV, tw, st);
     default:
       return launch_rows_v<P, fr_default(P)>(f, mask, mean_sub, inv_area, frame0, nfr, mode, rows, cols, C1, K4, H4, RU, RV,
                                           tw, st);
@@ -362,7 +360,8 @@ static int launch_cols(const float2* RU, const float2* RV, int rows, int C0, int
                        int nfr, int nz, float2* G, float2* S, const float2* tw, cudaStream_t st) {
   switch (tune_get(TUNE_FWD_COLS, P)) {
     case 1: return launch_cols_v<P, 1>(RU, RV, rows, C0, K4, H4, se, nfr, nz, G, S, tw, st);
-    case 4: return launch_cols_v<P, most_of(P)>(RU, RV, rows, C0, K4, H4, se, nfr, nz, G, S, tw, st);
+    case 2: return launch_cols_v<P, 2>(RU, RV, rows, C0, K4, H4, se, nfr, nz, G, S, tw, st);
+    case 4: return launch_cols_v<P, 4>(RU, RV, rows, C0, K4, H4, se, nfr, nz, G, S, tw, st);
     default: return launch_cols_v<P, FC_DEFAULT>(RU, RV, rows, C0, K4, H4, se, nfr, nz, G, S, tw, st);
   }
 }

@@ -271,23 +271,26 @@ static int launch_xc_cols_t(const XcJobs& J, int nj, int C1, int K4, int mS, flo
   return launched("k_xc_cols");
 }
 
-// The planner's choices of columns per CTA apply to the float32 spectra's
-// pruned windows, which are what it measures.
+template <int C0, typename E, bool PRUNED>
+static int launch_xc_cols_e(const XcJobs& J, int nj, int C1, int K4, int mS, float2* Tw, const float2* tw,
+                            cudaStream_t st) {
+  switch (tune_get(TUNE_XC_COLS, C0)) {
+    case 1: return launch_xc_cols_t<C0, E, 1, PRUNED>(J, nj, C1, K4, mS, Tw, tw, st);
+    case 2: return launch_xc_cols_t<C0, E, 2, PRUNED>(J, nj, C1, K4, mS, Tw, tw, st);
+    case 4: return launch_xc_cols_t<C0, E, 4, PRUNED>(J, nj, C1, K4, mS, Tw, tw, st);
+    default: return launch_xc_cols_t<C0, E, xc_nbc_default(C0), PRUNED>(J, nj, C1, K4, mS, Tw, tw, st);
+  }
+}
+
 template <int C0>
 static int launch_xc_cols(const XcJobs& J, int nj, int C1, int K4, int mS, float2* Tw, const float2* tw,
                           cudaStream_t st) {
-  constexpr int D = xc_nbc_default(C0);
   const bool pruned = J.rows <= Ip<C0>::NS;
   if (J.sc)
-    return pruned ? launch_xc_cols_t<C0, __half2, D, true>(J, nj, C1, K4, mS, Tw, tw, st)
-                  : launch_xc_cols_t<C0, __half2, D, false>(J, nj, C1, K4, mS, Tw, tw, st);
-  if (!pruned) return launch_xc_cols_t<C0, float2, D, false>(J, nj, C1, K4, mS, Tw, tw, st);
-  switch (tune_get(TUNE_XC_COLS, C0)) {
-    case 1: return launch_xc_cols_t<C0, float2, 1, true>(J, nj, C1, K4, mS, Tw, tw, st);
-    case 2: return launch_xc_cols_t<C0, float2, 2, true>(J, nj, C1, K4, mS, Tw, tw, st);
-    case 4: return launch_xc_cols_t<C0, float2, 4, true>(J, nj, C1, K4, mS, Tw, tw, st);
-    default: return launch_xc_cols_t<C0, float2, D, true>(J, nj, C1, K4, mS, Tw, tw, st);
-  }
+    return pruned ? launch_xc_cols_e<C0, __half2, true>(J, nj, C1, K4, mS, Tw, tw, st)
+                  : launch_xc_cols_e<C0, __half2, false>(J, nj, C1, K4, mS, Tw, tw, st);
+  return pruned ? launch_xc_cols_e<C0, float2, true>(J, nj, C1, K4, mS, Tw, tw, st)
+                : launch_xc_cols_e<C0, float2, false>(J, nj, C1, K4, mS, Tw, tw, st);
 }
 
 template <int C1, int NBR, bool PRUNED>
@@ -302,16 +305,22 @@ static int launch_xc_rows_v(const XcJobs& J, int nj, int C0, int K4, int mS, flo
   return launched("k_xc_rows");
 }
 
+template <int C1, bool PRUNED>
+static int launch_xc_rows_p(const XcJobs& J, int nj, int C0, int K4, int mS, float scale, const float2* Tw,
+                            const float* terms, float* out, const float2* tw, cudaStream_t st) {
+  switch (tune_get(TUNE_XC_ROWS, C1)) {
+    case 1: return launch_xc_rows_v<C1, 1, PRUNED>(J, nj, C0, K4, mS, scale, Tw, terms, out, tw, st);
+    case 2: return launch_xc_rows_v<C1, 2, PRUNED>(J, nj, C0, K4, mS, scale, Tw, terms, out, tw, st);
+    case 4: return launch_xc_rows_v<C1, 4, PRUNED>(J, nj, C0, K4, mS, scale, Tw, terms, out, tw, st);
+    default: return launch_xc_rows_v<C1, XC_NBR_DEFAULT, PRUNED>(J, nj, C0, K4, mS, scale, Tw, terms, out, tw, st);
+  }
+}
+
 template <int C1>
 static int launch_xc_rows(const XcJobs& J, int nj, int C0, int K4, int mS, float scale, const float2* Tw,
                           const float* terms, float* out, const float2* tw, cudaStream_t st) {
-  constexpr int D = XC_NBR_DEFAULT;
-  if (J.rows > Ip<C1>::NS) return launch_xc_rows_v<C1, D, false>(J, nj, C0, K4, mS, scale, Tw, terms, out, tw, st);
-  switch (tune_get(TUNE_XC_ROWS, C1)) {
-    case 1: return launch_xc_rows_v<C1, 1, true>(J, nj, C0, K4, mS, scale, Tw, terms, out, tw, st);
-    case 4: return launch_xc_rows_v<C1, 4, true>(J, nj, C0, K4, mS, scale, Tw, terms, out, tw, st);
-    default: return launch_xc_rows_v<C1, D, true>(J, nj, C0, K4, mS, scale, Tw, terms, out, tw, st);
-  }
+  return J.rows <= Ip<C1>::NS ? launch_xc_rows_p<C1, true>(J, nj, C0, K4, mS, scale, Tw, terms, out, tw, st)
+                              : launch_xc_rows_p<C1, false>(J, nj, C0, K4, mS, scale, Tw, terms, out, tw, st);
 }
 
 #define ZR_XC_DISPATCH(L, CALL)                               \
