@@ -12,7 +12,9 @@
 #include "fft_inplace.cuh"
 #include "internal.h"
 
-#define ZR_VERSION 100
+// Raised with every change of the transform kernels' variants: saved plans are
+// kept by it (100: the Stockham transforms).
+#define ZR_VERSION 101
 
 namespace zr {
 
