@@ -328,3 +328,23 @@ def test_windows_run_the_planned_sequences_per_cta(Cc, half):
                 assert a == (M, K4 // cols, 1) and b == (-(-w // (2 * rows)), M, 1)
     finally:
         _lib.call("zr_plan_set", C.byref(shape), C.byref(_lib.PlanChoice(0, 0, 0, 0)))
+
+
+def test_gain_sum_total_keeps_float64():
+    """A thread's share of the total keeps every bit that a float64 sum of its
+    pixels keeps: 16 shares of 1 + 2^-25 (1 + 2^-23) + 2^-26 (1 + 2^-23), whose
+    sum needs 50 bits, add up exactly, on the vector and on the pixel path."""
+    torch, _ = _init()
+    share = [1.0, 2.0 ** -25 * (1 + 2.0 ** -23), 2.0 ** -26 * (1 + 2.0 ** -23), 0.0]
+    img = np.tile(np.array(share, np.float32), 16).reshape(1, 8, 8)
+    want = 16 * (share[0] + share[1] + share[2])
+    assert (share[0] + share[1]) - share[0] == share[1]  # float64 holds it
+    for off in (0, 1):  # one float past the vector boundary: pixel by pixel
+        arena = torch.zeros(65, device="cuda")
+        arena[off:off + 64] = torch.from_numpy(img.ravel()).cuda()
+        fr = _lib.Frames(arena.data_ptr() + 4 * off, _lib.ZR_F32, None, None, None, 0.0, 1, 8, 8, 0)
+        out = torch.empty(64, device="cuda")
+        total = torch.zeros(1, dtype=torch.float64, device="cuda")
+        _lib.call("zr_gain_sum", C.byref(fr), out.data_ptr(), total.data_ptr(), gh.stream())
+        assert total.item() == want, (off, total.item() - want)
+        assert np.array_equal(out.cpu().numpy().reshape(8, 8), img[0])

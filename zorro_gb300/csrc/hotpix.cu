@@ -12,23 +12,29 @@
 
 namespace zr {
 
-// A running sum of floats as an unevaluated pair hi + lo (Knuth's two-sum:
-// exact error of every addition), so that a thread's share of the float64
-// total needs no float64 operation per pixel: a converted addition a pixel
-// kept the float64 pipe (2 lanes an SM) 79 % busy and bound the frame sum.
-// The terms are scaled by 2^-10 (exact) so that no sum of a few hundred of
-// them overflows.
-struct PairSum {
-  float hi = 0.0f, lo = 0.0f;
+// A running sum of floats as three floats hi + lo + lo2, by Knuth's two-sum
+// (the exact error of an addition) on the sum and again on its errors, so that
+// a thread's share of the float64 total needs no float64 operation per pixel:
+// a converted addition a pixel kept the float64 pipe (2 lanes an SM) 79 % busy
+// and bound the frame sum.  72 bits, so what is left is the rounding to float64
+// at the end.  The terms are scaled by 2^-10 (exact) so that no sum of a few
+// hundred of them overflows.
+struct TripleSum {
+  float hi = 0.0f, lo = 0.0f, lo2 = 0.0f;
+  static __device__ __forceinline__ float two_sum(float a, float b, float& err) {
+    const float t = __fadd_rn(a, b), d = __fsub_rn(t, a);
+    err = __fadd_rn(__fsub_rn(a, __fsub_rn(t, d)), __fsub_rn(b, d));
+    return t;
+  }
   __device__ __forceinline__ void add(float v) {
-    v *= 0.0009765625f;
-    const float t = __fadd_rn(hi, v), b = __fsub_rn(t, hi);
-    lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(hi, __fsub_rn(t, b)), __fsub_rn(v, b)));
-    hi = t;
+    float e, e2;
+    hi = two_sum(hi, v * 0.0009765625f, e);
+    lo = two_sum(lo, e, e2);
+    lo2 = __fadd_rn(lo2, e2);
   }
   // (an infinite or NaN sum has no error term)
   __device__ __forceinline__ double value() const {
-    return 1024.0 * (fabsf(hi) < INFINITY ? (double)hi + (double)lo : (double)hi);
+    return 1024.0 * (fabsf(hi) < INFINITY ? (double)hi + ((double)lo + (double)lo2) : (double)hi);
   }
 };
 
@@ -47,15 +53,15 @@ __device__ __forceinline__ void add_total(double part, double* __restrict__ tota
 
 __global__ void k_gain_sum(FrameSrc f, float* __restrict__ sum, double* __restrict__ total) {
   const long long npix = (long long)f.H * f.W;
-  PairSum part;
+  double part = 0.0;
   for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < npix; p += (long long)gridDim.x * blockDim.x) {
     const int y = (int)(p / f.W), x = (int)(p - (long long)y * f.W);
     float s = 0.0f;
     for (int n = 0; n < f.N; n++) s = __fadd_rn(s, load_corrected(f, n, y, x));
     sum[p] = s;
-    part.add(s);
+    part += (double)s;
   }
-  add_total(part.value(), total);
+  add_total(part, total);
 }
 
 // Same sum, four pixels per thread (H*W % 4 == 0, aligned vector loads), the
@@ -66,7 +72,7 @@ constexpr int GS_FRAMES = 8;
 template <int TYPE>
 __global__ void __launch_bounds__(256, 3) k_gain_sum_q(FrameSrc f, float* __restrict__ sum, double* __restrict__ total) {
   const long long n4 = (long long)f.H * f.W / 4;
-  PairSum part;
+  TripleSum part;
   for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < n4; q += (long long)gridDim.x * blockDim.x) {
     const long long p = 4 * q;
     float4 g = make_float4(1.f, 1.f, 1.f, 1.f);
