@@ -67,10 +67,14 @@ __global__ void k_gain_sum(FrameSrc f, float* __restrict__ sum, double* __restri
 // Same sum, four pixels per thread (H*W % 4 == 0, aligned vector loads), the
 // frames read GS_FRAMES at a time before any is added, so that each thread
 // keeps that many loads in flight; the additions stay in frame order.
+// Four CTAs an SM where a quad's eight loads fit 64 registers, three for
+// float32: 40 K2 frames of uint16 228 us with three, 207 with four, 20 of
+// float32 191 and 202.
 constexpr int GS_FRAMES = 8;
+__host__ __device__ constexpr int gs_ctas(int type) { return type == ZR_F32 ? 3 : 4; }
 
 template <int TYPE>
-__global__ void __launch_bounds__(256, 3) k_gain_sum_q(FrameSrc f, float* __restrict__ sum, double* __restrict__ total) {
+__global__ void __launch_bounds__(256, gs_ctas(TYPE)) k_gain_sum_q(FrameSrc f, float* __restrict__ sum, double* __restrict__ total) {
   const long long n4 = (long long)f.H * f.W / 4;
   TripleSum part;
   for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < n4; q += (long long)gridDim.x * blockDim.x) {
