@@ -348,3 +348,21 @@ def test_gain_sum_total_keeps_float64():
         _lib.call("zr_gain_sum", C.byref(fr), out.data_ptr(), total.data_ptr(), gh.stream())
         assert total.item() == want, (off, total.item() - want)
         assert np.array_equal(out.cpu().numpy().reshape(8, 8), img[0])
+
+
+@pytest.mark.parametrize("H,W", [(5, 7), (64, 64), (201, 181), (700, 1000)])
+@pytest.mark.parametrize("nbins", [1, 48, 103, 767, 769, 1600, 12289, 20000, 32768])
+def test_histogram_of_any_number_of_bins(H, W, nbins):
+    """Counts equal np.histogram's whatever the number of bins, hence of copies
+    a CTA counts in, over values on and around the edges and outside them."""
+    torch, _ = _init()
+    rng = np.random.default_rng(nbins)
+    v = (rng.normal(nbins / 2, nbins / 3, (H, W))).astype(np.float32)
+    v.flat[::3] = np.round(v.flat[::3] * 2) / 2
+    v.flat[:4] = [-0.5, nbins - 0.5, np.nextafter(np.float32(nbins - 0.5), np.float32(1e9)), np.inf]
+    want = np.histogram(v[np.isfinite(v)].astype(np.float64), np.arange(nbins + 1) - 0.5)[0]
+    dev = torch.from_numpy(v).cuda()
+    counts = torch.zeros(nbins + 8, dtype=torch.int32, device="cuda")
+    _lib.call("zr_histogram", dev.data_ptr(), H * W, -0.5, nbins, counts.data_ptr(), gh.stream())
+    got = counts.cpu().numpy()
+    assert np.array_equal(got[:nbins], want) and not got[nbins:].any()
