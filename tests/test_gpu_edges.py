@@ -366,3 +366,34 @@ def test_histogram_of_any_number_of_bins(H, W, nbins):
     _lib.call("zr_histogram", dev.data_ptr(), H * W, -0.5, nbins, counts.data_ptr(), gh.stream())
     got = counts.cpu().numpy()
     assert np.array_equal(got[:nbins], want) and not got[nbins:].any()
+
+
+@pytest.mark.parametrize("mu", [16000000.0 + 37 * i for i in range(12)])
+def test_hot_maps_of_a_narrow_fit_far_from_zero(mu):
+    """The logistic masks of sums whose mean is 1.2e9 fitted sigmas from zero:
+    the exponents K (s - mu) / sigma - K c are differences of 7e10, which float64
+    holds to 3 x 2^-53 of that, 2.4e-5; a mask moves by at most half of its
+    exponents' error, and 2e-5 holds that and the float32 roundings."""
+    torch, lib = _init()
+    H, W, sigma, K = 8, 12, 0.0137, float(np.float32(59.3))
+    p = _lib.HotpixParams()
+    p.mu, p.sigma, p.cutoff_lower, p.cutoff_upper = mu, sigma, -0.01, 0.02
+    p.logistic_k, p.relax, p.neighbour_thres, p.best_mean = K, 1.0, 0.01, mu / 10
+    for i, v in enumerate(hm.psf_kernel("K2").ravel()):
+        p.psf[i] = float(v)
+    s = np.full((H, W), mu, np.float32)
+    s[3, 4], s[5, 7] = mu + 1, mu - 1
+    assert float(s[0, 0]) == mu
+    dev = torch.from_numpy(s).cuda()
+    a, b = torch.empty(H, W, device="cuda"), torch.empty(H, W, device="cuda")
+    counts = torch.zeros(4, dtype=torch.int32, device="cuda")
+    wb = lib.zr_hotpix_work_bytes(H, W)
+    work = torch.empty(wb, dtype=torch.uint8, device="cuda")
+    _lib.call("zr_hotpix_maps", dev.data_ptr(), H, W, 10, C.byref(p), a.data_ptr(), b.data_ptr(), counts.data_ptr(),
+              work.data_ptr(), wb, gh.stream())
+    sg = (s.astype(np.float64) - mu) / sigma
+    with np.errstate(over="ignore"):
+        e1, e2 = np.exp(K * (sg - float(np.float32(-0.01)))), np.exp(K * (sg - float(np.float32(0.02))))
+        want = (1.0 - 1.0 / (1.0 + e1)) / (1.0 + e2)
+    assert np.abs(a.cpu().numpy() - want).max() <= 2e-5
+    assert counts.cpu().tolist()[:2] == [1, 1]

@@ -202,12 +202,13 @@ __device__ __forceinline__ int rfl(int i, int n) { return i < 0 ? -i - 1 : (i >=
 
 // The logistic exponents K (sigma - c relax), sigma = (s - mu) / sigma_fit, as
 // A s + C with A = K / sigma_fit and C = -K c relax - A mu folded on the host
-// in float64.  A pixel evaluates them with A and C split into float pairs (the
-// product's and the sum's rounding errors kept: 2^-47 of the larger term,
-// before the rounding to float32 that the float64 form ends with too); a
-// float64 multiply-add and its conversions kept the float64 pipe 85 % busy.
-// Sums or constants too large for the float products go through float64, step
-// by step when sigma_fit is 0.
+// in float64.  A pixel evaluates them with A and C split into float pairs, the
+// product's and the sum's rounding errors kept: off by 2^-46 of the larger term
+// at most, where a float64 multiply-add and its conversions kept the float64
+// pipe 85 % busy.  The pairs serve while |C| < 2^17, where that is below 2^-29,
+// out of sight of the exponentials' own roundings (40 K2 frames have a few tens; over 36 movies of 2 to 40 frames the maps' error against
+// float64 is the same either way, 2.5e-8 to 2.8e-8 rms).  Beyond it, and for sums
+// too large for the float products, float64, step by step when sigma_fit is 0.
 struct HotConst {
   double rsig, A, C1, C2;
   float Ah, Al, C1h, C1l, C2h, C2l;
@@ -517,9 +518,9 @@ extern "C" int zr_hotpix_maps(const float* unaligned_sum, int height, int width,
   split(h.A, h.Ah, h.Al);
   split(h.C1, h.C1h, h.C1l);
   split(h.C2, h.C2h, h.C2l);
-  // the float pairs hold their errors for |A s| and |C| well inside float's range
-  const double big = 1e18, amax = fabs(h.A);
-  h.s_max = h.rsig < INFINITY && amax < big && fabs(h.C1) < big && fabs(h.C2) < big ? 1e15f : 0.0f;
+  // (where |C| < 2^17 a larger |A s| only saturates; the products stay inside float's range)
+  const double cmax = fmax(fabs(h.C1), fabs(h.C2));
+  h.s_max = h.rsig < INFINITY && fabs(h.A) < 1e18 && cmax < 131072.0 ? 1e15f : 0.0f;
   const dim3 tiles((width + HF_TX - 1) / HF_TX, (height + HF_TY - 1) / HF_TY);
   k_hot_maps<<<tiles, HF_T, 0, (cudaStream_t)stream>>>(unaligned_sum, height, width, n_frames, p, h, s_dead, s_hot,
                                                        hot_a, hot_b, counts3);
