@@ -206,9 +206,10 @@ __device__ __forceinline__ int rfl(int i, int n) { return i < 0 ? -i - 1 : (i >=
 // product's and the sum's rounding errors kept: off by 2^-46 of the larger term
 // at most, where a float64 multiply-add and its conversions kept the float64
 // pipe 85 % busy.  The pairs serve while |C| < 2^17, where that is below 2^-29,
-// out of sight of the exponentials' own roundings (40 K2 frames have a few tens; over 36 movies of 2 to 40 frames the maps' error against
-// float64 is the same either way, 2.5e-8 to 2.8e-8 rms).  Beyond it, and for sums
-// too large for the float products, float64, step by step when sigma_fit is 0.
+// out of sight of the exponentials' own roundings (40 K2 frames have a few tens;
+// over 36 movies of 2 to 40 frames the maps' error against float64 is the same
+// either way, 2.5e-8 to 2.8e-8 rms).  Beyond it, and for sums too large for the
+// float products, float64, step by step when sigma_fit is 0.
 struct HotConst {
   double rsig, A, C1, C2;
   float Ah, Al, C1h, C1l, C2h, C2l;
