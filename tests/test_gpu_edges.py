@@ -397,3 +397,34 @@ def test_hot_maps_of_a_narrow_fit_far_from_zero(mu):
         want = (1.0 - 1.0 / (1.0 + e1)) / (1.0 + e2)
     assert np.abs(a.cpu().numpy() - want).max() <= 2e-5
     assert counts.cpu().tolist()[:2] == [1, 1]
+
+
+@pytest.mark.parametrize("box", [128, 256, 512, 1024])
+def test_rings_are_float64_means_of_the_plane(box):
+    """The FRC of one tile is exactly 1 at zero frequency, so frc2d holds the
+    plane that the rings average without a rounding: they are its rotational
+    mean (bilinear split, in extended precision here) within 4e-14: weights off
+    by 2^-47, twice a ring's weight of them in the sum and in its divisor, and
+    30 roundings of 2^-53."""
+    torch, lib = _init()
+    rng = np.random.default_rng(box)
+    base = rng.poisson(300.0, (box, box))
+    e, o = (torch.from_numpy((base + rng.poisson(60.0, (box, box))).astype(np.float32)).cuda() for _ in range(2))
+    offs = torch.zeros(2, dtype=torch.int32, device="cuda")
+    nr = int(np.ceil(np.sqrt(2.0) * (box // 2))) + 1
+    wb = lib.zr_frc_work_bytes(1, box)
+    work = torch.empty(wb, dtype=torch.uint8, device="cuda")
+    frc2d, frc = torch.empty(box, box, device="cuda"), torch.empty(nr, dtype=torch.float64, device="cuda")
+    _lib.call("zr_tiled_frc", e.data_ptr(), o.data_ptr(), box, box, box, offs.data_ptr(), 1, frc2d.data_ptr(),
+              frc.data_ptr(), nr, work.data_ptr(), wb, gh.stream())
+    v = frc2d.cpu().numpy().astype(np.longdouble)
+    assert v[box // 2, box // 2] == 1.0
+    x = np.arange(box) - box // 2
+    rho = np.sqrt((x[:, None] ** 2 + x[None, :] ** 2).astype(np.longdouble))
+    b0 = np.floor(rho).astype(int)
+    num, den = np.zeros(nr + 1, np.longdouble), np.zeros(nr + 1, np.longdouble)
+    for k, w in ((b0, 1 - (rho - b0)), (b0 + 1, rho - b0)):
+        np.add.at(num, k, v * w)
+        np.add.at(den, k, w)
+    live = den[:nr] > 0
+    assert np.abs(frc.cpu().numpy()[live] - (num[:nr] / den[:nr])[live]).max() <= 4e-14

@@ -147,12 +147,25 @@ __global__ void k_frc_mean(const double* __restrict__ half, int ngroups, int B, 
   if (kx > 0 && kx < hb) frc2d[((B - ky + hb) & m) * B + ((B - kx + hb) & m)] = (float)v;
 }
 
+// sqrt(n) - r (n < 2^20, |.| <= 1 within a ring), off by less than 2^-47: the float
+// root h, the remainder e = n - h^2 (exact), x = sqrt(n) - h from 2 h x + x^2 = e as
+// a float and what that leaves over, and Knuth's two-sum of h - r (exact) and x.
+// A float64 square root is off by 2^-44 here.  One float64 addition, as with
+// e / 2h alone, which is off by 2^-38; the square root itself took 7 us more for a
+// K2 sum (a float64 operation keeps a warp's pipe 16 cycles).
+__device__ __forceinline__ double root_minus(int n, int r) {
+  if (n == 0) return -(double)r;
+  const float h = sqrtf((float)n), g = 0.5f / h, e = fmaf(-h, h, (float)n);
+  const float x = __fmul_rn(e, g), x2 = __fmul_rn(fmaf(-x, x, fmaf(-2.0f * h, x, e)), g);
+  const float a = __fsub_rn(h, (float)r), t = __fadd_rn(a, x), b = __fsub_rn(t, a);
+  const float err = __fadd_rn(__fsub_rn(a, __fsub_rn(t, b)), __fsub_rn(x, b));
+  return (double)t + (double)__fadd_rn(err, x2);
+}
+
 // One ring r per CTA: pixels at radius rho in [r, r + 1) count with weight
 // r + 1 - rho, those in [r - 1, r) with rho - r + 1 (the bilinear split of
-// rotmean, gathered instead of scattered: no atomics).  rho = sqrt(n) for the
-// integer n = x^2 + y^2 as a float and its residual (n < 2^20: the square's
-// error is exact), 2^-47 relative; only the sums are float64.  A thread takes
-// one line along the axis it crosses the ring by, where |that coordinate| is
+// rotmean, gathered instead of scattered: no atomics), in float64.  A thread
+// takes one line along the axis it crosses the ring by, where |that coordinate| is
 // the larger one: four pixels a side at most
 // (whole rows of a ring's top, of 60 pixels, kept their threads for 48 us; the
 // scattered form with shared-memory atomics took 111 us).
@@ -176,12 +189,7 @@ __global__ void __launch_bounds__(FRC_RT) k_frc_rings(const double* __restrict__
     }
     for (int a = x0; a <= min(x1, hb); a++) {
       const int n = a * a + c2;
-      double d = -(double)r;  // rho - r
-      if (n > 0) {
-        const float rh = sqrtf((float)n);
-        const float rl = fmaf(-rh, rh, (float)n) * (0.5f / rh);
-        d = (double)(rh - (float)r) + (double)rl;
-      }
+      const double d = root_minus(n, r);  // rho - r
       const double wt = n >= r * r ? 1.0 - d : 1.0 + d;
 #pragma unroll
       for (int q = 0; q < 2; q++) {
