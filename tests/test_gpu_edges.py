@@ -428,3 +428,83 @@ def test_rings_are_float64_means_of_the_plane(box):
         np.add.at(den, k, w)
     live = den[:nr] > 0
     assert np.abs(frc.cpu().numpy()[live] - (num[:nr] / den[:nr])[live]).max() <= 4e-14
+
+
+def _hot_maps(s, sigma, n=10, mu=20.0):
+    torch, lib = _init()
+    H, W = s.shape
+    p = _lib.HotpixParams()
+    p.mu, p.sigma, p.cutoff_lower, p.cutoff_upper = mu, sigma, -4.0, 3.25
+    p.logistic_k, p.relax, p.neighbour_thres, p.best_mean = 6.0, 0.925, 0.01, mu / n
+    for i, k in enumerate(hm.psf_kernel("K2").ravel()):
+        p.psf[i] = float(k)
+    ds = torch.from_numpy(s).cuda()
+    a, b = (torch.full((H, W), 7.0, device="cuda") for _ in range(2))
+    cnt = torch.zeros(4, dtype=torch.int32, device="cuda")
+    wb = lib.zr_hotpix_work_bytes(H, W)
+    work = torch.empty(wb, dtype=torch.uint8, device="cuda")
+    _lib.call("zr_hotpix_maps", ds.data_ptr(), H, W, n, C.byref(p), a.data_ptr(), b.data_ptr(), cnt.data_ptr(),
+              work.data_ptr(), wb, gh.stream())
+    return p, a.cpu().numpy(), b.cpu().numpy(), cnt.cpu().tolist()
+
+
+@pytest.mark.parametrize("H,W", [(4, 4), (7, 63), (8, 64), (9, 65), (33, 130), (385, 833)])
+def test_hot_fill_and_counts_at_tile_edges(H, W):
+    """Both maps and all three counts against a float64 restatement (scipy's
+    reflected convolution, the neighbour mean with the reference's slices), with
+    single outliers, pairs and blocks of them on the rows and columns where
+    tiles of 8 and of 32 rows meet and on the image's border, and a NaN.  Masks:
+    exponents rounded to float32, as test_hotpix_map_tiles has it.  Fill: nine-tap
+    float32 sums and the masks' error, 2e-6 and 2e-5 of the largest value a
+    pixel's neighbourhood holds.  Pixels whose mask product lies within rounding
+    of its threshold are left out, and what a NaN reaches."""
+    import scipy.ndimage
+    rng = np.random.default_rng(H * W)
+    n, mu, sigma = 10, 20.0, 3.0
+    s = rng.normal(mu, sigma, (H, W)).clip(mu - 2 * sigma, mu + 1.5 * sigma).astype(np.float32)
+    ys = [y for y in (0, 1, 6, 7, 8, 9, 30, 31, 32, 33, 63, 64, 383, H - 1) if y < H]
+    xs = [x for x in (0, 1, 62, 63, 64, 65, 127, 128, 767, 768, W - 1) if x < W]
+    for y in ys:
+        for x in xs:
+            if rng.random() < 0.6:
+                s[y, x] = rng.choice([0.0, 55.0, 90.0])
+    if H > 32:
+        s[20:24, 40:44] = 80.0
+        s[12, 100] = np.nan
+    p, a, b, counts = _hot_maps(s, sigma)
+    v = s.astype(np.float64)
+    with np.errstate(all="ignore"):
+        q = (v - mu) / sigma
+        lo, up = (np.float64(np.float32(c) * np.float32(0.925)) for c in (-4.0, 3.25))
+        lm = (1.0 - 1.0 / (1.0 + np.exp(6.0 * (q - lo)))) / (1.0 + np.exp(6.0 * (q - up)))
+        psf = hm.psf_kernel("K2").astype(np.float64).reshape(3, 3)
+        conv, mean = 1.0 - lm, v / n
+        nom = conv * scipy.ndimage.convolve(conv, psf, mode="reflect")
+        mask = nom > p.neighbour_thres
+        fill = conv * ~mask * scipy.ndimage.convolve(mean, psf, mode="reflect")
+        for y, x in zip(*np.where(mask)):
+            hood = mask[y - 1:y + 2, x - 1:x + 2]  # empty where it would start at -1
+            ratio = hood.sum() / hood.size if hood.size else np.nan
+            if ratio > 0.66 or ratio <= 0.001 or np.isnan(ratio):
+                fill[y, x] += mu / n
+            else:
+                fill[y, x] += conv[y, x] * mean[y - 1:y + 2, x - 1:x + 2][~hood].mean()
+    assert counts[:2] == [np.sum(q < -4.0), np.sum(q > 3.25)]
+    np.testing.assert_allclose(a, lm, rtol=0, atol=88 * 2.0 ** -24 / 4 + 5e-7)
+    close = np.abs(nom - p.neighbour_thres) < 1e-5
+    assert abs(counts[2] - mask.sum()) <= close.sum()
+    out = scipy.ndimage.maximum_filter((close | np.isnan(v)).astype(np.uint8), 5) > 0
+    big = scipy.ndimage.maximum_filter(np.nan_to_num(mean), 5)
+    assert np.isnan(b[np.isnan(v)]).all() and np.isfinite(b[~out]).all() and out.mean() < 0.5
+    assert np.all(np.abs(b - fill)[~out] <= (2e-5 * big)[~out])
+    assert H < 9 or counts[2] > 0
+
+
+def test_hot_maps_of_a_fit_without_width():
+    """sigma_fit 0: every sum but the mean itself is masked out, and that one is
+    0 times infinity, as the step by step formula has it."""
+    s = np.full((40, 70), 20.0, np.float32)
+    s[::3, ::2] = np.linspace(-5.0, 60.0, s[::3, ::2].size).reshape(s[::3, ::2].shape)
+    _, a, _, counts = _hot_maps(s, 0.0)
+    assert np.array_equal(np.isnan(a), s == 20.0) and np.all(a[s != 20.0] == 0.0)
+    assert counts[:2] == [np.sum(s < 20.0), np.sum(s > 20.0)]

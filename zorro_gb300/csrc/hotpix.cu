@@ -8,6 +8,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "common.cuh"
 #include "internal.h"
@@ -269,9 +270,13 @@ __device__ __forceinline__ void hot_mask(float s, const zr_hotpix_params_t& p, c
 // Fused: the mask used to be a pass of its own (139 us for a K2 frame, bound
 // by the float64 pipe) whose 1 - lm the fill read back per 32 x 32 tile (129
 // us, 83 % of issue slots); together they take 160 us.
-constexpr int HF_TX = 64, HF_TY = 32;
-constexpr int HF_CW = HF_TX + 4, HF_CH = HF_TY + 4;  // 1 - lm, two-pixel ring
-constexpr int HF_MW = HF_TX + 2, HF_MH = HF_TY + 2;  // mean and mask, one-pixel ring
+// Tiles of 8 rows where those of 32 leave SMs idle: what takes the time there is
+// one tile's serial work (200 x 180: 13.2 us with 32 rows, 7.1 with 8; 512 x 512
+// 13.2 and 10.8; at 1024 x 1024, 512 tiles of 32 rows, 18.6 with those).
+constexpr int HF_SMS = 152;
+constexpr int HF_TX = 64;
+constexpr int HF_CW = HF_TX + 4;  // 1 - lm, two-pixel ring
+constexpr int HF_MW = HF_TX + 2;  // mean and mask, one-pixel ring
 constexpr int HF_T = 256;
 
 // 3 x 3 sums down a column: ``psf_strip`` calls f(row, sum) for rows r0 .. r0 +
@@ -299,10 +304,12 @@ __device__ __forceinline__ void psf_strip(const float* __restrict__ src, int r0,
   }
 }
 
+template <int HF_TY>
 __global__ void __launch_bounds__(HF_T) k_hot_maps(const float* __restrict__ sum, int H, int W, int nfr,
                                                    zr_hotpix_params_t p, HotConst h, float s_dead, float s_hot,
                                                    float* __restrict__ LM, float* __restrict__ B,
                                                    unsigned int* __restrict__ counts) {
+  constexpr int HF_CH = HF_TY + 4, HF_MH = HF_TY + 2;
   __shared__ float cv[HF_CH][HF_CW];
   __shared__ float mn[HF_MH][HF_MW];
   __shared__ uint8_t nm[HF_MH][HF_MW];
@@ -522,8 +529,13 @@ extern "C" int zr_hotpix_maps(const float* unaligned_sum, int height, int width,
   // (where |C| < 2^17 a larger |A s| only saturates; the products stay inside float's range)
   const double cmax = fmax(fabs(h.C1), fabs(h.C2));
   h.s_max = h.rsig < INFINITY && fabs(h.A) < 1e18 && cmax < 131072.0 ? 1e15f : 0.0f;
-  const dim3 tiles((width + HF_TX - 1) / HF_TX, (height + HF_TY - 1) / HF_TY);
-  k_hot_maps<<<tiles, HF_T, 0, (cudaStream_t)stream>>>(unaligned_sum, height, width, n_frames, p, h, s_dead, s_hot,
-                                                       hot_a, hot_b, counts3);
+  const int nx = (width + HF_TX - 1) / HF_TX;
+  auto run = [&](auto ty) {
+    constexpr int TY = decltype(ty)::value;
+    k_hot_maps<TY><<<dim3(nx, (height + TY - 1) / TY), HF_T, 0, (cudaStream_t)stream>>>(
+        unaligned_sum, height, width, n_frames, p, h, s_dead, s_hot, hot_a, hot_b, counts3);
+  };
+  if ((long long)nx * ((height + 31) / 32) < HF_SMS) run(std::integral_constant<int, 8>());
+  else run(std::integral_constant<int, 32>());
   return launched("k_hot_maps");
 }
