@@ -508,3 +508,40 @@ def test_hot_maps_of_a_fit_without_width():
     _, a, _, counts = _hot_maps(s, 0.0)
     assert np.array_equal(np.isnan(a), s == 20.0) and np.all(a[s != 20.0] == 0.0)
     assert counts[:2] == [np.sum(s < 20.0), np.sum(s > 20.0)]
+
+
+@pytest.mark.parametrize("kind", ["u8", "u16", "f16", "f32"])
+@pytest.mark.parametrize("gain,hot", [(0, 0), (1, 0), (0, 1), (1, 1)])
+@pytest.mark.parametrize("H,W", [(301, 303), (501, 703), (701, 703), (905, 1003), (1501, 1003)])
+def test_shift_sum_paths_agree(kind, gain, hot, H, W):
+    """Frames that lie one after the other with an odd number of pixels are read
+    pixel by pixel, a frame ahead or not by the number of tiles and by their
+    maps; the same frames a multiple of four elements apart in chunks of four
+    pixels.  Sums, half sums and aligned frames are the same bits, for rolls
+    that wrap in both directions and a frame that is not filtered."""
+    torch, _ = _init()
+    rng = np.random.default_rng(H + W)
+    N = 4
+    np_t, z = {"u8": (np.uint8, _lib.ZR_U8), "u16": (np.uint16, _lib.ZR_U16), "f16": (np.float16, _lib.ZR_F16),
+               "f32": (np.float32, _lib.ZR_F32)}[kind]
+    raw = rng.poisson(4.0, (N, H * W)).astype(np_t)
+    stride = (H * W + 3) // 4 * 4
+    spread = np.zeros((N, stride), np_t)
+    spread[:, :H * W] = raw
+    dev = [torch.from_numpy(v.view(np.int16) if kind == "u16" else v).cuda() for v in (raw, spread)]
+    maps = [torch.from_numpy(rng.uniform(0.9, 1.1, (H, W)).astype(np.float32)).cuda() for _ in range(3)]
+    ptr = [m.data_ptr() if on else None for m, on in zip(maps, (gain, hot, hot))]
+    t = np.array([[0.0, 0.0], [3.25, -7.5], [-11.0625, 4.75], [0.5, 250.125]])
+    sh = torch.from_numpy(hm.shift_table(t, H, W).view(np.uint8)).cuda()
+    got = []
+    for v, gap in zip(dev, (0, stride)):
+        fr = _lib.Frames(v.data_ptr(), z, *ptr, 0.0, N, H, W, gap)
+        for halves in (False, True):
+            out, ali = torch.zeros(3, H, W, device="cuda"), torch.zeros(N, H, W, device="cuda")
+            h = [out[i].data_ptr() if halves else None for i in (1, 2)]
+            _lib.call("zr_shift_sum", C.byref(fr), sh.data_ptr(), out[0].data_ptr(), *h, ali.data_ptr(), gh.stream())
+            got.append((out, ali))
+    for out, ali in got[1:]:
+        assert torch.equal(ali, got[0][1]) and torch.equal(out[0], got[0][0][0])
+    assert torch.equal(got[1][0], got[3][0])
+    assert torch.equal(got[1][0][1], got[0][1][0] + got[0][1][2])

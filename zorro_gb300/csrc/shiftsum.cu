@@ -20,8 +20,8 @@ constexpr int SS_NCH = (SS_TX + 2 + 3 + 3) / 4;  // 4-pixel chunks that cover a 
 constexpr int SS_TW = 4 * SS_NCH + 4;            // tile pitch: a guard column before the first chunk
 constexpr int SS_NQ = (SS_TX + 2 + 31) / 32;     // columns a lane reads of a row pixel by pixel
 // the corrections a frame's pixels take, resolved at compile time
-// (SS_BIG: any, and pixel offsets of more than 32 bits)
-enum { SS_NONE = 0, SS_HOT = 1, SS_GAIN_HOT = 2, SS_ANY = 3, SS_BIG = 4 };
+// (SS_ANY: a gain divisor too; SS_BIG: any, and pixel offsets of more than 32 bits)
+enum { SS_NONE = 0, SS_HOT = 1, SS_GAIN = 2, SS_GAIN_HOT = 3, SS_ANY = 4, SS_BIG = 5 };
 
 __device__ __forceinline__ int refl1(int i, int n) { return i < 0 ? -i - 1 : (i >= n ? 2 * n - i - 1 : i); }
 
@@ -90,7 +90,8 @@ struct SsRow {
 //
 // R = 1 serves images whose 8-row tiles all run at once.  The walk over the
 // frames is what takes the time there, so the next frame's loads are in flight
-// while this one is filtered: 40 frames of 512 x 512 with their aligned frames
+// while this one is filtered (AHEAD, which also serves larger images that are
+// read pixel by pixel: launch_shift): 40 frames of 512 x 512 with their aligned frames
 // 83 us, 117 without; 27 of 302 x 114, 45 and 70.
 //
 // What bounds it: issue slots.  The arithmetic is 6 operations a pixel, the
@@ -101,7 +102,7 @@ struct SsRow {
 // frames: 2135 us with 64 x 16 tiles whose chunks were stored and summed pixel
 // by pixel, 1360 us now; the half sums of 20 such frames 1071 -> 740 us.  Two
 // rows a thread (40 registers, six CTAs an SM) against four: 1438 and 1523 us.
-template <int TYPE, bool VEC, int MAPS, bool HALVES, int R, int CTAS>
+template <int TYPE, bool VEC, int MAPS, bool HALVES, int R, int CTAS, bool AHEAD>
 __global__ void __launch_bounds__(SS_THR, CTAS)
     k_shift_sum(FrameSrc f, const zr_shift_t* __restrict__ sh, float* __restrict__ sum,
                 float* __restrict__ even, float* __restrict__ odd, float* __restrict__ aligned) {
@@ -163,10 +164,9 @@ __global__ void __launch_bounds__(SS_THR, CTAS)
   // rows of the aligned frames start on 8 bytes (any float-aligned buffer is taken)
   const bool pairs = x + 4 <= W && (W & 1) == 0 && (reinterpret_cast<uintptr_t>(aligned) & 7) == 0;
   constexpr int NR = (TH + 7) / 8;  // tile rows a warp reads
-  constexpr bool AHEAD = R == 1;    // loads a frame ahead
   static_assert(!(AHEAD && VEC), "pixel by pixel");
   const int extra = SS_THR - 1 - threadIdx.x;               // (from the last warp down: the first ones have the odd rows)
-  const bool gain = MAPS == SS_GAIN_HOT || (MAPS >= SS_ANY && f.gain);
+  const bool gain = MAPS == SS_GAIN || MAPS == SS_GAIN_HOT || (MAPS >= SS_ANY && f.gain);
   const bool hot = MAPS == SS_GAIN_HOT || MAPS == SS_HOT || (MAPS >= SS_ANY && f.ha);
   auto wraps = [&](const zr_shift_t& t) { return first_col(t.roll_x) + ncol > W; };
   // first pixel of chunk k of a row with source r, -1 where the row does not reach it
@@ -419,28 +419,53 @@ struct SsArgs {
   cudaStream_t st;
 };
 
-template <int TYPE, bool VEC, int MAPS, int R, int CTAS>
+template <int TYPE, bool VEC, int MAPS, int R, int CTAS, bool AHEAD = false>
 static void launch_halves(const SsArgs& a, bool halves) {
   if (halves)
-    k_shift_sum<TYPE, VEC, MAPS, true, R, CTAS><<<a.grid, SS_THR, 0, a.st>>>(a.f, a.shifts, a.sum, a.even, a.odd,
-                                                                            a.aligned);
+    k_shift_sum<TYPE, VEC, MAPS, true, R, CTAS, AHEAD><<<a.grid, SS_THR, 0, a.st>>>(a.f, a.shifts, a.sum, a.even,
+                                                                                    a.odd, a.aligned);
   else
-    k_shift_sum<TYPE, VEC, MAPS, false, R, CTAS><<<a.grid, SS_THR, 0, a.st>>>(a.f, a.shifts, a.sum, a.even, a.odd,
-                                                                             a.aligned);
+    k_shift_sum<TYPE, VEC, MAPS, false, R, CTAS, AHEAD><<<a.grid, SS_THR, 0, a.st>>>(a.f, a.shifts, a.sum, a.even,
+                                                                                     a.odd, a.aligned);
 }
 
-// small: CTAs an SM of the kernel that loads a frame ahead, 0 for the other
+// small: CTAs an SM of the kernel with tiles of 8 rows, 0 for those of 16.
+//
+// Frames read pixel by pixel: what a warp waits for are its loads, so it has the
+// next frame's in flight while it filters (AHEAD), as far as the registers for
+// them go: five columns of three rows, for the counts and for every map.  30
+// frames of 1001 x 1003, microseconds: without maps 103 ahead (four CTAs an SM)
+// and 164 not; of 901 x 903 with a gain 105 ahead (three) and 146 not, but just
+// over one wave of those, 1001 x 1003, 158 and 148, until the fifth CTA an SM
+// is full too: 1401 x 1403 252 and 282; with gain and hot-pixel maps (two) 97
+// ahead at 701 x 703, where two are a wave, and 130 not, 184 and 169 at 1001 x
+// 1003.
 template <int TYPE>
 static void launch_shift(const SsArgs& a, bool vec, int small, bool halves, int maps) {
   if (maps == SS_BIG) return launch_halves<TYPE, false, SS_BIG, 2, 5>(a, halves);
-  if (small == 2) return launch_halves<TYPE, false, SS_ANY, 1, 2>(a, halves);
-  if (small == 3) return launch_halves<TYPE, false, SS_ANY, 1, 3>(a, halves);
-  if (!vec) return launch_halves<TYPE, false, SS_ANY, 2, 5>(a, halves);
-  switch (maps) {
+  if (small == 2) return launch_halves<TYPE, false, SS_ANY, 1, 2, true>(a, halves);
+  if (small == 3) return launch_halves<TYPE, false, SS_ANY, 1, 3, true>(a, halves);
+  if (vec) switch (maps) {
     case SS_NONE: return launch_halves<TYPE, true, SS_NONE, 2, 6>(a, halves);
     case SS_HOT: return launch_halves<TYPE, true, SS_HOT, 2, 6>(a, halves);
+    case SS_GAIN: return launch_halves<TYPE, true, SS_GAIN, 2, 6>(a, halves);
     case SS_GAIN_HOT: return launch_halves<TYPE, true, SS_GAIN_HOT, 2, 6>(a, halves);
-    default: launch_halves<TYPE, true, SS_ANY, 2, 4>(a, halves);
+    default: return launch_halves<TYPE, true, SS_ANY, 2, 4>(a, halves);
+  }
+  const long long tiles = (long long)a.grid.x * a.grid.y;
+  const bool two = tiles <= 2 * SS_SMS;
+  switch (maps) {
+    case SS_NONE: return launch_halves<TYPE, false, SS_NONE, 2, 4, true>(a, halves);
+    case SS_GAIN:
+      return tiles <= 3 * SS_SMS || tiles > 5 * SS_SMS ? launch_halves<TYPE, false, SS_GAIN, 2, 3, true>(a, halves)
+                                                       : launch_halves<TYPE, false, SS_GAIN, 2, 5>(a, halves);
+    case SS_HOT:
+      return two ? launch_halves<TYPE, false, SS_HOT, 2, 2, true>(a, halves)
+                 : launch_halves<TYPE, false, SS_HOT, 2, 5>(a, halves);
+    case SS_GAIN_HOT:
+      return two ? launch_halves<TYPE, false, SS_GAIN_HOT, 2, 2, true>(a, halves)
+                 : launch_halves<TYPE, false, SS_GAIN_HOT, 2, 5>(a, halves);
+    default: return launch_halves<TYPE, false, SS_ANY, 2, 5>(a, halves);
   }
 }
 
@@ -471,12 +496,12 @@ extern "C" int zr_shift_sum(const zr_frames_t* frames, const zr_shift_t* shifts,
   const int nx = (f.W + SS_TX - 1) / SS_TX;
   const bool big = (long long)f.H * f.W >= (1LL << 30);
   const long long tiles = (long long)nx * ((f.H + 7) / 8);
-  const int small = big ? 0 : (tiles <= 2 * SS_SMS ? 2 : (tiles <= 3 * SS_SMS ? 3 : 0));
+  const int small = big ? 0 : (tiles <= 2 * SS_SMS ? 2 : (vec && tiles <= 3 * SS_SMS ? 3 : 0));
   const dim3 grid(nx, small ? (f.H + 7) / 8 : (f.H + 15) / 16);
   // (byte offsets of pixels within 32 bits, for frames of less than 2^30)
   const int maps = big              ? SS_BIG
                    : f.gdiv != 0.0f ? SS_ANY
-                   : f.gain         ? (f.ha ? SS_GAIN_HOT : SS_ANY)
+                   : f.gain         ? (f.ha ? SS_GAIN_HOT : SS_GAIN)
                                     : (f.ha ? SS_HOT : SS_NONE);
   const SsArgs a{f, shifts, image_sum, even_sum, odd_sum, aligned, grid, st};
   switch (f.type) {
