@@ -545,3 +545,58 @@ def test_shift_sum_paths_agree(kind, gain, hot, H, W):
         assert torch.equal(ali, got[0][1]) and torch.equal(out[0], got[0][0][0])
     assert torch.equal(got[1][0], got[3][0])
     assert torch.equal(got[1][0][1], got[0][1][0] + got[0][1][2])
+
+
+@pytest.mark.parametrize("kind,maps,H,W,P,Cc", [
+    ("u8", True, 57, 61, 64, 64), ("f32", False, 100, 128, 128, 64), ("f16", True, 200, 233, 256, 128),
+    ("u16", False, 301, 499, 512, 256), ("f32", True, 997, 1001, 1024, 512), ("u8", False, 1500, 1533, 1536, 768),
+    ("u8", True, 2040, 1999, 2048, 1024), ("f32", False, 3000, 3071, 3072, 1536)])
+def test_spectra_of_masked_frames_and_of_masks(kind, maps, H, W, P, Cc):
+    """G and S of frames under a mask of any values, the mask's own spectrum and
+    that of the default mask, against float64 transforms: 6e-8 log2 of the
+    transform's length in the 2-norm, twice that for the squares."""
+    torch, lib = _init()
+    rng = np.random.default_rng(P)
+    N = 2
+    np_t, z = {"u8": (np.uint8, _lib.ZR_U8), "u16": (np.uint16, _lib.ZR_U16), "f16": (np.float16, _lib.ZR_F16),
+               "f32": (np.float32, _lib.ZR_F32)}[kind]
+    raw = rng.poisson(5.0, (N, H, W)).astype(np_t)
+    dev = torch.from_numpy(raw.view(np.int16) if kind == "u16" else raw).cuda()
+    mask = rng.uniform(0.0, 1.0, (P, P)).astype(np.float32) * (rng.random((P, P)) > 0.1)
+    host = [rng.uniform(0.9, 1.1, (H, W)).astype(np.float32) for _ in range(3)] if maps else []
+    dm = [torch.from_numpy(m).cuda() for m in host]
+    fr = _lib.Frames(dev.data_ptr(), z, *([m.data_ptr() for m in dm] if maps else [None] * 3), 0.0, N, H, W, 0)
+    v = raw.astype(np.float64)
+    if maps:
+        v = v * host[0] * host[1] + host[2]
+    K4 = lib.zr_spectrum_pitch(Cc)
+    G, S = (torch.empty(N, K4, Cc + 4, 2, device="cuda") for _ in range(2))
+    sums = torch.from_numpy(v.reshape(N, -1).sum(1)).cuda()
+    wb = lib.zr_spectra_work_bytes(P, N, Cc)
+    work = torch.empty(wb, dtype=torch.uint8, device="cuda")
+    dmask = torch.from_numpy(mask).cuda()
+
+    def layout(u):
+        F = np.fft.rfft2(u)
+        rows = [r if r < Cc // 2 else P - Cc + r for r in range(Cc)] + [Cc // 2]
+        return F[rows][:, :Cc // 2 + 1].T
+
+    def check(t, u, tol):
+        got = t.cpu().numpy().astype(np.float64)
+        got = (got[..., 0] + 1j * got[..., 1])[:Cc // 2 + 1, :Cc + 1]
+        want = layout(u)
+        assert np.linalg.norm(got - want) <= tol * np.linalg.norm(want)
+
+    tol = 6e-8 * 2 * np.log2(P)
+    _lib.call("zr_spectra", C.byref(fr), dmask.data_ptr(), sums.data_ptr(), 0, N, 0, P, P, Cc, Cc, G.data_ptr(),
+              S.data_ptr(), work.data_ptr(), wb, gh.stream())
+    for n in range(N):
+        mu = float(np.float32(sums[n].item() / (H * W)))
+        u = np.zeros((P, P))
+        u[:H, :W] = mask[:H, :W].astype(np.float64) * (v[n] - mu)
+        check(G[n], u, tol)
+        check(S[n], u * u, 2 * tol)
+    for m, u in ((dmask.data_ptr(), mask.astype(np.float64)), (None, np.pad(np.ones((H, W)), ((0, P - H), (0, P - W))))):
+        _lib.call("zr_spectra", C.byref(fr), m, None, 0, 1, 1, P, P, Cc, Cc, G.data_ptr(), None, work.data_ptr(), wb,
+                  gh.stream())
+        check(G[0], u, tol)

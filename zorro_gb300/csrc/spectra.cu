@@ -180,22 +180,28 @@ __global__ void __launch_bounds__(ip_threads(P1, FR), minb_of(ip_threads(P1, FR)
     // their padded rows)
     if (cols >= 14 * P::A1) pixels(std::integral_constant<int, 14>());
     else pixels(std::integral_constant<int, 0>());
-  } else {
+  } else if (mode == 0) {
     ip_pass1<P1, FR, T, -1, false>(sm, [&](int b, int j, float2* v) {
-      const int y = y0 + b;
+      const int y = y0 + b, lim = y < rows ? cols - j : 0;
+      const float* m = mask + (size_t)y * P1 + j;
+      float u[16], k[16];
+#pragma unroll
+      for (int r = 0; r < 16; r++) k[r] = r * P::A1 < lim ? __ldg(m + r * P::A1) : 0.0f;
+      if (y < rows) corrected16<P::A1, 0>(f, n, y, j, cols, u);
 #pragma unroll
       for (int r = 0; r < 16; r++) {
-        const int x = j + r * P::A1;
-        v[r] = make_float2(0.0f, 0.0f);
-        if (y < rows && x < cols) {
-          const float m = mask ? __ldg(mask + (size_t)y * P1 + x) : 1.0f;
-          if (mode == 0) {
-            const float w = m * (load_corrected(f, n, y, x) - mu);
-            v[r] = make_float2(w, w * w);
-          } else {
-            v[r].x = m;
-          }
-        }
+        const float w = r * P::A1 < lim ? k[r] * (u[r] - mu) : 0.0f;
+        v[r] = make_float2(w, w * w);
+      }
+    });
+  } else {  // the mask itself
+    ip_pass1<P1, FR, T, -1, false>(sm, [&](int b, int j, float2* v) {
+      const int y = y0 + b, lim = y < rows ? cols - j : 0;
+      const float* m = mask + (size_t)y * P1 + j;
+#pragma unroll
+      for (int r = 0; r < 16; r++) {
+        const bool in = r * P::A1 < lim;
+        v[r] = make_float2(in ? (mask ? __ldg(m + r * P::A1) : 1.0f) : 0.0f, 0.0f);
       }
     });
   }
