@@ -9,8 +9,8 @@
 // The filters are real and even in frequency, so the accumulated spectrum is
 // Hermitian: only kx in [0, P1/2] is kept.  Two aligned frames share one
 // complex row FFT; the column pass applies each frame's filter and
-// accumulates in shared memory; the inverse column pass keeps only the H
-// output rows and the final row pass packs two rows per complex inverse FFT.
+// accumulates in registers; the inverse column pass keeps only the H output
+// rows and the final row pass packs two rows per complex inverse FFT.
 #include <math.h>
 
 #include <type_traits>
@@ -138,23 +138,6 @@ __device__ __forceinline__ float crit_dose(const zr_dose_params_t& p, int fy, in
   return p.voltage_scaling * (p.crit_a * powf(q, p.crit_b) + p.crit_c);
 }
 
-__device__ __forceinline__ void dose_weight(const zr_dose_params_t& p, int P0, int P1, int ky, int kx, float dose_end,
-                                            float tq, float& w) {
-  const int fy = ky < P0 / 2 ? ky : ky - P0;
-  const int fx = kx;
-  const float q = sqrtf((float)fx * (float)fx * (p.inv_ps_x * p.inv_ps_x) + (float)fy * (float)fy * (p.inv_ps_y * p.inv_ps_y));
-  float crit;
-  if (ky == P0 / 2 && kx == P1 / 2) {
-    const float c = crit_dose(p, fy, P1 / 2 - 1);
-    crit = c * c;
-  } else {
-    crit = p.voltage_scaling * (p.crit_a * powf(q, p.crit_b) + p.crit_c);
-  }
-  const float filt = expf((-0.5f * dose_end) / crit);
-  const float thres = expf(-powf(q / tq, p.cutoff_order));
-  w = thres * filt;
-}
-
 // The whole filter of 40 K2 frames went from 2708 to 2395 us with the in-place
 // transforms (fft_inplace.cuh) and to 2235 us with the row pass above; the row
 // and column passes' intermediates (2.7 GB each way) and the 2.3 GB of frames
@@ -197,14 +180,14 @@ __global__ void __launch_bounds__(ds_ct(P0), ds_minb(ds_ct(P0)))
   // shared memory)
   constexpr bool SPREAD = P::NS < T;
   constexpr int PER = SPREAD ? P0 / T : P::RL, STEP = SPREAD ? T : P::NS;
-  const bool mine = (int)threadIdx.x < STEP;
+  static_assert(STEP == T, "every thread holds its rows");
   float2 acc[PER];
   float fm[PER];
 #pragma unroll
   for (int r = 0; r < PER; r++) {
     const size_t o = (size_t)kx * P0 + threadIdx.x + r * STEP;
-    acc[r] = first || !mine ? make_float2(0.0f, 0.0f) : ACC[o];
-    fm[r] = (first || !mine || !prm.normalize) ? 0.0f : FM[o];
+    acc[r] = first ? make_float2(0.0f, 0.0f) : ACC[o];
+    fm[r] = (first || !prm.normalize) ? 0.0f : FM[o];
   }
   const float LOG2E = 1.4426950408889634f;
   for (int nl = 0; nl < nfr; nl++) {
@@ -223,7 +206,7 @@ __global__ void __launch_bounds__(ds_ct(P0), ds_minb(ds_ct(P0)))
       ip_last_inplace<P0, 1, T, -1>(sm, tw);
       __syncthreads();
     }
-    if (live && mine) {
+    if (live) {
       float2 v[PER];
       if constexpr (SPREAD) {
 #pragma unroll
@@ -244,7 +227,6 @@ __global__ void __launch_bounds__(ds_ct(P0), ds_minb(ds_ct(P0)))
       }
     }
   }
-  if (!mine) return;
 #pragma unroll
   for (int r = 0; r < PER; r++) {
     const size_t o = (size_t)kx * P0 + threadIdx.x + r * STEP;

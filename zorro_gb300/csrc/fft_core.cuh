@@ -8,8 +8,8 @@
 // pass radix 2, 4 or 8 when log2(L) is not a multiple of 4): every thread reads
 // its butterflies' inputs into registers, the CTA synchronises, and the outputs
 // are written back.  No ping-pong buffer is needed.  (The other transforms use
-// fft_inplace.cuh, which takes fewer exchanges; the FRC keeps this one's
-// roundings, which its float64 ring sums show.)
+// fft_inplace.cuh, which takes fewer exchanges.  The FRC stays with this one for
+// the bits of its results, not for their accuracy, which is 1e-6 either way.)
 //
 // Twiddles come from a table of W_TWN^k = exp(-2 pi i k / TWN), TWN = 2^14 x
 // 3^2 x 5, computed in double precision on the host and rounded to float

@@ -20,11 +20,6 @@ inline bool is_pow2(long long v) { return v > 0 && (v & (v - 1)) == 0; }
 inline bool fft_len_ok(long long v) {
   return is_pow2(v) || v == 384 || v == 768 || v == 1536 || v == 3072 || v == 6144;
 }
-inline int ilog2(long long v) {
-  int l = 0;
-  while ((1LL << l) < v) ++l;
-  return l;
-}
 
 // Threads for a batched shared-memory FFT of NB sequences of length L:
 // ZR_FFT_EPT elements per thread and pass (radix-8 butterflies of 8).

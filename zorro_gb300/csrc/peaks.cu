@@ -1,6 +1,7 @@
 // Peak search on the correlation windows (locatePeak, zorro.py:1099-1231).
 //
-// One CTA per pair keeps the w x w window in shared memory and runs, with all
+// Each window is searched by one CTA, or by a cluster of them that share its rows
+// out (k_peaks); a CTA keeps the w x w window in shared memory and runs, with all
 // threads in lock step:
 //   * suppressOrigin (zorro.py:1078-1083, literal stencil);
 //   * Bmode 'opti': a bounded Brent minimisation over sigma in [0, 7] of
@@ -48,7 +49,6 @@ struct PkShared {
   alignas(16) float wy[2 * PK_MAXR + 4];  // 16-byte aligned: read four taps at a time
   alignas(16) float wx[2 * PK_MAXR + 4];
   alignas(16) float ws[2 * PK_MAXR + 4];  // the search's weights, both axes
-  double red[PK_NW][3];
   float redf[PK_NW];
   int redi[PK_NW];
   float ws1[PK_NW], ws2[PK_NW], wmx[PK_NW];  // per-warp partials of the filter statistics
@@ -105,31 +105,6 @@ __device__ int gauss_weights(double sigma, float* w) {
 }
 
 // Block reductions (all threads must call).
-__device__ double3 block_sum3(PkShared& sh, double a, double b, double c) {
-  for (int o = 16; o > 0; o >>= 1) {
-    a += __shfl_down_sync(0xffffffffu, a, o);
-    b += __shfl_down_sync(0xffffffffu, b, o);
-    c += __shfl_down_sync(0xffffffffu, c, o);
-  }
-  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (lane == 0) { sh.red[wid][0] = a; sh.red[wid][1] = b; sh.red[wid][2] = c; }
-  __syncthreads();
-  if (wid == 0) {
-    a = lane < PK_NW ? sh.red[lane][0] : 0.0;
-    b = lane < PK_NW ? sh.red[lane][1] : 0.0;
-    c = lane < PK_NW ? sh.red[lane][2] : 0.0;
-    for (int o = 16; o > 0; o >>= 1) {
-      a += __shfl_down_sync(0xffffffffu, a, o);
-      b += __shfl_down_sync(0xffffffffu, b, o);
-      c += __shfl_down_sync(0xffffffffu, c, o);
-    }
-    if (lane == 0) { sh.bc[0] = a; sh.bc[1] = b; sh.bc[2] = c; }
-  }
-  __syncthreads();
-  double3 r = make_double3(sh.bc[0], sh.bc[1], sh.bc[2]);
-  __syncthreads();
-  return r;
-}
 
 // max value with the smallest index among equal values; where no thread has
 // one (all of them NaN), NaN and index 0, as np.argmax has it
