@@ -469,9 +469,11 @@ extern "C" int zr_histogram(const float* values, long long n, double first_edge,
   const double k = first_edge + 0.5;
   if (k == floor(k) && fabs(k) < 4194304.0) {
     // as many copies as 48 KB of shared memory holds, one a warp at most, and no
-    // more counters than twice a CTA's pixels, which have to be cleared and
-    // added up (200 x 180 sums in 1600 bins 6.8 us with seven copies, 5.0 with one)
-    const long long fit = 48 * 1024 / (long long)smem, worth = 2 * ((n + blocks - 1) / blocks) / nbins;
+    // more counters than half a CTA's pixels, which have to be cleared and added
+    // up: 1900 x 1900 sums of a mean of 20 in 3000 bins 8.3 us with one copy and
+    // 10.3 with three, 200 x 180 in 1600 5.0 and 6.8 with seven; a K2 sum in
+    // 46 takes 14.4 with sixteen
+    const long long fit = 48 * 1024 / (long long)smem, worth = (n + blocks - 1) / blocks / nbins / 2;
     const int copies = (int)std::max(1LL, std::min({16LL, fit, worth}));
     ZR_TRY(cuda_check(cudaFuncSetAttribute(k_histogram_half, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            (int)(smem * copies)), "hist attr"));
