@@ -234,6 +234,29 @@ def test_whole_planes_of_nan():
     assert np.isnan(r["corr"][0]) and abs(r["corr"][1] - 1.0) < 1e-5
 
 
+@pytest.mark.parametrize("mS", [8, 9, 20, 33, 47, 48, 51, 100, 112])
+@pytest.mark.parametrize("use_mask", [0, 1])
+@pytest.mark.parametrize("M", [1, 20, 60, 160])
+def test_unfiltered_windows(mS, use_mask, M):
+    """Without a filter the peak is the first largest value of the window or its
+    disc (zeros outside compete) and its significance (max - mean) / std.  The
+    statistics are float32 sums of at most 49 pixels a thread and 5 levels of a
+    warp, float64 above: std is within 28 roundings, mean within 56 of std."""
+    w = 2 * mS
+    win = _windows(np.random.default_rng(mS), M, mS)
+    win[1::2] = np.round(win[1::2] * np.float32(2000.0))  # ties
+    y, x = np.mgrid[:w, :w] - mS
+    disc = (y * y + x * x < mS * mS) if use_mask else np.ones((w, w), bool)
+    got = _locate(win, mS, bmode=0, use_mask=use_mask, sub_pix_reg=1, suppress_origin=0)
+    for k in range(M):
+        at = int(np.argmax(np.where(disc, win[k], np.float32(0.0))))
+        r, v = got[k], win[k].astype(np.float64)
+        assert (r["cy"], r["cx"], r["corr"]) == (at // w, at % w, win[k].flat[at])
+        assert (r["sy"], r["sx"]) == (at // w - mS, at % w - mS)
+        sig = (np.where(disc, v, 0.0).max() - v[disc].mean()) / v[disc].std()
+        assert abs(r["peaksig"] - sig) <= 2.0 ** -24 * (30 * sig + 60), (k, r["peaksig"], sig)
+
+
 @pytest.mark.parametrize("mS", [8, 9, 25, 47, 48])
 def test_one_windows_record_at_any_number(mS):
     """Around a wave of 152 windows, and on both sides of the size from which

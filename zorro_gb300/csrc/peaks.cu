@@ -431,6 +431,23 @@ __device__ PkSums filter_rows(const float* C, float* V, const PkRows& L, int mS,
       a.mx = fmaxf(a.mx, v);
     }
   };
+  if (MODE == 1 && ry == 0 && rx == 0) {  // no filter (the one weight is 1): the window's own values
+    const int n = L.quad ? 2 : 1;
+    for (int yb = n * ty; owner && yb < w; yb += n * L.rb)
+      for (int y = yb; y < min(w, yb + n); y++) {
+        const float* row = C + y * w;
+        if (L.quad) {
+          const float4 v = *reinterpret_cast<const float4*>(row + 4 * tx);
+          add(y, 4 * tx, v.x);
+          add(y, 4 * tx + 1, v.y);
+          add(y, 4 * tx + 2, v.z);
+          add(y, 4 * tx + 3, v.w);
+        } else {
+          for (int x = tx; x < w; x += 64) add(y, x, row[x]);
+        }
+      }
+    return a;
+  }
   auto horizontal = [&](int m, int x, float (&f)[8]) {
     const float* p = V + m * L.vp + L.pad + x - rx - OFF;
     switch (OFF) {
@@ -1461,10 +1478,15 @@ extern "C" int zr_locate_peaks(const float* cwin, int M, int max_shift, const zr
   // Windows below 96 pixels, each a CTA: two cluster barriers a function value
   // take longer than the rows they share out (20 windows of 40 x 40 169 us, 193
   // in clusters of two, 191 of four; of 82 x 82 201, 208 and 201; of 96 x 96
-  // 199, 197 and 181; of 100 x 100 208, 191 and 171).  Larger ones: full waves of
-  // one CTA per window and SM, then what is left with as many CTAs per window as
-  // fit the SMs.
-  if (w < 96) return launch_peaks<1>(cwin, M, max_shift, *params, pad, vfloats, base + vbytes, results, tw, st);
+  // 199, 197 and 181; of 100 x 100 208, 191 and 171).  So are unfiltered windows
+  // of any size, and those of one given filter where they are more than a wave:
+  // a second wave that starts as SMs fall free takes less than a second launch
+  // (190 of 128 x 128 unfiltered 29 us against 33, with a filter and 16-fold
+  // sub-pixels 68 against 94; 20 of 200 x 200 with a filter 43 in clusters, 66
+  // without).  In the search, full waves of one CTA per window and SM, then what
+  // is left with as many CTAs per window as fit the SMs.
+  if (w < 96 || (params->bmode != 1 && (params->bmode != 2 || M > PK_SMS)))
+    return launch_peaks<1>(cwin, M, max_shift, *params, pad, vfloats, base + vbytes, results, tw, st);
   const int full = M / PK_SMS * PK_SMS, rest = M - full;
   if (full) ZR_TRY(launch_peaks<1>(cwin, full, max_shift, *params, pad, vfloats, base + vbytes, results, tw, st));
   cwin += (size_t)full * w * w;
