@@ -116,8 +116,10 @@ __device__ __forceinline__ void corrected32(const FrameSrc& f, int n, int y, int
 // Row pass: FR rows of one frame per CTA.  The first FFT pass reads the
 // pixels (consecutive lanes, consecutive pixels) and the last one untangles
 // the half-plane rows of u and u^2 in registers, so the rows pass through
-// shared memory twice and the CTA meets at two barriers.
-template <int P1, int FR>
+// shared memory twice and the CTA meets at two barriers.  MASKS: frames under a
+// mask, and masks themselves (a kernel of their own: in one with the plain
+// frames their loads made those spill, spectra of eight K2 frames 588 -> 596 us).
+template <int P1, int FR, bool MASKS>
 __global__ void __launch_bounds__(ip_threads(P1, FR), minb_of(ip_threads(P1, FR)))
     k_fwd_rows(FrameSrc f, const float* __restrict__ mask, const double* __restrict__ mean_sub,
                double inv_area, int frame0, int mode, int rows, int cols, int C1, int K4, int H4, bool wide,
@@ -131,8 +133,37 @@ __global__ void __launch_bounds__(ip_threads(P1, FR), minb_of(ip_threads(P1, FR)
   const int nl = blockIdx.x;
   const int n = frame0 + nl;
   float mu = 0.0f;
-  if (mode == 0 && mean_sub) mu = (float)(mean_sub[n] * inv_area);
-  if (mode == 0 && !mask && wide) {
+  if ((!MASKS || mode == 0) && mean_sub) mu = (float)(mean_sub[n] * inv_area);
+  if constexpr (MASKS) {
+    if (mode == 0) {
+      ip_pass1<P1, FR, T, -1, false>(sm, [&](int b, int j, float2* v) {
+        const int y = y0 + b, lim = y < rows ? cols - j : 0;
+        const float* m = mask + (size_t)y * P1 + j;
+        float u[16], k[16];
+#pragma unroll
+        for (int r = 0; r < 16; r++) k[r] = r * P::A1 < lim ? __ldg(m + r * P::A1) : 0.0f;
+        if (y < rows) corrected16<P::A1, 0>(f, n, y, j, cols, u);
+#pragma unroll
+        for (int r = 0; r < 16; r++) {
+          const float w = r * P::A1 < lim ? k[r] * (u[r] - mu) : 0.0f;
+          v[r] = make_float2(w, w * w);
+        }
+      });
+    } else if (mask) {  // the mask itself
+      ip_pass1<P1, FR, T, -1, false>(sm, [&](int b, int j, float2* v) {
+        const int y = y0 + b, lim = y < rows ? cols - j : 0;
+        const float* m = mask + (size_t)y * P1 + j;
+#pragma unroll
+        for (int r = 0; r < 16; r++) v[r] = make_float2(r * P::A1 < lim ? __ldg(m + r * P::A1) : 0.0f, 0.0f);
+      });
+    } else {  // (ones inside the frame)
+      ip_pass1<P1, FR, T, -1, false>(sm, [&](int b, int j, float2* v) {
+        const int lim = y0 + b < rows ? cols - j : 0;
+#pragma unroll
+        for (int r = 0; r < 16; r++) v[r] = make_float2(r * P::A1 < lim ? 1.0f : 0.0f, 0.0f);
+      });
+    }
+  } else if (wide) {
     auto pixels = [&](auto full) {
       constexpr int FULL = decltype(full)::value;
       ip_pass1_pairs<P1, FR, T, -1>(sm, [&](int b, int j, int odd, float2* v0, float2* v1) {
@@ -156,7 +187,7 @@ __global__ void __launch_bounds__(ip_threads(P1, FR), minb_of(ip_threads(P1, FR)
     };
     if (cols >= 14 * P::A1) pixels(std::integral_constant<int, 14>());
     else pixels(std::integral_constant<int, 0>());
-  } else if (mode == 0 && !mask) {
+  } else {
     auto pixels = [&](auto full) {
       constexpr int FULL = decltype(full)::value;
       ip_pass1<P1, FR, T, -1, false>(sm, [&](int b, int j, float2* v) {
@@ -180,30 +211,6 @@ __global__ void __launch_bounds__(ip_threads(P1, FR), minb_of(ip_threads(P1, FR)
     // their padded rows)
     if (cols >= 14 * P::A1) pixels(std::integral_constant<int, 14>());
     else pixels(std::integral_constant<int, 0>());
-  } else if (mode == 0) {
-    ip_pass1<P1, FR, T, -1, false>(sm, [&](int b, int j, float2* v) {
-      const int y = y0 + b, lim = y < rows ? cols - j : 0;
-      const float* m = mask + (size_t)y * P1 + j;
-      float u[16], k[16];
-#pragma unroll
-      for (int r = 0; r < 16; r++) k[r] = r * P::A1 < lim ? __ldg(m + r * P::A1) : 0.0f;
-      if (y < rows) corrected16<P::A1, 0>(f, n, y, j, cols, u);
-#pragma unroll
-      for (int r = 0; r < 16; r++) {
-        const float w = r * P::A1 < lim ? k[r] * (u[r] - mu) : 0.0f;
-        v[r] = make_float2(w, w * w);
-      }
-    });
-  } else {  // the mask itself
-    ip_pass1<P1, FR, T, -1, false>(sm, [&](int b, int j, float2* v) {
-      const int y = y0 + b, lim = y < rows ? cols - j : 0;
-      const float* m = mask + (size_t)y * P1 + j;
-#pragma unroll
-      for (int r = 0; r < 16; r++) {
-        const bool in = r * P::A1 < lim;
-        v[r] = make_float2(in ? (mask ? __ldg(m + r * P::A1) : 1.0f) : 0.0f, 0.0f);
-      }
-    });
   }
   __syncthreads();
   ip_pass2<P1, FR, T, -1, false>(sm, tw);
@@ -216,7 +223,7 @@ __global__ void __launch_bounds__(ip_threads(P1, FR), minb_of(ip_threads(P1, FR)
     float2 *ou = RU + o, *ov = RV + o;
     auto put = [&](int k, float2 zk, float2 zm) {
       ou[k * step] = make_float2(0.5f * (zk.x + zm.x), 0.5f * (zk.y - zm.y));
-      if (mode == 0) ov[k * step] = make_float2(0.5f * (zk.y + zm.y), -0.5f * (zk.x - zm.x));
+      if (!MASKS || mode == 0) ov[k * step] = make_float2(0.5f * (zk.y + zm.y), -0.5f * (zk.x - zm.x));
     };
 #pragma unroll
     for (int q = 0; q < P::RL; q++) {
@@ -231,7 +238,7 @@ __global__ void __launch_bounds__(ip_threads(P1, FR), minb_of(ip_threads(P1, FR)
     if ((y0 + b) >> 2 >= H4) continue;
     const size_t o = frame_out + ru_at(k, y0 + b, K4, H4);
     RU[o] = make_float2(0.0f, 0.0f);
-    if (mode == 0) RV[o] = make_float2(0.0f, 0.0f);
+    if (!MASKS || mode == 0) RV[o] = make_float2(0.0f, 0.0f);
   }
 }
 
@@ -322,18 +329,26 @@ static bool wide_pixels(const FrameSrc& f, int cols) {
          (uintptr_t)f.raw % (2 * esize) == 0;
 }
 
-template <int P, int FR>
-static int launch_rows_v(const FrameSrc& f, const float* mask, const double* mean_sub, double inv_area,
+template <int P, int FR, bool MASKS>
+static int launch_rows_m(const FrameSrc& f, const float* mask, const double* mean_sub, double inv_area,
                          int frame0, int nfr, int mode, int rows, int cols, int C1, int K4, int H4,
                          float2* RU, float2* RV, const float2* tw, cudaStream_t st) {
   constexpr int T = ip_threads(P, FR);
   const size_t smem = (size_t)FR * ip_ld(P, FR) * sizeof(float2);
-  ZR_TRY(cuda_check(cudaFuncSetAttribute(k_fwd_rows<P, FR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+  ZR_TRY(cuda_check(cudaFuncSetAttribute(k_fwd_rows<P, FR, MASKS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                     "k_fwd_rows attr"));
-  k_fwd_rows<P, FR><<<dim3(nfr, (rows + FR - 1) / FR), T, smem, st>>>(f, mask, mean_sub, inv_area, frame0, mode,
-                                                                       rows, cols, C1, K4, H4, wide_pixels(f, cols),
-                                                                       RU, RV, tw);
+  k_fwd_rows<P, FR, MASKS><<<dim3(nfr, (rows + FR - 1) / FR), T, smem, st>>>(f, mask, mean_sub, inv_area, frame0, mode,
+                                                                              rows, cols, C1, K4, H4,
+                                                                              wide_pixels(f, cols), RU, RV, tw);
   return launched("k_fwd_rows");
+}
+
+template <int P, int FR>
+static int launch_rows_v(const FrameSrc& f, const float* mask, const double* mean_sub, double inv_area,
+                         int frame0, int nfr, int mode, int rows, int cols, int C1, int K4, int H4,
+                         float2* RU, float2* RV, const float2* tw, cudaStream_t st) {
+  const auto run = mask || mode != 0 ? launch_rows_m<P, FR, true> : launch_rows_m<P, FR, false>;
+  return run(f, mask, mean_sub, inv_area, frame0, nfr, mode, rows, cols, C1, K4, H4, RU, RV, tw, st);
 }
 
 template <int P>
