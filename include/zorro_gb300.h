@@ -150,7 +150,8 @@ int zr_hotpix_thresholds(double mu, double sigma, float cutoff_lower, float cuto
  * folded into per-pixel affine maps hot_a (logisticMask) and hot_b
  * (singletonOutlierMask*psfFiltMean + neighbourFilt).  counts3 (accumulated)
  * receives guessDeadpix, guessHotpix and neighborPix.  ``work`` holds
- * zr_hotpix_work_bytes() bytes. */
+ * zr_hotpix_work_bytes() bytes (asked for as ever, though the maps are made in
+ * one kernel that keeps nothing in it). */
 size_t zr_hotpix_work_bytes(int height, int width);
 int zr_hotpix_maps(const float* unaligned_sum, int height, int width, int n_frames,
                    const zr_hotpix_params_t* params, float* hot_a, float* hot_b,
@@ -168,7 +169,9 @@ int zr_unpack_u4(const void* packed, int n_frames, int height, int width, void* 
  * the crop keeping rows [0, Hb/2) and [H - Hb/2, H) and columns likewise; the
  * frames are read with their gain (hot-pixel maps are not applied: the
  * reference bins before its hot-pixel filter).  Hb and Wb even; every side
- * in 513..8192 (Bluestein transforms of 2048..16384 points).  work:
+ * in 513..8192 (transformed directly where the library has the length, else as
+ * Bluestein transforms of 2048..16384 points) or one of 9216, 10240, 11520,
+ * 12288, 15360 and 16384.  work:
  * zr_bin_work_bytes(H, W, Hb, Wb) bytes. */
 size_t zr_bin_work_bytes(int H, int W, int Hb, int Wb);
 int zr_bin_fourier(const zr_frames_t* frames, int Hb, int Wb, float* out, void* work, size_t work_bytes,
